@@ -169,8 +169,8 @@ def _state(case, seed):
         V[:, 1] -= 0.5
         return X, V
     xs, vs = [], []
-    for m in _models(case):
-        X = _rest(m)[0].astype(np.float64)
+    rests = [_rest(m)[0].astype(np.float64) for m in _models(case)]
+    for m, X in zip(_models(case), rests):
         c = X.mean(0)
         A = rng.uniform(-0.01, 0.01, (3, 3))
         if case["kind"] == "twist":
@@ -182,10 +182,18 @@ def _state(case, seed):
             x[:, 1] -= x[:, 1].min() + rng.uniform(0, 5e-4)  # the lowest vertices in the ground
             v += np.array([rng.uniform(-0.3, 0.3), -0.5, rng.uniform(-0.3, 0.3)])
         elif case["kind"] == "cluster":
-            v[:, 1] -= 4.0 * len(xs)  # each body falls on the one below within the step
+            if xs:  # each body falls on the one below within the step
+                x[:, 1] += xs[-1][:, 1].max() + 1e-3 - x[:, 1].min()
+            v[:, 1] -= 2.0 * len(xs)
         elif case["kind"] == "collide":
-            g = np.array([0.5, 0.5, 0.5]) - c
-            v += 10.0 * g / max(np.linalg.norm(g), 1e-6)  # towards the middle: trajectories meet
+            v[:, 1] -= 0.2
+            # a ball (odd) whose nearest neighbour is a cube has come close to it and touches it
+            near = np.argsort([np.linalg.norm(q.mean(0) - c) - np.ptp(q, 0).max() / 2 for q in rests])
+            k = int([j for j in near if j != len(xs)][0])
+            if len(xs) % 2 and k % 2 == 0:
+                u = (rests[k].mean(0) - c) / np.linalg.norm(rests[k].mean(0) - c)
+                x += (((rests[k] - c) @ u).min() - ((x - c) @ u).max() - 1e-3) * u
+                v += 0.6 * u
         if case["kind"] == "twist":
             v = np.zeros_like(x)
             x[m["fixedPoints"]] = X[m["fixedPoints"]]
