@@ -4,10 +4,10 @@
 // 14.6k incidences), a cluster of C blocks (C <= 16, one per SM) takes one scene at a
 // time from a work counter and runs all its iterations without touching global memory
 // for positions or records:
-//   * every block holds a copy of all the scene's states (active and fixed vertices) in
-//     its shared memory, and the incidence records of the vertices it owns: of each
-//     color, the block of rank r owns a contiguous chunk, whose records are one
-//     contiguous range of the record arrays;
+//   * every block holds a copy of all the scene's states and rest positions (active and
+//     fixed vertices) in its shared memory, and the neighbour and incidence records of the
+//     vertices it owns: of each color, the block of rank r owns a chunk of whole slices of
+//     kSlice vertices, whose records are one contiguous range of each record array;
 //   * per color, each block solves its chunk (L lanes per vertex, neighbour states and
 //     records from its own shared memory) and writes every new state into all C copies:
 //     its own, and the other blocks' through distributed shared memory;
@@ -33,32 +33,34 @@ namespace cg = cooperative_groups;
 
 constexpr int kClusterMaxColors = 64;  // colors per scene that the per-block color table holds
 
-// One incidence record in shared memory.
-template <typename R>
-struct RecS;
-template <>
-struct RecS<float> {
-    RecRaw<float> r;
-    __device__ __forceinline__ void from_global(const int4* n, const R4<float>* a, const R4<float>* b, const float*,
-                                                int i) {
-        r.n = n[i];
-        r.a = reinterpret_cast<const float4*>(a)[i];
-        r.b = reinterpret_cast<const float4*>(b)[i];
+// Neighbour states and rest positions from the block's shared copies; the staged neighbour
+// records hold positions in those copies instead of slots.
+template <typename ST>
+struct FetchCluster {
+    const typename ST::U* u;
+    const float4* rest;
+    __device__ __forceinline__ void operator()(int i, typename ST::U& q, float4& X) const {
+        q = ST::nb(u[i]);
+        X = rest[i];
     }
 };
-template <>
-struct RecS<double> {
-    RecRaw<double> r;
-    __device__ __forceinline__ void from_global(const int4* n, const R4<double>* a, const R4<double>* b,
-                                                const double* c, int i) {
-        r.n = n[i];
-        const double2* pa = reinterpret_cast<const double2*>(a + i);
-        const double2* pb = reinterpret_cast<const double2*>(b + i);
-        r.a0 = pa[0];
-        r.a1 = pa[1];
-        r.b0 = pb[0];
-        r.b1 = pb[1];
-        r.c = c[i];
+
+// Vertices of a color of n that one of C blocks owns: whole slices.
+__host__ __device__ __forceinline__ int cluster_chunk(int n, int C) {
+    const int per = (n + C - 1) / C;
+    return (per + kSlice - 1) / kSlice * kSlice;
+}
+
+// The same where only the states fit in shared memory: records and rest positions are read
+// through the caches, and the records' slots are looked up in the copy.
+template <typename ST>
+struct FetchClusterLean {
+    const typename ST::U* u;
+    const float4* rest;
+    int4 sl;
+    __device__ __forceinline__ void operator()(int s, typename ST::U& q, float4& X) const {
+        q = ST::nb(u[s < sl.y ? s - sl.x : (sl.y - sl.x) + (s - sl.z)]);
+        X = __ldg(rest + s);
     }
 };
 
@@ -69,7 +71,10 @@ struct ClusterScenes {
     const int4* scene_slots;   // per scene: active slots [x, y), fixed slots [z, w)
     int32_t nscenes, iterations, friction_start;
     int32_t pos_cap;           // states each block's shared copy holds
-    int32_t rec_cap;           // records each block holds
+    int32_t nbr_cap, inc_cap;  // neighbour and incidence records each block holds
+    int32_t stage_cap;         // staging entries per vertex
+    const int4* ranges;        // per color and rank: its records in the global arrays (colors of all
+                               // scenes, C per color): first and last + 1 NbrRec and IncRec
 };
 
 // A state broadcast from lane src of the warp (every field of the trait's state type).
@@ -85,20 +90,26 @@ __device__ __forceinline__ typename ST::U shfl_state(typename ST::U u, int src) 
     return u;
 }
 
-template <int L, typename ST, typename R>
+// LEAN: only the states in shared memory (nbr_cap and inc_cap 0), for a scene whose records
+// and rest positions do not fit beside them.
+template <int L, bool MULTI, bool LEAN, typename ST, typename R>
 __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> c, ClusterScenes S, int32_t* work) {
     using U = typename ST::U;
+    constexpr int NB = L >= 16 ? 1 : 2;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = int(cluster.block_rank());
     const int C = int(cluster.num_blocks());
     extern __shared__ __align__(16) unsigned char smem[];
     U* spos = reinterpret_cast<U*>(smem);
-    RecS<R>* srec = reinterpret_cast<RecS<R>*>(smem + sizeof(U) * size_t(S.pos_cap));
+    float4* srest = reinterpret_cast<float4*>(smem + sizeof(U) * size_t(S.pos_cap));
+    NbrRec<R>* snbr = reinterpret_cast<NbrRec<R>*>(srest + (LEAN ? 0 : S.pos_cap));
+    IncRec<R>* sinc = reinterpret_cast<IncRec<R>*>(snbr + S.nbr_cap);
+    unsigned char* stage = reinterpret_cast<unsigned char*>(sinc + S.inc_cap);
     __shared__ int s_scene;
-    __shared__ int s_rec_base[kClusterMaxColors + 1];
+    __shared__ int2 s_rec_base[kClusterMaxColors + 1];
     const int groups = int(blockDim.x) / L;
-    const int g = int(threadIdx.x) / L;
-    const int lane = int(threadIdx.x) & (L - 1);
+    const int g = int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
+    const int sub = Lanes<L>::sub();
     for (;;) {
         // rank 0 takes the next scene and hands it to every block of the cluster
         if (rank == 0 && threadIdx.x == 0) {
@@ -113,33 +124,45 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
         const int4 sl = S.scene_slots[sc];
         const int na = sl.y - sl.x;
         auto loc = [&](int s) { return s < sl.y ? s - sl.x : na + (s - sl.z); };
+        const auto fetch = [&] {
+            if constexpr (LEAN) return FetchClusterLean<ST>{spos, P.rest, sl};
+            else return FetchCluster<ST>{spos, srest};
+        }();
+        constexpr int RR = LEAN ? kRecKept : kRecShared;
         // this block's chunk of color ci: [beg, end)
         auto chunk = [&](int ci, int& beg, int& end) {
             const int2 rg = S.colors[ci];
-            const int per = (rg.y - rg.x + C - 1) / C;
+            const int per = cluster_chunk(rg.y - rg.x, C);
             beg = min(rg.y, rg.x + rank * per);
             end = min(rg.y, beg + per);
         };
-        if (threadIdx.x == 0) {
-            int base = 0;
+        // per color, where the chunk's records start in the shared arrays, less their global number
+        if (!LEAN && threadIdx.x == 0) {
+            int2 base = make_int2(0, 0);
             for (int ci = c0; ci < c1; ++ci) {
-                int beg, end;
-                chunk(ci, beg, end);
-                s_rec_base[ci - c0] = base;
-                base += P.inc_ofs[end] - P.inc_ofs[beg];
+                const int4 r = S.ranges[ci * C + rank];
+                s_rec_base[ci - c0] = make_int2(base.x - r.x, base.y - r.z);
+                base.x += r.y - r.x;
+                base.y += r.w - r.z;
             }
-            s_rec_base[c1 - c0] = base;
         }
-        // stage: all the scene's states, this block's records
+        // stage: all the scene's states and rest positions, this block's records
         const int nloc = na + (sl.w - sl.z);
-        for (int i = threadIdx.x; i < nloc; i += blockDim.x) spos[i] = P.u[i < na ? sl.x + i : sl.z + (i - na)];
+        for (int i = threadIdx.x; i < nloc; i += blockDim.x) {
+            const int s = i < na ? sl.x + i : sl.z + (i - na);
+            spos[i] = P.u[s];
+            if (!LEAN) srest[i] = P.rest[s];
+        }
         __syncthreads();
-        for (int ci = c0; ci < c1; ++ci) {
-            int beg, end;
-            chunk(ci, beg, end);
-            const int r0 = P.inc_ofs[beg], nr = P.inc_ofs[end] - r0, b = s_rec_base[ci - c0];
-            for (int i = threadIdx.x; i < nr; i += blockDim.x)
-                srec[b + i].from_global(P.rec_n, P.rec_a, P.rec_b, P.rec_c, r0 + i);
+        for (int ci = c0; !LEAN && ci < c1; ++ci) {
+            const int4 r = S.ranges[ci * C + rank];
+            const int2 sb = s_rec_base[ci - c0];
+            for (int i = r.x + int(threadIdx.x); i < r.y; i += blockDim.x) {
+                NbrRec<R> n = P.nbr[i];
+                n.slot = loc(n.slot);
+                snbr[sb.x + i] = n;
+            }
+            for (int i = r.z + int(threadIdx.x); i < r.w; i += blockDim.x) sinc[sb.y + i] = P.inc[i];
         }
         cluster.sync();  // every copy staged before any block writes into another's
         for (int it = 0; it < S.iterations; ++it) {
@@ -147,45 +170,49 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
             for (int ci = c0; ci < c1; ++ci) {
                 int beg, end;
                 chunk(ci, beg, end);
-                const int rb = s_rec_base[ci - c0], r0 = P.inc_ofs[beg];
+                const int2 sb = LEAN ? make_int2(0, 0) : s_rec_base[ci - c0];
+                const NbrRec<R>* nbr = LEAN ? P.nbr : snbr + sb.x;
+                const IncRec<R>* inc = LEAN ? P.inc : sinc + sb.y;
                 for (int base = beg; base < end; base += groups) {
                     const int v = base + g;
                     const bool valid = v < end;
                     Acc<R> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
                     U uo{};
-                    MeshMat<R> mat;
+                    MeshMat<R> mat{};
+                    float4 Xo = make_float4(0.f, 0.f, 0.f, 0.f);
+                    int4 seg = make_int4(0, 0, 0, 0);
                     if (valid) {
-                        if (lane == 0) prefetch_tail(P, v);
+                        if (sub == 0) prefetch_tail<L>(P, v);
+                        seg = P.vrec[v];
                         mat = P.mats[P.slot_mesh[v]];
                         uo = spos[v - sl.x];
-                        const U uon = ST::nb(uo);
-                        const int e = rb + P.inc_ofs[v + 1] - r0;
-                        for (int r = rb + P.inc_ofs[v] - r0 + lane; r < e; r += L) {
-                            const RecRaw<R>& rec = srec[r].r;
-                            const U q0 = ST::nb(spos[loc(rec.n.x)]), q1 = ST::nb(spos[loc(rec.n.y)]),
-                                    q2 = ST::nb(spos[loc(rec.n.z)]);
-                            R m0[3], m1[3], m2[3];
-                            rec.rows(m0, m1, m2);
-                            R e0[3], e1[3], e2[3];
-                            ST::diff(q0, uon, e0);
-                            ST::diff(q1, uon, e1);
-                            ST::diff(q2, uon, e2);
-                            incidence<R>(e0, e1, e2, m0, m1, m2, mat.mu, mat.lmbd, acc);
-                        }
+                        Xo = LEAN ? __ldg(P.rest + v) : srest[v - sl.x];
                     }
+                    const U uon = ST::nb(uo);
+                    SegRecs<R, NB> rec;
+                    const Stage<32 / L, ST, R> st = warp_stage<L, ST, R>(stage, S.stage_cap);
+                    preload<L, RR>(rec, nbr, inc, seg, sub);
+                    accumulate_segment<L, RR, false, ST>(rec, sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
+                    if constexpr (MULTI)
+                        if (valid)
+                            accumulate_more<L, RR, false, ST>(rec, P, nbr, inc, P.vmore[v], sub, st, fetch, uon, Xo, mat.mu, mat.lmbd,
+                                                       acc);
+                    __syncwarp();
                     reduce_group<L, R>(acc);
                     // lane 0 solves; the group's lanes then write the new state into the C
                     // copies, one remote store each, instead of lane 0 writing all of them
                     U un{};
                     int moved = 0;
-                    if (valid && lane == 0)
-                        moved = vertex_tail<ST, R, false>(P, c, v, uo, mat, acc, friction, nullptr, beg, end, &un) ? 1 : 0;
-                    const int src = int(threadIdx.x) & ~(L - 1) & 31;
+                    if (valid && sub == 0) {
+                        finish_acc(acc, mat.mu, mat.lmbd);
+                        moved = vertex_tail<ST, R, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr, &un) ? 1 : 0;
+                    }
+                    const int src = Lanes<L>::vertex();
                     moved = __shfl_sync(0xffffffffu, moved, src);
                     un = shfl_state<ST>(un, src);
                     if (valid && moved) {
                         const int lv = v - sl.x;
-                        for (int r = lane; r < C; r += L) *cluster.map_shared_rank(&spos[lv], r) = un;
+                        for (int r = sub; r < C; r += L) *cluster.map_shared_rank(&spos[lv], r) = un;
                     }
                 }
                 cluster.sync();  // this color's states in every copy before the next color

@@ -20,6 +20,8 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <thread>
+#include <tuple>
 #include <vector>
 
 #include "../../include/gaia_vbd.h"
@@ -81,28 +83,6 @@ inline int div_up(int64_t a, int64_t b) { return int((a + b - 1) / b); }
 
 }  // namespace
 
-// One incidence record (layout in vbd_kernels.cuh).
-template <typename R>
-void make_record(int4& n, dev::R4<R>& a, dev::R4<R>& b, R* c, const int* nb, double mv[3][3]);
-template <>
-inline void make_record<float>(int4& n, dev::R4<float>& a, dev::R4<float>& b, float*, const int* nb,
-                               double mv[3][3]) {
-    float m2z = float(mv[2][2]);
-    int bits;
-    std::memcpy(&bits, &m2z, 4);
-    n = make_int4(nb[0], nb[1], nb[2], bits);
-    a = dev::R4<float>{float(mv[0][0]), float(mv[0][1]), float(mv[0][2]), float(mv[1][0])};
-    b = dev::R4<float>{float(mv[1][1]), float(mv[1][2]), float(mv[2][0]), float(mv[2][1])};
-}
-template <>
-inline void make_record<double>(int4& n, dev::R4<double>& a, dev::R4<double>& b, double* c, const int* nb,
-                                double mv[3][3]) {
-    n = make_int4(nb[0], nb[1], nb[2], 0);
-    a = dev::R4<double>{mv[0][0], mv[0][1], mv[0][2], mv[1][0]};
-    b = dev::R4<double>{mv[1][1], mv[1][2], mv[2][0], mv[2][1]};
-    *c = mv[2][2];
-}
-
 enum { kSweepMerged = 0, kSweepScenes = 1, kSweepCluster = 2, kSweepGrid = 3 };
 constexpr int kVariantDeep = 4;  // solve variant: k_solve_deep
 constexpr int kVariantGrid = 5;  // solve variant: k_sweep_grid
@@ -146,14 +126,14 @@ class Engine : public EngineBase {
     using S4 = typename ST::U;   // per-vertex displacement state
     using V4 = typename ST::V;   // per-vertex velocity
     using Sc = typename ST::Sc;
-    using R4 = dev::R4<R>;
 
 public:
     // cluster mode: a cluster size whose blocks hold every scene (states and owned records)
     struct ClusterFit {
         int C;
-        int32_t pos_cap, rec_cap;
-        size_t bytes;
+        int32_t pos_cap, nbr_cap, inc_cap;
+        size_t bytes;  // without the staging areas
+        bool lean;     // only the states in shared memory
     };
 
     // mode: kSweepMerged (one launch per merged color and iteration), kSweepScenes (one
@@ -178,7 +158,6 @@ public:
             throw std::runtime_error("blockSize must be a multiple of 32 in [64, 256]");
         use_pdl_ = sc_.p.usePDL;
         small_color_ = sc_.p.smallColorVertices;
-        set_tma_smem_limits();
         variant_fixed_ = sc_.p.solveVariant;
         if (variant_fixed_ != -1 && variant_fixed_ != 0 && variant_fixed_ != 1 && variant_fixed_ != kVariantDeep &&
             variant_fixed_ != kVariantPrefetch && variant_fixed_ != kVariantPipe)
@@ -283,44 +262,7 @@ public:
         for (int m = 0; m < nmesh_; ++m)
             for (int v = 0; v < meshes[m].nv; ++v) slot_mesh_[slot_of_[mesh_off_[m] + v]] = m;
 
-        // incidence records in slot order
-        inc_ofs_.assign(size_t(nactive_) + 1, 0);
-        for (int32_t s = 0; s < nactive_; ++s) {
-            int32_t gi = orig_of_[s];
-            int m = slot_mesh_[s];
-            int v = gi - int32_t(mesh_off_[m]);
-            inc_ofs_[s + 1] = inc_ofs_[s] + (meshes[m].nbr_ofs[v + 1] - meshes[m].nbr_ofs[v]);
-        }
-        ninc_ = inc_ofs_[nactive_];
-        if (int64_t(ninc_) > int64_t(INT32_MAX)) throw std::runtime_error("too many incidences");
-        h_rec_n_.resize(ninc_);
-        h_rec_a_.resize(ninc_);
-        h_rec_b_.resize(ninc_);
-        if (sizeof(R) == 8) h_rec_c_.resize(ninc_);
-        for (int32_t s = 0; s < nactive_; ++s) {
-            int32_t gi = orig_of_[s];
-            int m = slot_mesh_[s];
-            const TetMesh& M = meshes[m];
-            int v = gi - int32_t(mesh_off_[m]);
-            int32_t r = inc_ofs_[s];
-            for (int k = M.nbr_ofs[v]; k < M.nbr_ofs[v + 1]; ++k, ++r) {
-                int t = M.nbr_tet[k], o = M.nbr_order[k];
-                const double* Di = &M.dminv[9 * size_t(t)];
-                int others[3], q = 0;
-                for (int j = 0; j < 4; ++j)
-                    if (j != o) others[q++] = j;
-                if (o & 1) std::swap(others[0], others[1]);  // keeps det[m0;m1;m2] = det(DmInv)
-                double mv[3][3];
-                int nb[3];
-                for (int i = 0; i < 3; ++i) {
-                    int j = others[i];
-                    for (int c = 0; c < 3; ++c)
-                        mv[i][c] = j == 0 ? -(Di[3 * c] + Di[3 * c + 1] + Di[3 * c + 2]) : Di[3 * c + (j - 1)];
-                    nb[i] = slot_of_[mesh_off_[m] + M.tets[4 * size_t(t) + j]];
-                }
-                set_record(r, nb, mv);
-            }
-        }
+        build_records();
         // per-slot state
         h_pos_.resize(nslots_);
         h_vel_.resize(nslots_);
@@ -412,8 +354,262 @@ public:
         c_.spin_limit = p.waitPollLimit >= 0 ? p.waitPollLimit : dev::kMbarSpinLimit;
     }
 
-    void set_record(int32_t r, const int* nb, double mv[3][3]) {
-        make_record<R>(h_rec_n_[r], h_rec_a_[r], h_rec_b_[r], sizeof(R) == 8 ? &h_rec_c_[r] : nullptr, nb, mv);
+    // One-ring and incidence records of the active slots (layout in vbd_kernels.cuh), the host
+    // threads taking contiguous ranges of slices; a color (of the merged sweep, or of one
+    // scene) starts a slice. Neighbours are listed by slot, so that the k-th neighbours of
+    // consecutive vertices of a regular mesh are consecutive too; incidences keep the mesh's
+    // ascending tet order, and a segment closes when the next tet's vertices would take it
+    // past kSegNbrs neighbours.
+    void build_records() {
+        const auto& meshes = sc_.meshes;
+        inc_ofs_.assign(size_t(nactive_) + 1, 0);
+        int64_t total = 0;
+        for (int32_t s = 0; s < nactive_; ++s) {
+            const int m = slot_mesh_[s], v = orig_of_[s] - int32_t(mesh_off_[m]);
+            total += meshes[m].nbr_ofs[v + 1] - meshes[m].nbr_ofs[v];
+            if (total > int64_t(INT32_MAX) / 2) throw std::runtime_error("too many incidences");
+            inc_ofs_[s + 1] = int32_t(total);
+        }
+        ninc_ = int32_t(total);
+        std::vector<int2> slices;  // slot ranges
+        auto cut = [&](int beg, int end) {
+            for (int v = beg; v < end; v += dev::kSlice) slices.push_back(make_int2(v, std::min(end, v + dev::kSlice)));
+        };
+        if (mode_ == kSweepScenes || mode_ == kSweepCluster)
+            for (int2 c : scene_colors_) cut(c.x, c.y);
+        else
+            for (size_t g = 0; g < group_beg_.size(); ++g) cut(group_beg_[g], group_end_[g]);
+        struct Seg {
+            int32_t slot;                // its vertex
+            int4 r;                      // as vrec
+        };
+        struct Part {                    // of one host thread
+            std::vector<dev::NbrRec<R>> nbr;
+            std::vector<dev::IncRec<R>> inc;
+            std::vector<Seg> more;       // further segments
+        };
+        const int nt = std::max(1, std::min<int>(int(std::thread::hardware_concurrency()), int(ninc_ / 65536) + 1));
+        std::vector<Part> part{size_t(nt)};
+        vrec_.assign(size_t(nactive_), make_int4(0, 0, 0, 0));
+        auto range = [&](int k) { return size_t(int64_t(slices.size()) * k / nt); };
+        auto work = [&](int k) {
+            Part& out = part[size_t(k)];
+            std::vector<dev::NbrRec<R>> nbr;
+            std::vector<dev::IncRec<R>> inc;
+            // the lists of one segment into place: every kSlice-th record from the segment's first
+            auto place = [&](int4 seg) {
+                for (int i = 0; i < seg.z; ++i) out.nbr[size_t(seg.x + dev::kSlice * i)] = nbr[size_t(i)];
+                for (int i = 0; i < seg.w; ++i) out.inc[size_t(seg.y + dev::kSlice * i)] = inc[size_t(i)];
+            };
+            std::vector<std::vector<dev::NbrRec<R>>> ln(dev::kSlice);
+            std::vector<std::vector<dev::IncRec<R>>> li(dev::kSlice);
+            for (size_t sl = range(k); sl < range(k + 1); ++sl) {
+                const int2 rg = slices[sl];
+                size_t mn = 0, mi = 0;
+                std::vector<Seg> extra;
+                std::vector<std::pair<std::vector<dev::NbrRec<R>>, std::vector<dev::IncRec<R>>>> extra_lists;
+                for (int32_t s = rg.x; s < rg.y; ++s) {
+                    bool first = true;
+                    segments_of(s, nbr, inc, [&] {
+                        if (first) {
+                            ln[size_t(s - rg.x)] = nbr;
+                            li[size_t(s - rg.x)] = inc;
+                            mn = std::max(mn, nbr.size());
+                            mi = std::max(mi, inc.size());
+                        } else {
+                            extra.push_back({s, make_int4(0, 0, int(nbr.size()), int(inc.size()))});
+                            extra_lists.emplace_back(nbr, inc);
+                        }
+                        first = false;
+                    });
+                }
+                const size_t nb = out.nbr.size(), ib = out.inc.size();
+                size_t en = 0, ei = 0;
+                for (auto& e : extra_lists) {
+                    en += e.first.size();
+                    ei += e.second.size();
+                }
+                out.nbr.resize(nb + dev::kSlice * (mn + en));
+                out.inc.resize(ib + dev::kSlice * (mi + ei));
+                for (int32_t s = rg.x; s < rg.y; ++s) {
+                    nbr = ln[size_t(s - rg.x)];
+                    inc = li[size_t(s - rg.x)];
+                    vrec_[size_t(s)] = make_int4(int(nb) + (s - rg.x), int(ib) + (s - rg.x), int(nbr.size()), int(inc.size()));
+                    place(vrec_[size_t(s)]);
+                }
+                int n1 = int(nb + dev::kSlice * mn), i1 = int(ib + dev::kSlice * mi);
+                for (size_t e = 0; e < extra.size(); ++e) {
+                    nbr = extra_lists[e].first;
+                    inc = extra_lists[e].second;
+                    extra[e].r.x = n1;
+                    extra[e].r.y = i1;
+                    place(extra[e].r);
+                    n1 += dev::kSlice * int(nbr.size());
+                    i1 += dev::kSlice * int(inc.size());
+                    out.more.push_back(extra[e]);
+                }
+            }
+        };
+        std::vector<std::thread> th;
+        for (int k = 1; k < nt; ++k) th.emplace_back(work, k);
+        work(0);
+        for (auto& t : th) t.join();
+        size_t nn = 0, ni = 0;
+        for (auto& q : part) {
+            nn += q.nbr.size();
+            ni += q.inc.size();
+        }
+        if (std::max(nn, ni) > size_t(INT32_MAX) / 2) throw std::runtime_error("too many incidences");
+        // the parts end to end, padded for the copies of whole slices that run past the last list
+        max_nbr_all_ = max_inc_all_ = 2;
+        h_nbr_.clear();
+        h_inc_.clear();
+        h_nbr_.reserve(nn + size_t(dev::kSlice) * 1024);
+        h_inc_.reserve(ni + size_t(dev::kSlice) * 1024);
+        segs_.clear();
+        std::vector<Seg> more;
+        for (int k = 0; k < nt; ++k) {
+            Part& q = part[size_t(k)];
+            const int n0 = int(h_nbr_.size()), i0 = int(h_inc_.size());
+            if (range(k) < range(k + 1))
+                for (int32_t s = slices[range(k)].x; s < slices[range(k + 1) - 1].y; ++s) {
+                    vrec_[size_t(s)].x += n0;
+                    vrec_[size_t(s)].y += i0;
+                }
+            for (Seg& e : q.more) {
+                e.r.x += n0;
+                e.r.y += i0;
+                more.push_back(e);
+            }
+            h_nbr_.insert(h_nbr_.end(), q.nbr.begin(), q.nbr.end());
+            h_inc_.insert(h_inc_.end(), q.inc.begin(), q.inc.end());
+        }
+        nbr_end_ = int(h_nbr_.size());
+        inc_end_ = int(h_inc_.size());
+        for (const int4& r : vrec_) {
+            max_nbr_all_ = std::max(max_nbr_all_, (r.z + 1) & ~1);
+            max_inc_all_ = std::max(max_inc_all_, r.w);
+        }
+        for (const Seg& e : more) max_nbr_all_ = std::max(max_nbr_all_, (e.r.z + 1) & ~1);
+        h_nbr_.resize(h_nbr_.size() + size_t(dev::kSlice) * max_nbr_all_, dev::NbrRec<R>{});
+        h_inc_.resize(h_inc_.size() + size_t(dev::kSlice) * max_inc_all_, dev::IncRec<R>{});
+        multi_seg_ = !more.empty();
+        vmore_.clear();
+        if (multi_seg_) {
+            vmore_.assign(size_t(nactive_), make_int2(0, 0));
+            std::stable_sort(more.begin(), more.end(), [](const Seg& a, const Seg& b) { return a.slot < b.slot; });
+            for (size_t i = 0; i < more.size(); ++i) {
+                int2& q = vmore_[size_t(more[i].slot)];
+                if (q.y == 0) q.x = int(i);
+                q.y = int(i) + 1;
+                segs_.push_back(more[i].r);
+            }
+        }
+    }
+
+    // The segments of slot s one after another in nbr and inc (done() is called after each).
+    template <typename Fn>
+    void segments_of(int32_t s, std::vector<dev::NbrRec<R>>& nbr, std::vector<dev::IncRec<R>>& inc, Fn&& done) const {
+        const int m = slot_mesh_[s];
+        const TetMesh& M = sc_.meshes[m];
+        const int v = orig_of_[s] - int32_t(mesh_off_[m]);
+        int32_t slots[dev::kSegNbrs];
+        double K[dev::kSegNbrs];
+        int n = 0;
+        inc.clear();
+        auto close = [&] {
+            // by slot: rank of each neighbour, records in that order, positions renamed
+            int order[dev::kSegNbrs];
+            uint32_t rank[dev::kSegNbrs];
+            for (int i = 0; i < n; ++i) order[i] = i;
+            std::sort(order, order + n, [&](int a, int b) { return slots[a] < slots[b]; });
+            nbr.resize(size_t(n));
+            for (int i = 0; i < n; ++i) {
+                rank[order[i]] = uint32_t(i);
+                nbr[size_t(i)] = dev::NbrRec<R>{};
+                nbr[size_t(i)].slot = slots[order[i]];
+                nbr[size_t(i)].k = R(K[order[i]]);
+            }
+            for (auto& q : inc) q.idx = rank[q.idx & 255u] | rank[(q.idx >> 8) & 255u] << 8 | rank[(q.idx >> 16) & 255u] << 16;
+            done();
+            n = 0;
+            inc.clear();
+        };
+        for (int q = M.nbr_ofs[v]; q < M.nbr_ofs[v + 1]; ++q) {
+            const int t = M.nbr_tet[q], o = M.nbr_order[q];
+            const double* Di = &M.dminv[9 * size_t(t)];
+            double row[4][3];
+            for (int c = 0; c < 3; ++c) {
+                row[0][c] = -(Di[3 * c] + Di[3 * c + 1] + Di[3 * c + 2]);
+                for (int j = 1; j < 4; ++j) row[j][c] = Di[3 * c + (j - 1)];
+            }
+            int others[3], w = 0;
+            for (int j = 0; j < 4; ++j)
+                if (j != o) others[w++] = j;
+            if (o & 1) std::swap(others[0], others[1]);  // keeps det of the rows = det(DmInv)
+            int32_t sl[3];
+            int at[3], fresh = 0;
+            auto find = [&](int32_t x) {
+                for (int i = 0; i < n; ++i)
+                    if (slots[i] == x) return i;
+                return -1;
+            };
+            for (int i = 0; i < 3; ++i) {
+                sl[i] = slot_of_[mesh_off_[m] + M.tets[4 * size_t(t) + others[i]]];
+                fresh += find(sl[i]) < 0 ? 1 : 0;
+            }
+            if (n + fresh > dev::kSegNbrs) close();
+            for (int i = 0; i < 3; ++i) {
+                at[i] = find(sl[i]);
+                if (at[i] < 0) {
+                    at[i] = n;
+                    slots[n] = sl[i];
+                    K[n++] = 0.0;
+                }
+                const double* a = row[o];
+                const double* b = row[others[i]];
+                K[at[i]] += M.vol[t] * (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]);
+            }
+            dev::IncRec<R> rec{};
+            rec.idx = uint32_t(at[0]) | uint32_t(at[1]) << 8 | uint32_t(at[2]) << 16;
+            rec.w = R(1.0 / (6.0 * M.vol[t]));
+            inc.push_back(rec);
+        }
+        close();
+    }
+
+    // Longest lists in the slot range [beg, end): neighbours (even: the staging entries per
+    // vertex) and incidences.
+    int2 max_lists(int beg, int end) {
+        if (multi_seg_) return make_int2(max_nbr_all_, max_inc_all_);
+        const auto key = std::make_pair(beg, end);
+        auto it = lists_cache_.find(key);
+        if (it != lists_cache_.end()) return it->second;
+        int2 m = make_int2(2, 1);
+        for (int v = beg; v < end; ++v) {
+            m.x = std::max(m.x, (vrec_[size_t(v)].z + 1) & ~1);
+            m.y = std::max(m.y, vrec_[size_t(v)].w);
+        }
+        return lists_cache_[key] = m;
+    }
+    // Bytes of the staging areas of a block of B threads.
+    static size_t stage_bytes(int cap, int L, int B) {
+        return size_t(B / L) * size_t(cap) * (16 * dev::Stage<1, ST, R>::kParts);
+    }
+    // Fewest lanes per vertex, at least L, whose staging fits the shared memory of a block
+    // (32 where a vertex has several segments: those kernels take one vertex per warp).
+    int fit_lanes(int L, int B, int beg, int end) {
+        if (multi_seg_) return 32;
+        while (L < 32 && stage_bytes(max_lists(beg, end).x, L, B) > kTmaSmemMax) L *= 2;
+        return L;
+    }
+    // The limit of a kernel's dynamic shared memory, raised once for every launch: a captured
+    // launch must not depend on what a later one asks for. The 48 KB that need no raise hold
+    // the kernel's static shared memory too.
+    template <typename K>
+    static void allow_smem(K kern, size_t bytes) {
+        if (bytes > 40 * 1024)
+            GAIA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
     }
 
     void upload() {
@@ -425,10 +621,11 @@ public:
         d_xprev_.upload(h_pos_, &bytes_, st_);
         d_vprev_.upload(h_vel_, &bytes_, st_);
         d_inc_ofs_.upload(inc_ofs_, &bytes_, st_);
-        d_rec_n_.upload(h_rec_n_, &bytes_, st_);
-        d_rec_a_.upload(h_rec_a_, &bytes_, st_);
-        d_rec_b_.upload(h_rec_b_, &bytes_, st_);
-        d_rec_c_.upload(h_rec_c_, &bytes_, st_);
+        d_vrec_.upload(vrec_, &bytes_, st_);
+        d_vmore_.upload(vmore_, &bytes_, st_);
+        d_segs_.upload(segs_, &bytes_, st_);
+        d_nbr_.upload(h_nbr_, &bytes_, st_);
+        d_inc_.upload(h_inc_, &bytes_, st_);
         d_slot_mesh_.upload(slot_mesh_, &bytes_, st_);
         d_mats_.upload(h_mats_, &bytes_, st_);
         d_slot_of_.upload(slot_of_, &bytes_, st_);
@@ -450,10 +647,8 @@ public:
         d_probe_.alloc(12, &bytes_);
         GAIA_CUDA(cudaStreamSynchronize(st_));
         // keep host copies small: records are device-only from here on
-        std::vector<int4>().swap(h_rec_n_);
-        std::vector<R4>().swap(h_rec_a_);
-        std::vector<R4>().swap(h_rec_b_);
-        std::vector<R>().swap(h_rec_c_);
+        std::vector<dev::NbrRec<R>>().swap(h_nbr_);
+        std::vector<dev::IncRec<R>>().swap(h_inc_);
     }
 
     dev::Ptrs<ST, R> ptrs() const {
@@ -464,11 +659,11 @@ public:
         P.xprev = d_xprev_.p;
         P.vel = d_vel_.p;
         P.vprev = d_vprev_.p;
-        P.inc_ofs = d_inc_ofs_.p;
-        P.rec_n = d_rec_n_.p;
-        P.rec_a = d_rec_a_.p;
-        P.rec_b = d_rec_b_.p;
-        P.rec_c = d_rec_c_.p;
+        P.vrec = d_vrec_.p;
+        P.vmore = d_vmore_.p;
+        P.segs = d_segs_.p;
+        P.nbr = d_nbr_.p;
+        P.inc = d_inc_.p;
         P.slot_mesh = d_slot_mesh_.p;
         P.mats = d_mats_.p;
         P.counters = d_counters_.p;
@@ -619,28 +814,60 @@ public:
     // Launch of one color's solve. pdl: launched as a programmatic dependent of
     // the previous kernel in the stream (its static-data prologue overlaps that
     // kernel's tail; k_solve waits on griddepcontrol before reading positions).
-    template <bool PROBE, int L>
-    void launch_solve_l(int grid, int B, int beg, int end, int friction, double* probe, bool pdl, int pf = 0) {
+    template <bool PROBE, bool DEEP, int L, bool MULTI = false>
+    void launch_solve_l(int B, int beg, int end, int friction, double* probe, bool pdl, bool prefetch) {
+        const int cap = max_lists(beg, end).x;
+        const size_t smem = stage_bytes(cap, L, B);
+        auto kern = dev::k_solve<L, ST, R, PROBE, DEEP, MULTI>;
+        allow_smem(kern, smem);
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid);
+        cfg.gridDim = dim3(div_up(int64_t(end - beg) * L, B));
         cfg.blockDim = dim3(B);
-        cfg.dynamicSmemBytes = 0;
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st_;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = pdl ? attr : nullptr;
         cfg.numAttrs = pdl ? 1 : 0;
-        GAIA_CUDA(cudaLaunchKernelEx(&cfg, dev::k_solve<L, ST, R, PROBE>, ptrs(), c_, beg, end, friction, probe, pf));
+        // the prefetching variant fetches for the warps one resident wave ahead
+        const int pf = prefetch ? std::max(1, blocks_per_sm(kern, B, smem)) * sm_count() * (B / 32) : 0;
+        GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, friction, probe, pf, cap));
     }
 
-    // Largest record count of any block of vpb consecutive vertices in [beg, end).
-    int max_records(int beg, int end, int vpb) {
+    template <typename K>
+    int blocks_per_sm(K kern, int B, size_t smem) {
+        const auto key = std::make_tuple(reinterpret_cast<const void*>(kern), B, smem);
+        auto it = occ_cache_.find(key);
+        if (it != occ_cache_.end()) return it->second;
+        int per_sm = 0;
+        GAIA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, B, smem));
+        return occ_cache_[key] = per_sm;
+    }
+
+    int sm_count() {
+        if (sms_ == 0) {
+            int dev = 0;
+            GAIA_CUDA(cudaGetDevice(&dev));
+            GAIA_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
+        }
+        return sms_;
+    }
+
+    // Largest neighbour and incidence record ranges of any block of vpb consecutive vertices
+    // in [beg, end), as rec_tile (vbd_kernels.cuh) takes them.
+    int2 max_records(int beg, int end, int vpb) {
         auto key = std::make_pair(beg, vpb);
         auto it = maxrec_cache_.find(key);
         if (it != maxrec_cache_.end()) return it->second;
-        int m = 0;
-        for (int v0 = beg; v0 < end; v0 += vpb) m = std::max(m, inc_ofs_[std::min(end, v0 + vpb)] - inc_ofs_[v0]);
+        const int2 lists = max_lists(beg, end);
+        int2 m = make_int2(0, 0);
+        for (int v0 = beg; v0 < end; v0 += vpb) {
+            const int4 r0 = vrec_[size_t(v0)], r1 = vrec_[size_t(std::min(end, v0 + vpb) - 1)];
+            const int mask = ~(dev::kSlice - 1);
+            m.x = std::max(m.x, (r1.x & mask) + dev::kSlice * lists.x - (r0.x & mask));
+            m.y = std::max(m.y, (r1.y & mask) + dev::kSlice * lists.y - (r0.y & mask));
+        }
         maxrec_cache_[key] = m;
         return m;
     }
@@ -651,9 +878,12 @@ public:
             return false;
         } else {
             const int vpb = B / L;
-            const int mr = max_records(beg, end, vpb);
-            const size_t smem = 16 + 48 * size_t(mr);
+            const int2 mr = max_records(beg, end, vpb);
+            const int2 lists = max_lists(beg, end);
+            const size_t smem = 16 + 8 * (size_t(mr.x) + size_t(mr.y)) + stage_bytes(lists.x, L, B);
             if (smem > kTmaSmemMax) return false;
+            auto kern = dev::k_solve_tma<L, ST>;
+            allow_smem(kern, smem);
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(div_up(end - beg, vpb));
             cfg.blockDim = dim3(B);
@@ -664,7 +894,7 @@ public:
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = pdl ? attr : nullptr;
             cfg.numAttrs = pdl ? 1 : 0;
-            GAIA_CUDA(cudaLaunchKernelEx(&cfg, dev::k_solve_tma<L, ST>, ptrs(), c_, beg, end, friction, mr));
+            GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, friction, lists.x, lists.y, mr.x, mr.y));
             return true;
         }
     }
@@ -676,26 +906,17 @@ public:
             return false;
         } else {
             const int vpt = B / L;
-            const int mr = max_records(beg, end, vpt);
-            const size_t smem = 16 + 2 * 48 * size_t(mr);
+            const int2 mr = max_records(beg, end, vpt);
+            const int2 lists = max_lists(beg, end);
+            const size_t smem = 16 + 2 * 8 * (size_t(mr.x) + size_t(mr.y)) + stage_bytes(lists.x, L, B);
             if (smem > kTmaSmemMax) return false;
             auto kern = dev::k_solve_pipe<L, ST>;
-            const auto key = std::make_pair(L * 100000 + B, int(smem));
-            int per_sm = 0;
-            auto it = pipe_occ_.find(key);
-            if (it != pipe_occ_.end()) {
-                per_sm = it->second;
-            } else {
-                GAIA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, B, smem));
-                pipe_occ_[key] = per_sm;
-            }
+            allow_smem(kern, smem);
+            const int per_sm = blocks_per_sm(kern, B, smem);
             if (per_sm < 1) return false;
-            int dev = 0, sms = 0;
-            GAIA_CUDA(cudaGetDevice(&dev));
-            GAIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             const int ntiles = div_up(end - beg, vpt);
             cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(unsigned(std::min(ntiles, per_sm * sms)));
+            cfg.gridDim = dim3(unsigned(std::min(ntiles, per_sm * sm_count())));
             cfg.blockDim = dim3(B);
             cfg.dynamicSmemBytes = smem;
             cfg.stream = st_;
@@ -704,7 +925,7 @@ public:
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = pdl ? attr : nullptr;
             cfg.numAttrs = pdl ? 1 : 0;
-            GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, friction, mr));
+            GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, friction, lists.x, lists.y, mr.x, mr.y));
             return true;
         }
     }
@@ -730,81 +951,34 @@ public:
         }
     }
 
-    void set_tma_smem_limits() {
-        if constexpr (sizeof(R) == 4) {
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_tma<2, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_tma<4, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_tma<8, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_tma<16, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_tma<32, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_pipe<2, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_pipe<4, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_pipe<8, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_pipe<16, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
-            GAIA_CUDA(cudaFuncSetAttribute(dev::k_solve_pipe<32, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmaSmemMax)));
+    template <bool PROBE, bool DEEP>
+    void launch_solve_reg(int L, int B, int beg, int end, int friction, double* probe, bool pdl, bool prefetch) {
+        B = std::min(B, 256);  // the probe of an engine whose schedule runs larger blocks
+        if (multi_seg_) {
+            launch_solve_l<PROBE, false, 32, true>(B, beg, end, friction, probe, pdl, prefetch);
+            return;
         }
-    }
-
-    template <int L>
-    void launch_solve_deep_l(int grid, int B, int beg, int end, int friction, bool pdl) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(B);
-        cfg.stream = st_;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = pdl ? attr : nullptr;
-        cfg.numAttrs = pdl ? 1 : 0;
-        GAIA_CUDA(cudaLaunchKernelEx(&cfg, dev::k_solve_deep<L, ST, R>, ptrs(), c_, beg, end, friction));
+        switch (fit_lanes(L, B, beg, end)) {
+            case 2: launch_solve_l<PROBE, DEEP, 2>(B, beg, end, friction, probe, pdl, prefetch); break;
+            case 4: launch_solve_l<PROBE, DEEP, 4>(B, beg, end, friction, probe, pdl, prefetch); break;
+            case 8: launch_solve_l<PROBE, DEEP, 8>(B, beg, end, friction, probe, pdl, prefetch); break;
+            case 16: launch_solve_l<PROBE, false, 16>(B, beg, end, friction, probe, pdl, prefetch); break;
+            default: launch_solve_l<PROBE, false, 32>(B, beg, end, friction, probe, pdl, prefetch); break;
+        }
     }
 
     template <bool PROBE>
     void launch_solve(int L, int B, int beg, int end, int friction, double* probe, bool pdl = false,
                       int variant = 0) {
         if (end <= beg) return;
-        if (!PROBE && variant == 1 && launch_solve_tma(L, B, beg, end, friction, pdl)) return;
-        if (!PROBE && variant == kVariantPipe && launch_solve_pipe(L, B, beg, end, friction, pdl)) return;
-        if (!PROBE && variant == kVariantDeep) {
-            const int grid = div_up(int64_t(end - beg) * L, B);
-            switch (L) {
-                case 2: launch_solve_deep_l<2>(grid, B, beg, end, friction, pdl); break;
-                case 4: launch_solve_deep_l<4>(grid, B, beg, end, friction, pdl); break;
-                case 8: launch_solve_deep_l<8>(grid, B, beg, end, friction, pdl); break;
-                case 16: launch_solve_deep_l<16>(grid, B, beg, end, friction, pdl); break;
-                default: launch_solve_deep_l<32>(grid, B, beg, end, friction, pdl); break;
-            }
-            return;
+        if constexpr (PROBE) {
+            launch_solve_reg<true, false>(L, B, beg, end, friction, probe, pdl, false);
+        } else {
+            if (variant == 1 && !multi_seg_ && launch_solve_tma(L, B, beg, end, friction, pdl)) return;
+            if (variant == kVariantPipe && !multi_seg_ && launch_solve_pipe(L, B, beg, end, friction, pdl)) return;
+            if (variant == kVariantDeep) launch_solve_reg<false, true>(L, B, beg, end, friction, probe, pdl, false);
+            else launch_solve_reg<false, false>(L, B, beg, end, friction, probe, pdl, variant == kVariantPrefetch);
         }
-        int grid = div_up(int64_t(end - beg) * L, B);
-        const bool pf = !PROBE && variant == kVariantPrefetch;
-        switch (L) {
-            case 2: launch_solve_l<PROBE, 2>(grid, B, beg, end, friction, probe, pdl, pf ? wave_blocks<2>(B) : 0); break;
-            case 4: launch_solve_l<PROBE, 4>(grid, B, beg, end, friction, probe, pdl, pf ? wave_blocks<4>(B) : 0); break;
-            case 8: launch_solve_l<PROBE, 8>(grid, B, beg, end, friction, probe, pdl, pf ? wave_blocks<8>(B) : 0); break;
-            case 16:
-                launch_solve_l<PROBE, 16>(grid, B, beg, end, friction, probe, pdl, pf ? wave_blocks<16>(B) : 0);
-                break;
-            default:
-                launch_solve_l<PROBE, 32>(grid, B, beg, end, friction, probe, pdl, pf ? wave_blocks<32>(B) : 0);
-                break;
-        }
-    }
-
-    // Blocks of k_solve<L> resident on the whole device at once (one wave): the distance at
-    // which the prefetching variant fetches records ahead.
-    template <int L>
-    int wave_blocks(int B) {
-        const auto key = std::make_pair(L, B);
-        auto it = wave_cache_.find(key);
-        if (it != wave_cache_.end()) return it->second;
-        int per_sm = 0, dev = 0, sms = 0;
-        GAIA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_solve<L, ST, R, false>, B, 0));
-        GAIA_CUDA(cudaGetDevice(&dev));
-        GAIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const int w = std::max(1, per_sm * sms);
-        wave_cache_[key] = w;
-        return w;
     }
 
     // Launch configuration of every merged color. Colors differ in size and in
@@ -1056,18 +1230,15 @@ public:
         save.alloc(nslots_, nullptr);
         GAIA_CUDA(cudaMemcpyAsync(save.p, d_pos_.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
         const int Ls[] = {2, 4, 8, 16, 32};
-        // blocks of 64 too for the tile pipeline, whose two tile buffers bound the blocks per SM
-        const std::vector<int> Bs = {128, 256}, Bs_pipe = {64, 128, 256};
-        // kernel variants: 0 register-pipelined, 1 TMA-staged (FP32 compute only), 4 deeper
-        // register pipeline, 6 register-pipelined with the records of the block one resident
-        // wave ahead bulk-prefetched into L2 (FP32 compute only), 7 double-buffered TMA tiles
-        // on a persistent grid (FP32 compute only)
+        const std::vector<int> Bs = {64, 128, 256};
+        // kernel variants: 0 register gathers, 4 asynchronous one-ring copies, 6 as 0 with the data of
+        // the warps one resident wave ahead prefetched into L2 (FP32 compute only). The TMA
+        // variants 1 and 7 run on request only: with 8-byte records a block's range is a few KB,
+        // and waiting for all of it costs more than the loads it saves (100^3 twist, FP32, best
+        // shape: 47.3 us per color against 43.3 us for variant 0 and 41.2 us for 6).
         std::vector<int> variants = {0, kVariantDeep};
-        if (sizeof(R) == 4) {
-            variants.push_back(1);
-            variants.push_back(kVariantPrefetch);
-            variants.push_back(kVariantPipe);
-        }
+        if (sizeof(R) == 4) variants.push_back(kVariantPrefetch);
+        if (variant_fixed_ >= 0) variants = {variant_fixed_};
         const int reps = 4;
         ccfg_.assign(group_beg_.size(), ColorCfg{});
         double total = 0.0;
@@ -1076,12 +1247,21 @@ public:
             if (end <= beg) continue;
             ColorCfg best;
             best.ms = 1e30f;
+            // A color of up to kLatencyColor vertices is one chain of loads and arithmetic, which a
+            // warp per vertex makes shortest; its time apart from the chain of launches is the
+            // launch itself (4.7 us whatever the shape), so timing it alone picks at random. 10^3
+            // drop, 100 vertices per color, FP32: 32 lanes 2.6 us per color in the chain, 16 lanes
+            // 2.8-3.1 us, 8 lanes 3.4-3.7 us; and one shape for all small colors keeps its code in
+            // the instruction cache from launch to launch.
+            const bool chain = sizeof(R) == 4 && end - beg <= kLatencyColor && variant_fixed_ < 0;
             for (int var : variants) {
-                if (variant_fixed_ >= 0 && var != variant_fixed_) continue;
+                if (chain && var != 0) continue;
                 for (int L : Ls) {
                     if (lanes_ && L != lanes_) continue;
-                    for (int B : var == kVariantPipe ? Bs_pipe : Bs) {
+                    if (chain && !lanes_ && L != 32) continue;
+                    for (int B : Bs) {
                         if (block_ && B != block_) continue;
+                        if (chain && !block_ && B != 128) continue;
                         launch_solve<false>(L, B, beg, end, 1, nullptr, false, var);  // warm-up
                         GAIA_CUDA(cudaEventRecord(ev_a_, st_));
                         for (int r = 0; r < reps; ++r) launch_solve<false>(L, B, beg, end, 1, nullptr, false, var);
@@ -1141,28 +1321,35 @@ public:
         GAIA_CUDA(cudaStreamSynchronize(st_));
     }
 
-    template <int L, int MAXB>
+    template <int L, int MAXB, bool MULTI>
     void launch_scenes_lb(int B) {
-        auto kern = dev::k_sweep_scenes<L, ST, R, MAXB>;
-        int per_sm = 0;
-        GAIA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, B, 0));
+        auto kern = dev::k_sweep_scenes<L, MULTI, ST, R, MAXB>;
+        const int cap = max_nbr_all_;
+        const size_t smem = stage_bytes(cap, L, B);
+        allow_smem(kern, smem);
+        const int per_sm = blocks_per_sm(kern, B, smem);
         const int grid = std::max(1, std::min(nscenes_, std::max(per_sm, 1) * num_sms_));
-        kern<<<grid, B, 0, st_>>>(ptrs(), c_, d_scene_colors_.p, d_scene_ofs_.p, d_scene_order_.p, nscenes_,
-                                  sc_.p.iterations, sc_.p.frictionStartIter, d_scene_work_.p);
+        kern<<<grid, B, smem, st_>>>(ptrs(), c_, d_scene_colors_.p, d_scene_ofs_.p, d_scene_order_.p, nscenes_,
+                                     sc_.p.iterations, sc_.p.frictionStartIter, d_scene_work_.p, cap);
         GAIA_CUDA(cudaGetLastError());
     }
 
-    template <int L>
+    template <int L, bool MULTI = false>
     void launch_scenes_l(int B) {
-        if (B <= 256) launch_scenes_lb<L, 256>(B);
-        else launch_scenes_lb<L, 1024>(B);
+        if (B <= 256) launch_scenes_lb<L, 256, MULTI>(B);
+        else launch_scenes_lb<L, 1024, MULTI>(B);
     }
 
     // One substep's iterations: reset the work counter, one persistent launch.
     void enqueue_scenes_sweep(int L, int B) {
         if (nscenes_ == 0 || sc_.p.iterations == 0) return;
         GAIA_CUDA(cudaMemsetAsync(d_scene_work_.p, 0, sizeof(int32_t), st_));
-        switch (L) {
+        while (B > 64 && stage_bytes(max_nbr_all_, 32, B) > kTmaSmemMax) B /= 2;
+        if (multi_seg_) {
+            launch_scenes_l<32, true>(B);
+            return;
+        }
+        switch (fit_lanes(L, B, 0, nactive_)) {
             case 2: launch_scenes_l<2>(B); break;
             case 4: launch_scenes_l<4>(B); break;
             case 8: launch_scenes_l<8>(B); break;
@@ -1231,26 +1418,41 @@ public:
         const size_t budget = size_t(std::max(0, smem_optin - 4096));  // static shared memory and slack
         cluster_fits_.clear();
         for (int C : {2, 4, 8, 16}) {
-            int64_t pos_cap = 0, rec_cap = 0;
+            int64_t pos_cap = 0, nbr_cap = 0, inc_cap = 0;
             bool ok = true;
+            const std::vector<int4> rg = cluster_ranges(C);
             for (int m = 0; m < nmesh_ && ok; ++m) {
                 const int4 sl = slots[size_t(m)];
                 pos_cap = std::max<int64_t>(pos_cap, int64_t(sl.y - sl.x) + (sl.w - sl.z));
                 if (scene_ofs_[m + 1] - scene_ofs_[m] > dev::kClusterMaxColors) ok = false;
-                std::vector<int64_t> per_rank(size_t(C), 0);
-                for (int32_t ci = scene_ofs_[m]; ci < scene_ofs_[m + 1]; ++ci) {
-                    const int2 rg = scene_colors_[ci];
-                    const int per = (rg.y - rg.x + C - 1) / C;
-                    for (int r = 0; r < C; ++r) {
-                        const int beg = std::min(rg.y, rg.x + r * per), end = std::min(rg.y, beg + per);
-                        per_rank[size_t(r)] += inc_ofs_[end] - inc_ofs_[beg];
+                for (int r = 0; r < C; ++r) {
+                    int64_t nbr = 0, inc = 0;
+                    for (int32_t ci = scene_ofs_[m]; ci < scene_ofs_[m + 1]; ++ci) {
+                        const int4 q = rg[size_t(ci) * C + r];
+                        nbr += q.y - q.x;
+                        inc += q.w - q.z;
                     }
+                    nbr_cap = std::max(nbr_cap, nbr);
+                    inc_cap = std::max(inc_cap, inc);
                 }
-                for (int64_t x : per_rank) rec_cap = std::max(rec_cap, x);
             }
-            const size_t bytes = sizeof(S4) * size_t(pos_cap) + sizeof(dev::RecS<R>) * size_t(rec_cap);
-            if (ok && bytes <= budget) cluster_fits_.push_back({C, int32_t(pos_cap), int32_t(rec_cap), bytes});
+            nbr_cap = (nbr_cap + 1) & ~int64_t(1);
+            inc_cap = (inc_cap + 1) & ~int64_t(1);
+            // states, rest positions and records; the staging areas come on top (per lanes and block)
+            const size_t min_stage = stage_bytes(max_nbr_all_, 32, 64);
+            const size_t lean = sizeof(S4) * size_t(pos_cap);
+            const size_t bytes = lean + sizeof(float4) * size_t(pos_cap) + sizeof(dev::NbrRec<R>) * size_t(nbr_cap) +
+                                 sizeof(dev::IncRec<R>) * size_t(inc_cap);
+            // an explicit "cluster" keeps the limit it is documented with: the states and 48 bytes
+            // (FP64: 96) per owned incidence in each block
+            if (sc_.p.sweepMode == "cluster" && lean + (sizeof(R) == 8 ? 96 : 48) * size_t(cluster_incidences(C)) > budget)
+                ok = false;
+            if (ok && bytes + min_stage <= budget)
+                cluster_fits_.push_back({C, int32_t(pos_cap), int32_t(nbr_cap), int32_t(inc_cap), bytes, false});
+            else if (ok && sc_.p.sweepMode == "cluster" && lean + min_stage <= budget)
+                cluster_fits_.push_back({C, int32_t(pos_cap), 0, 0, lean, true});
         }
+        cluster_budget_ = budget;
         if (cluster_fits_.empty())
             throw std::runtime_error("sweepMode \"cluster\" is not supported: a scene does not fit in the shared "
                                      "memory of a 16-block cluster");
@@ -1259,7 +1461,53 @@ public:
                                      std::to_string(sc_.p.clusterSize) + ": a scene does not fit in the shared "
                                      "memory of a cluster of that many blocks");
         d_scene_slots_.upload(slots, &bytes_, st_);
+        std::vector<std::vector<int4>> ranges;
+        for (auto& f : cluster_fits_) ranges.push_back(cluster_ranges(f.C));
+        for (size_t i = 0; i < ranges.size(); ++i) {
+            auto& buf = cluster_range_bufs_[cluster_fits_[i].C];
+            buf.reset(new DevBuf<int4>());
+            buf->upload(ranges[i], &bytes_, st_);
+        }
         GAIA_CUDA(cudaStreamSynchronize(st_));
+    }
+
+    // Incidences of the fullest block of a cluster of C blocks when each color's vertices are
+    // dealt out evenly.
+    int64_t cluster_incidences(int C) const {
+        int64_t most = 0;
+        for (int m = 0; m < nmesh_; ++m) {
+            std::vector<int64_t> per_rank(size_t(C), 0);
+            for (int32_t ci = scene_ofs_[m]; ci < scene_ofs_[m + 1]; ++ci) {
+                const int2 rg = scene_colors_[ci];
+                const int per = (rg.y - rg.x + C - 1) / C;
+                for (int r = 0; r < C; ++r) {
+                    const int beg = std::min(rg.y, rg.x + r * per), end = std::min(rg.y, beg + per);
+                    per_rank[size_t(r)] += inc_ofs_[end] - inc_ofs_[beg];
+                }
+            }
+            for (int64_t x : per_rank) most = std::max(most, x);
+        }
+        return most;
+    }
+
+    // Records of every color's chunk of every rank in a cluster of C blocks (C per color): the
+    // chunks are whole slices, so a chunk's records end where the next slice's begin.
+    std::vector<int4> cluster_ranges(int C) const {
+        std::vector<int4> out;
+        const int mask = ~(dev::kSlice - 1);
+        auto at = [&](int v) {
+            if (v >= nactive_) return make_int2(nbr_end_, inc_end_);
+            return make_int2(vrec_[size_t(v)].x & mask, vrec_[size_t(v)].y & mask);
+        };
+        for (const int2 c : scene_colors_) {
+            const int per = dev::cluster_chunk(c.y - c.x, C);
+            for (int r = 0; r < C; ++r) {
+                const int beg = std::min(c.y, c.x + r * per), end = std::min(c.y, beg + per);
+                const int2 a = at(beg), b = at(end);
+                out.push_back(beg < end ? make_int4(a.x, b.x, a.y, b.y) : make_int4(0, 0, 0, 0));
+            }
+        }
+        return out;
     }
 
     const ClusterFit* cluster_fit(int C) const {
@@ -1268,10 +1516,12 @@ public:
         return nullptr;
     }
 
-    template <int L>
+    template <int L, bool MULTI = false, bool LEAN = false>
     void launch_cluster_l(const ClusterFit& f, int B) {
-        auto kern = dev::k_sweep_cluster<L, ST, R>;
-        GAIA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(f.bytes)));
+        auto kern = dev::k_sweep_cluster<L, MULTI, LEAN, ST, R>;
+        const int cap = max_nbr_all_;
+        const size_t smem = f.bytes + stage_bytes(cap, L, B);
+        GAIA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cluster_budget_)));
         if (f.C > 8) GAIA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
@@ -1282,7 +1532,7 @@ public:
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         cfg.blockDim = dim3(unsigned(B));
-        cfg.dynamicSmemBytes = f.bytes;
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st_;
         cfg.gridDim = dim3(unsigned(f.C));
         int nclusters = 0;
@@ -1298,7 +1548,10 @@ public:
         S.iterations = sc_.p.iterations;
         S.friction_start = sc_.p.frictionStartIter;
         S.pos_cap = f.pos_cap;
-        S.rec_cap = f.rec_cap;
+        S.nbr_cap = f.nbr_cap;
+        S.inc_cap = f.inc_cap;
+        S.stage_cap = cap;
+        S.ranges = cluster_range_bufs_.at(f.C)->p;
         GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, S, d_scene_work_.p));
     }
 
@@ -1307,6 +1560,20 @@ public:
         const ClusterFit* f = cluster_fit(C);
         if (!f) throw std::runtime_error("clusterSize: scenes do not fit a cluster of " + std::to_string(C) + " blocks");
         GAIA_CUDA(cudaMemsetAsync(d_scene_work_.p, 0, sizeof(int32_t), st_));
+        // more lanes per vertex, then fewer threads, where the staging areas do not fit beside the scene
+        auto fits = [&](int l) { return f->bytes + stage_bytes(max_nbr_all_, l, B) <= cluster_budget_; };
+        while (L < 32 && !fits(L)) L *= 2;
+        while (B > 64 && !fits(L)) B /= 2;
+        if (f->lean) {
+            while (B > 64 && f->bytes + stage_bytes(max_nbr_all_, 32, B) > cluster_budget_) B /= 2;
+            if (multi_seg_) launch_cluster_l<32, true, true>(*f, B);
+            else launch_cluster_l<32, false, true>(*f, B);
+            return;
+        }
+        if (multi_seg_) {
+            launch_cluster_l<32, true>(*f, B);
+            return;
+        }
         switch (L) {
             case 4: launch_cluster_l<4>(*f, B); break;
             case 8: launch_cluster_l<8>(*f, B); break;
@@ -1388,16 +1655,15 @@ public:
 
     // Blocks of the grid sweep: enough for the largest color at one vertex per group, at most
     // as many as are resident at once (the cooperative launch requires it).
-    template <int L>
-    int grid_blocks(int B) const {
-        int per_sm = 0;
-        GAIA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_sweep_grid<L, ST, R>, B, 0));
+    template <int L, bool MULTI>
+    int grid_blocks(int B, size_t smem) {
+        const int per_sm = blocks_per_sm(dev::k_sweep_grid<L, MULTI, ST, R>, B, smem);
         if (per_sm < 1) throw std::runtime_error("grid sweep: no block of this size fits on an SM");
         const int need = std::max(1, int(div_up(int64_t(grid_max_color_) * L, B)));
         return std::min(need, per_sm * num_sms_);
     }
 
-    template <int L>
+    template <int L, bool MULTI = false>
     void launch_grid_l(int B) {
         dev::GridSweep G;
         G.colors = d_grid_colors_.p;
@@ -1411,17 +1677,25 @@ public:
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        cfg.gridDim = dim3(unsigned(grid_blocks<L>(B)));
+        const int cap = max_nbr_all_;
+        const size_t smem = stage_bytes(cap, L, B);
+        allow_smem(dev::k_sweep_grid<L, MULTI, ST, R>, smem);
+        cfg.gridDim = dim3(unsigned(grid_blocks<L, MULTI>(B, smem)));
         cfg.blockDim = dim3(unsigned(B));
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st_;
-        GAIA_CUDA(cudaLaunchKernelEx(&cfg, dev::k_sweep_grid<L, ST, R>, ptrs(), c_, G));
+        GAIA_CUDA(cudaLaunchKernelEx(&cfg, dev::k_sweep_grid<L, MULTI, ST, R>, ptrs(), c_, G, cap));
     }
 
     // One substep's iterations: the barrier's counter and flag zeroed, one cooperative launch.
     void enqueue_grid_sweep(int L, int B) {
         if (grid_ncolors_ == 0 || sc_.p.iterations == 0) return;
         GAIA_CUDA(cudaMemsetAsync(d_grid_bar_.p, 0, 2 * sizeof(uint32_t), st_));
-        switch (L) {
+        if (multi_seg_) {
+            launch_grid_l<32, true>(B);
+            return;
+        }
+        switch (fit_lanes(L, B, 0, nactive_)) {
             case 2: launch_grid_l<2>(B); break;
             case 4: launch_grid_l<4>(B); break;
             case 8: launch_grid_l<8>(B); break;
@@ -1921,6 +2195,8 @@ private:
     DevBuf<int2> d_scene_colors_;
     DevBuf<int32_t> d_scene_ofs_, d_scene_order_, d_scene_work_;
     std::vector<ClusterFit> cluster_fits_;
+    size_t cluster_budget_ = 0;  // dynamic shared memory of a cluster's block
+    std::map<int, std::unique_ptr<DevBuf<int4>>> cluster_range_bufs_;
     DevBuf<int4> d_scene_slots_;
     // grid mode: the merged colors' slot ranges, the barrier's counter and abort flag
     DevBuf<int2> d_grid_colors_;
@@ -1933,10 +2209,11 @@ private:
     DevBuf<uint32_t> d_grid_bar_;
     int32_t grid_ncolors_ = 0, grid_max_color_ = 0;
     int variant_fixed_ = -1;   // from PhysicsParams solveVariant (-1 = autotune)
-    std::map<std::pair<int, int>, int> maxrec_cache_;
-    std::map<std::pair<int, int>, int> wave_cache_;  // (lanes, block) -> resident blocks of k_solve
-    std::map<std::pair<int, int>, int> pipe_occ_;    // (lanes and block, shared bytes) -> k_solve_pipe blocks per SM
+    std::map<std::pair<int, int>, int2> maxrec_cache_;
+    std::map<std::tuple<const void*, int, size_t>, int> occ_cache_;  // (kernel, block, shared bytes) -> blocks per SM
+    int sms_ = 0;
     static constexpr size_t kTmaSmemMax = 200 * 1024;
+    static constexpr int kLatencyColor = 1024;
     static constexpr int kContactBlocks = 64;
     double tuned_ms_ = 0.0;
     int64_t launches_per_substep_ = 0, launches_per_step_ = 0;
@@ -1945,12 +2222,17 @@ private:
     dev::Consts<R> c_{};
     std::vector<int64_t> mesh_off_;
     std::vector<int32_t> slot_of_, orig_of_, slot_mesh_, inc_ofs_, group_beg_, group_end_;
-    std::vector<int4> h_rec_n_;
-    std::vector<R4> h_rec_a_, h_rec_b_;
+    // one-ring and incidence records
+    std::vector<dev::NbrRec<R>> h_nbr_;
+    std::vector<dev::IncRec<R>> h_inc_;
+    std::vector<int4> vrec_, segs_;
+    std::vector<int2> vmore_;
+    bool multi_seg_ = false;  // some vertex has more than kSegNbrs neighbours
+    int max_nbr_all_ = 2, max_inc_all_ = 1, nbr_end_ = 0, inc_end_ = 0;
+    std::map<std::pair<int, int>, int2> lists_cache_;
     std::vector<S4> h_pos_;
     std::vector<V4> h_vel_;
     std::vector<float4> h_rest_;
-    std::vector<R> h_rec_c_;
     std::vector<dev::MeshMat<R>> h_mats_;
     std::vector<dev::DeformerDev> h_defs_;
     std::vector<int32_t> h_def_slot_, h_def_idx_;
@@ -1958,9 +2240,11 @@ private:
     DevBuf<S4> d_pos_, d_y_, d_xprev_, d_acc_pp_, d_acc_prev_;
     DevBuf<V4> d_vel_, d_vprev_;
     DevBuf<int32_t> d_inc_ofs_, d_slot_mesh_, d_slot_of_, d_def_slot_, d_def_idx_, d_tet_mesh_;
-    DevBuf<int4> d_rec_n_, d_tet_slots_;
-    DevBuf<R4> d_rec_a_, d_rec_b_;
-    DevBuf<R> d_rec_c_;
+    DevBuf<int4> d_tet_slots_;
+    DevBuf<int4> d_vrec_, d_segs_;
+    DevBuf<int2> d_vmore_;
+    DevBuf<dev::NbrRec<R>> d_nbr_;
+    DevBuf<dev::IncRec<R>> d_inc_;
     DevBuf<dev::MeshMat<R>> d_mats_;
     DevBuf<unsigned long long> d_counters_;
     DevBuf<double> d_time_, d_def_a_, d_def_b_, d_stage_f64_, d_probe_, d_tet_dminv_, d_tet_vol_;

@@ -13,8 +13,8 @@
 // its next poll), counts a device timeout and returns. Blocks never wait on anything but
 // that counter and flag, which every block of the co-resident grid reaches, so in a correct
 // launch the barrier completes; the limit only turns a lost block into a status.
-// The per-vertex arithmetic is k_solve's (same incidence loop and lane assignment, same
-// reduction and tail), so for the same lanes per vertex the result equals the per-color
+// The per-vertex arithmetic is k_solve's (same neighbour and incidence loops and lane
+// assignment, same reduction and tail), so for the same lanes per vertex the result equals the per-color
 // launches' bit for bit.
 #pragma once
 #include <cuda_runtime.h>
@@ -63,13 +63,15 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t target, int
     return s_ok != 0;
 }
 
-template <int L, typename ST, typename R>
-__global__ void __launch_bounds__(256) k_sweep_grid(Ptrs<ST, R> P, Consts<R> c, GridSweep G) {
+template <int L, bool MULTI, typename ST, typename R>
+__global__ void __launch_bounds__(256) k_sweep_grid(Ptrs<ST, R> P, Consts<R> c, GridSweep G, int cap) {
     using U = typename ST::U;
+    extern __shared__ __align__(16) unsigned char smem[];
     const int per_block = int(blockDim.x) / L;
     const int ngroups = int(gridDim.x) * per_block;
-    const int gid = int(blockIdx.x) * per_block + int(threadIdx.x) / L;
-    const int lane = int(threadIdx.x) & (L - 1);
+    const int gid = int(blockIdx.x) * per_block + int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
+    const int sub = Lanes<L>::sub();
+    const FetchGlobal<ST, kStateGrid> fetch{P.u, P.rest};
     uint32_t target = 0;
     for (int it = 0; it < G.iterations; ++it) {
         const int friction = it >= G.friction_start ? 1 : 0;
@@ -78,20 +80,9 @@ __global__ void __launch_bounds__(256) k_sweep_grid(Ptrs<ST, R> P, Consts<R> c, 
             for (int base = rg.x; base < rg.y; base += ngroups) {
                 const int v = base + gid;
                 const bool valid = v < rg.y;
-                Acc<R> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
                 U uo{};
-                MeshMat<R> mat;
-                if (valid) {
-                    mat = P.mats[P.slot_mesh[v]];
-                    const int r = P.inc_ofs[v] + lane, e = P.inc_ofs[v + 1];
-                    RecRaw<R> cur;
-                    if (r < e) cur.load_kept(P.rec_n, P.rec_a, P.rec_b, P.rec_c, r);
-                    if (lane == 0) prefetch_tail(P, v);
-                    uo = ST::ldcg_own(P.u, v);
-                    accumulate_records<L, ST, R, kStateGrid>(P, r, e, cur, uo, mat.mu, mat.lmbd, acc);
-                }
-                reduce_group<L, R>(acc);
-                if (valid && lane == 0) vertex_tail<ST, R, false>(P, c, v, uo, mat, acc, friction, nullptr, rg.x, rg.y);
+                if (valid) uo = ST::ldcg_own(P.u, v);
+                solve_in_sweep<L, MULTI, ST, R>(P, c, v, valid, sub, smem, cap, fetch, uo, friction);
             }
             if (it + 1 == G.iterations && ci + 1 == G.ncolors) break;  // the kernel's end orders the last color
             target += gridDim.x;

@@ -26,26 +26,36 @@
 //     y[s]     = inertia target, as a displacement (ST::U)
 //     xprev[s] = displacement at the start of the substep (ST::U)
 //     vel[s]   = velocity (ST::V: FP32, or FP64 in the fp64 mode)
-//   * incidence records, one per (solvable vertex, incident tet), stored in
-//     slot order (CSR offsets inc_ofs): the slots of the tet's three other
-//     vertices and their rows of dF/dx ("m vectors", from the FP64 DmInv):
-//       FP32: rec_n = int4{n0, n1, n2, bits(m2.z)}, rec_a = {m0.xyz, m1.x},
-//             rec_b = {m1.yz, m2.xy}                          -> 48 B
-//       FP64: rec_n = int4{n0, n1, n2, 0}, rec_a, rec_b (double4), rec_c = m2.z -> 88 B
-//     The own vertex's row is -(m0+m1+m2), and the rest volume is
-//     1 / (6 det[m0;m1;m2]) (the rows are stored in an order that makes the
-//     determinant equal det(DmInv)), so neither is stored.
+//   * per solvable vertex, in slot order, its one-ring and its incident tets:
+//       NbrRec (8 B FP32, 16 B FP64): slot of a neighbour n and K_n = sum over the tets that
+//         hold both vertices of A m_o . m_n (A = rest volume, m = rows of dF/dx, from the
+//         FP64 DmInv), the material-free edge weight of the linear part of the force;
+//       IncRec (8 B FP32, 16 B FP64): per incident tet the positions of its three other
+//         vertices in the vertex's neighbour list (8 bits each, in the order whose rows have
+//         determinant det DmInv) and w = 1 / (6 A) = det DmInv.
+//     The records of eight consecutive vertices are interleaved (record k of a vertex lies
+//     kSlice places after its record k - 1), so that lanes on neighbouring vertices read
+//     neighbouring records. vrec[s] = (first NbrRec, first IncRec, their numbers). Lists of
+//     more than kSegNbrs neighbours are cut into segments, the further ones in vmore.
 //
-// Per incidence the Neo-Hookean block is evaluated in closed form. With
-// G = sum_j (u_j - u_o) m_j^T (so F = I + G), J = det F, g = cof(F) m_o (= dJ/dx_o):
-//   force  -= A [ mu F m_o + lambda (J - a) g ]      (evaluated in G, see above)
-//   H      += A [ lambda g g^T ] + A mu |m_o|^2 I
-// which equals the reference's contraction of its 9x9 d2E/dF2 with the vertex
-// row of dF/dx (VBDPhysicsCompute.cu:2035-2232, VBD_NeoHookean.cpp:379-581):
-// det F is affine in x_o, so the (J - a) d2J/dF2 term contracts to zero.
+// Per vertex the Neo-Hookean block is evaluated in closed form from differences of rest
+// positions, r = X_n - X_o, and of displacements, e = u_n - u_o. With (0, 1, 2) the tet's
+// other vertices, N = (r1 - r0) x (r2 - r0) six times the rest area vector of the face
+// opposite o over its height, D the same of the deformed face and C = D - N,
+//   A m_o = -N / 6,  A cof(F) m_o = -D / 6,  6 A (det F - 1) = D . (r0 + e0) - N . r0
+// so that, with G = F - I and G m_o = sum_n (m_n . m_o) e_n, the force and Hessian of
+//   P = mu (G - (cof F - I)) + lambda (J - 1) cof F
+// summed over the tets of o are
+//   f = -mu sum_n K_n e_n - mu/6 sum_t C_t + lambda/6 sum_t (w S D)_t,  S = N.e0 + C.(r0 + e0)
+//   H = lambda/6 sum_t (w D D^T)_t - mu sum_n K_n I
+// (the same terms as the reference's contraction of its 9x9 d2E/dF2 with the vertex row of
+// dF/dx, VBDPhysicsCompute.cu:2035-2232, VBD_NeoHookean.cpp:379-581: det F is affine in x_o,
+// so the (J - a) d2J/dF2 term contracts to zero). Every difference is formed from small
+// quantities: C = a x de + db x b' with a, b' edges and db, de differences of displacements.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "cloth_dev.cuh"
 #include "vbd_state.cuh"
@@ -92,6 +102,34 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // those, blocks whose final drain wait ran out too.
 enum { CNT_FP64_SOLVES = 0, CNT_FAILED_SOLVES = 1, CNT_NONFINITE = 2, CNT_TIMEOUT = 3, CNT_DRAIN = 4, CNT_N = 8 };
 
+// One-ring and incidence records (see the top of the file), each one vector load.
+constexpr int kSegNbrs = 128;  // neighbours per segment at most (8-bit positions)
+constexpr int kSlice = 8;      // vertices whose records are interleaved
+template <typename R>
+struct NbrRec;
+template <>
+struct alignas(8) NbrRec<float> {
+    int32_t slot;
+    float k;
+};
+template <>
+struct alignas(16) NbrRec<double> {
+    int32_t slot, pad;
+    double k;
+};
+template <typename R>
+struct IncRec;
+template <>
+struct alignas(8) IncRec<float> {
+    uint32_t idx;
+    float w;
+};
+template <>
+struct alignas(16) IncRec<double> {
+    uint32_t idx, pad;
+    double w;
+};
+
 template <typename ST, typename R>
 struct Ptrs {
     typename ST::U* u;
@@ -100,11 +138,11 @@ struct Ptrs {
     typename ST::U* xprev;
     typename ST::V* vel;
     typename ST::V* vprev;
-    const int32_t* inc_ofs;
-    const int4* rec_n;
-    const R4<R>* rec_a;
-    const R4<R>* rec_b;
-    const R* rec_c;            // FP64 only
+    const int4* vrec;          // per slot: first NbrRec, first IncRec, number of each
+    const int2* vmore;         // per slot its further segments [x, y) in segs; null: there are none
+    const int4* segs;          // the further segments, as vrec
+    const NbrRec<R>* nbr;
+    const IncRec<R>* inc;
     const int32_t* slot_mesh;
     const MeshMat<R>* mats;
     unsigned long long* counters;
@@ -145,53 +183,28 @@ struct DeformVerts {
 __device__ __forceinline__ float f_bits(int v) { return __int_as_float(v); }
 
 // Symmetric 3x3 solve by LDL^T (the same algorithm as the oracle's
-// solve3x3_ldlt). H = {h00, h01, h02, h11, h12, h22}.
+// solve3x3_ldlt), with one reciprocal per pivot instead of two divisions (three IEEE
+// divisions instead of six on the vertex's serial path; in FP64 a division is a dozen
+// instructions of a pipe that issues one every 16 cycles). H = {h00, h01, h02, h11, h12, h22}.
 template <typename R>
 __device__ __forceinline__ bool ldlt3(const R* H, const R* b, R* x, R rel_tol) {
-    R scale = fmax(fabs(H[0]), fmax(fabs(H[3]), fabs(H[5])));
+    const R scale = fmax(fabs(H[0]), fmax(fabs(H[3]), fabs(H[5])));
     if (!(scale > R(0))) return false;
-    R tol = rel_tol * scale;
-    R d0 = H[0];
+    const R tol = rel_tol * scale;
+    const R d0 = H[0];
     if (!(d0 > tol)) return false;
-    R l10 = H[1] / d0, l20 = H[2] / d0;
-    R d1 = H[3] - l10 * H[1];
+    const R r0 = R(1) / d0;
+    const R l10 = H[1] * r0, l20 = H[2] * r0;
+    const R d1 = H[3] - l10 * H[1];
     if (!(d1 > tol)) return false;
-    R l21 = (H[4] - l20 * H[1]) / d1;
-    R d2 = H[5] - l20 * H[2] - l21 * l21 * d1;
+    const R r1 = R(1) / d1;
+    const R l21 = (H[4] - l20 * H[1]) * r1;
+    const R d2 = H[5] - l20 * H[2] - l21 * l21 * d1;
     if (!(d2 > tol)) return false;
-    R z0 = b[0];
-    R z1 = b[1] - l10 * z0;
-    R z2 = b[2] - l20 * z0 - l21 * z1;
-    z0 /= d0;
-    z1 /= d1;
-    z2 /= d2;
-    x[2] = z2;
-    x[1] = z1 - l21 * x[2];
-    x[0] = z0 - l10 * x[1] - l20 * x[2];
-    return isfinite(x[0]) && isfinite(x[1]) && isfinite(x[2]);
-}
-
-// FP32: one reciprocal per pivot instead of two divisions per pivot (three IEEE divisions
-// instead of six on the vertex's serial path); the FP64 factorisation divides.
-template <>
-__device__ __forceinline__ bool ldlt3<float>(const float* H, const float* b, float* x, float rel_tol) {
-    const float scale = fmaxf(fabsf(H[0]), fmaxf(fabsf(H[3]), fabsf(H[5])));
-    if (!(scale > 0.f)) return false;
-    const float tol = rel_tol * scale;
-    const float d0 = H[0];
-    if (!(d0 > tol)) return false;
-    const float r0 = 1.f / d0;
-    const float l10 = H[1] * r0, l20 = H[2] * r0;
-    const float d1 = H[3] - l10 * H[1];
-    if (!(d1 > tol)) return false;
-    const float r1 = 1.f / d1;
-    const float l21 = (H[4] - l20 * H[1]) * r1;
-    const float d2 = H[5] - l20 * H[2] - l21 * l21 * d1;
-    if (!(d2 > tol)) return false;
-    const float r2 = 1.f / d2;
-    const float z0 = b[0];
-    const float z1 = b[1] - l10 * z0;
-    const float z2 = b[2] - l20 * z0 - l21 * z1;
+    const R r2 = R(1) / d2;
+    const R z0 = b[0];
+    const R z1 = b[1] - l10 * z0;
+    const R z2 = b[2] - l20 * z0 - l21 * z1;
     x[2] = z2 * r2;
     x[1] = z1 * r1 - l21 * x[2];
     x[0] = z0 * r0 - l10 * x[1] - l20 * x[2];
@@ -229,62 +242,25 @@ __device__ __forceinline__ bool solve3<double>(const double* H, const double* b,
     return ldlt3<double>(H, b, x, kFp64Pivot);
 }
 
-// One incidence record as loaded from HBM (streaming loads: each record is
-// read once per iteration). load() issues the loads; the fields are decoded
-// where they are used, so a record can be in flight while the previous one
-// is being computed.
-template <typename R>
-struct RecRaw;
-template <>
-struct RecRaw<float> {
-    int4 n;
-    float4 a, b;
-    __device__ __forceinline__ void load(const int4* rec_n, const R4<float>* rec_a, const R4<float>* rec_b,
-                                         const float*, int r) {
-        n = __ldcs(rec_n + r);
-        a = __ldcs(reinterpret_cast<const float4*>(rec_a) + r);
-        b = __ldcs(reinterpret_cast<const float4*>(rec_b) + r);
+// How records are read: streamed (once per launch), kept in the caches (every iteration by
+// the persistent sweeps) or from shared memory.
+enum RecRead { kRecStream = 0, kRecKept = 1, kRecShared = 2 };
+template <int RR, typename T>
+__device__ __forceinline__ T ld_rec(const T* p) {
+    if constexpr (RR == kRecShared) {
+        return *p;
+    } else {
+        T t;
+        if constexpr (sizeof(T) == 8) {
+            const int2 q = RR == kRecStream ? __ldcs(reinterpret_cast<const int2*>(p)) : __ldg(reinterpret_cast<const int2*>(p));
+            memcpy(&t, &q, sizeof(t));
+        } else {
+            const int4 q = RR == kRecStream ? __ldcs(reinterpret_cast<const int4*>(p)) : __ldg(reinterpret_cast<const int4*>(p));
+            memcpy(&t, &q, sizeof(t));
+        }
+        return t;
     }
-    // cached (not streaming): for a kernel that reads the same records every iteration
-    __device__ __forceinline__ void load_kept(const int4* rec_n, const R4<float>* rec_a, const R4<float>* rec_b,
-                                              const float*, int r) {
-        n = __ldg(rec_n + r);
-        a = __ldg(reinterpret_cast<const float4*>(rec_a) + r);
-        b = __ldg(reinterpret_cast<const float4*>(rec_b) + r);
-    }
-    __device__ __forceinline__ void rows(float* m0, float* m1, float* m2) const {
-        m0[0] = a.x; m0[1] = a.y; m0[2] = a.z;
-        m1[0] = a.w; m1[1] = b.x; m1[2] = b.y;
-        m2[0] = b.z; m2[1] = b.w; m2[2] = f_bits(n.w);
-    }
-};
-template <>
-struct RecRaw<double> {
-    int4 n;
-    double2 a0, a1, b0, b1;
-    double c;
-    __device__ __forceinline__ void load(const int4* rec_n, const R4<double>* rec_a, const R4<double>* rec_b,
-                                         const double* rec_c, int r) {
-        n = __ldcs(rec_n + r);
-        const double2* pa = reinterpret_cast<const double2*>(rec_a + r);
-        const double2* pb = reinterpret_cast<const double2*>(rec_b + r);
-        a0 = __ldcs(pa); a1 = __ldcs(pa + 1); b0 = __ldcs(pb); b1 = __ldcs(pb + 1);
-        c = __ldcs(rec_c + r);
-    }
-    __device__ __forceinline__ void load_kept(const int4* rec_n, const R4<double>* rec_a, const R4<double>* rec_b,
-                                              const double* rec_c, int r) {
-        n = __ldg(rec_n + r);
-        const double2* pa = reinterpret_cast<const double2*>(rec_a + r);
-        const double2* pb = reinterpret_cast<const double2*>(rec_b + r);
-        a0 = __ldg(pa); a1 = __ldg(pa + 1); b0 = __ldg(pb); b1 = __ldg(pb + 1);
-        c = __ldg(rec_c + r);
-    }
-    __device__ __forceinline__ void rows(double* m0, double* m1, double* m2) const {
-        m0[0] = a0.x; m0[1] = a0.y; m0[2] = a1.x;
-        m1[0] = a1.y; m1[1] = b0.x; m1[2] = b0.y;
-        m2[0] = b1.x; m2[1] = b1.y; m2[2] = c;
-    }
-};
+}
 
 // Accumulator of one vertex: force (3), lambda-part of the Hessian (6, upper
 // triangle), and S = sum A mu |m_o|^2 (the isotropic part).
@@ -293,71 +269,320 @@ struct Acc {
     R f0, f1, f2, h00, h01, h02, h11, h12, h22, S;
 };
 
-// e0, e1, e2 = u_j - u_o (relative displacements) of the three other vertices.
-template <typename R>
-__device__ __forceinline__ void incidence(const R* e0, const R* e1, const R* e2, const R* m0, const R* m1,
-                                          const R* m2, R mu, R lmbd, Acc<R>& acc) {
-    R G[3][3];
+// Where a vertex's one-ring comes from. Global memory: either copied into the staging area
+// asynchronously (past L1: the lines were written by earlier launches, earlier in the same
+// kernel by the same block before a block barrier, or by other blocks before a grid barrier),
+// or loaded into registers: Plain loads (states written by earlier launches or by the same
+// block), or through L2 only (Grid: written by other blocks of the same launch). Never through
+// the read-only path: the compiler may move such loads above the wait for the previous color.
+enum StateRead { kStatePlain = 0, kStateGrid = 1 };
+template <typename ST, int MODE>
+struct FetchGlobal {
+    const typename ST::U* u;
+    const float4* rest;
+    __device__ __forceinline__ void operator()(int s, typename ST::U& q, float4& X) const {
+        if constexpr (MODE == kStateGrid) q = ST::ldcg(u, s);
+        else q = ST::ld(u, s);
+        X = __ldg(rest + s);
+    }
+};
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+// This thread's copies have landed (and are visible to it).
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// A warp solves W = 32 / L vertices, L lanes each: lane i works on vertex i % W, as its
+// sub-lane i / W. The lanes of a quarter warp are then on different vertices (up to L = 4),
+// so that their accesses to shared memory fall into different banks, and the lanes on
+// sub-lane 0, which run the vertex tails, are neighbours on neighbouring vertices.
+template <int L>
+struct Lanes {
+    static constexpr int kW = 32 / L;
+    __device__ __forceinline__ static int vertex() { return int(threadIdx.x) & (kW - 1); }   // within the warp
+    __device__ __forceinline__ static int sub() { return (int(threadIdx.x) & 31) / kW; }
+};
+
+// A vertex's staged one-ring in shared memory: per neighbour e = u_n - u_o and r = X_n - X_o
+// in the compute type, in 16-byte parts (each a plane of the warp's area, the entries of its W
+// vertices interleaved; `cap` entries per vertex): FP32 {e, r.x} {r.y, r.z, -, -}, FP64
+// {e.x, e.y} {e.z, r.x} {r.y, r.z}. The same parts first hold the neighbour as it lies in
+// global memory (its state in ST::kNbParts parts, then its rest position) where it is copied
+// asynchronously; the lane that copied an entry turns it into differences in place.
+template <int W, typename ST, typename R>
+struct Stage {
+    static constexpr int kRaw = ST::kNbParts + 1;
+    static constexpr int kParts = sizeof(R) == 8 ? 3 : kRaw;  // 16-byte parts per neighbour
+    float4* p;
+    int plane;
+    __device__ __forceinline__ Stage(unsigned char* q, int cap, int v)
+        : p(reinterpret_cast<float4*>(q) + v), plane(cap * W) {}
+    __device__ __forceinline__ float4* part(int i, int k) const { return p + i * W + k * plane; }
+    __device__ __forceinline__ void put(int i, const R* e, const R* r) const {
+        if constexpr (sizeof(R) == 4) {
+            *part(i, 0) = make_float4(e[0], e[1], e[2], r[0]);
+            *reinterpret_cast<float2*>(part(i, 1)) = make_float2(r[1], r[2]);
+        } else {
+            *reinterpret_cast<double2*>(part(i, 0)) = make_double2(e[0], e[1]);
+            *reinterpret_cast<double2*>(part(i, 1)) = make_double2(e[2], r[0]);
+            *reinterpret_cast<double2*>(part(i, 2)) = make_double2(r[1], r[2]);
+        }
+    }
+    __device__ __forceinline__ void get(int i, R* e, R* r) const {
+        if constexpr (sizeof(R) == 4) {
+            const float4 a = *part(i, 0);
+            const float2 b = *reinterpret_cast<const float2*>(part(i, 1));
+            e[0] = a.x; e[1] = a.y; e[2] = a.z;
+            r[0] = a.w; r[1] = b.x; r[2] = b.y;
+        } else {
+            const double2 a = *reinterpret_cast<const double2*>(part(i, 0));
+            const double2 b = *reinterpret_cast<const double2*>(part(i, 1));
+            const double2 c = *reinterpret_cast<const double2*>(part(i, 2));
+            e[0] = a.x; e[1] = a.y; e[2] = b.x;
+            r[0] = b.y; r[1] = c.x; r[2] = c.y;
+        }
+    }
+    // the neighbour in global slot s into entry i, asynchronously, and back out of it
+    __device__ __forceinline__ void copy(int i, const typename ST::U* u, const float4* rest, int s) const {
+        const float4* q = reinterpret_cast<const float4*>(u + s);
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+        for (int k = 0; k < ST::kNbParts; ++k) cp_async16(part(i, k), q + k);
+        cp_async16(part(i, ST::kNbParts), rest + s);
+    }
+    __device__ __forceinline__ void raw(int i, typename ST::U& q, float4& X) const {
+        float4 w[sizeof(typename ST::U) / 16] = {};
 #pragma unroll
-        for (int c = 0; c < 3; ++c) G[r][c] = e0[r] * m0[c] + e1[r] * m1[c] + e2[r] * m2[c];
-    // rest volume from the stored rows: A = 1 / (6 det[m0; m1; m2])
-    R detM = m0[0] * (m1[1] * m2[2] - m1[2] * m2[1]) - m0[1] * (m1[0] * m2[2] - m1[2] * m2[0]) +
-             m0[2] * (m1[0] * m2[1] - m1[1] * m2[0]);
-    R A = R(1) / (R(6) * detM);
-    R mo[3] = {-(m0[0] + m1[0] + m2[0]), -(m0[1] + m1[1] + m2[1]), -(m0[2] + m1[2] + m2[2])};
-    // Cg = cof(I + G) - I, entrywise
-    R C00 = G[1][1] + G[2][2] + (G[1][1] * G[2][2] - G[1][2] * G[2][1]);
-    R C11 = G[0][0] + G[2][2] + (G[0][0] * G[2][2] - G[0][2] * G[2][0]);
-    R C22 = G[0][0] + G[1][1] + (G[0][0] * G[1][1] - G[0][1] * G[1][0]);
-    R C01 = G[1][2] * G[2][0] - G[1][0] * (R(1) + G[2][2]);
-    R C02 = G[1][0] * G[2][1] - (R(1) + G[1][1]) * G[2][0];
-    R C10 = G[0][2] * G[2][1] - G[0][1] * (R(1) + G[2][2]);
-    R C12 = G[0][1] * G[2][0] - (R(1) + G[0][0]) * G[2][1];
-    R C20 = G[0][1] * G[1][2] - G[0][2] * (R(1) + G[1][1]);
-    R C21 = G[0][2] * G[1][0] - (R(1) + G[0][0]) * G[1][2];
-    // dJ = det(I + G) - 1 = G00 (1 + Cg00) + G01 C01 + G02 C02 + Cg00
-    R dJ = G[0][0] * (R(1) + C00) + G[0][1] * C01 + G[0][2] * C02 + C00;
-    // g = cof(F) m_o = m_o + Cg m_o
-    R cm0 = C00 * mo[0] + C01 * mo[1] + C02 * mo[2];
-    R cm1 = C10 * mo[0] + C11 * mo[1] + C12 * mo[2];
-    R cm2 = C20 * mo[0] + C21 * mo[1] + C22 * mo[2];
-    R g0 = mo[0] + cm0, g1 = mo[1] + cm1, g2 = mo[2] + cm2;
-    R Gm0 = G[0][0] * mo[0] + G[0][1] * mo[1] + G[0][2] * mo[2];
-    R Gm1 = G[1][0] * mo[0] + G[1][1] * mo[1] + G[1][2] * mo[2];
-    R Gm2 = G[2][0] * mo[0] + G[2][1] * mo[1] + G[2][2] * mo[2];
-    // P m_o = mu (G - Cg) m_o + lambda dJ g
-    R Am = A * mu;
-    R Ald = A * lmbd * dJ;
-    acc.f0 -= Am * (Gm0 - cm0) + Ald * g0;
-    acc.f1 -= Am * (Gm1 - cm1) + Ald * g1;
-    acc.f2 -= Am * (Gm2 - cm2) + Ald * g2;
-    R Al = A * lmbd;
-    R lg0 = Al * g0, lg1 = Al * g1, lg2 = Al * g2;
-    acc.h00 += lg0 * g0;
-    acc.h01 += lg0 * g1;
-    acc.h02 += lg0 * g2;
-    acc.h11 += lg1 * g1;
-    acc.h12 += lg1 * g2;
-    acc.h22 += lg2 * g2;
-    acc.S += Am * (mo[0] * mo[0] + mo[1] * mo[1] + mo[2] * mo[2]);
+        for (int k = 0; k < ST::kNbParts; ++k) w[k] = *part(i, k);
+        memcpy(&q, w, sizeof(q));
+        X = *part(i, ST::kNbParts);
+    }
+};
+
+// The staging area of this lane's vertex: the warps' areas follow each other, `cap` entries per
+// vertex.
+template <int L, typename ST, typename R>
+__device__ __forceinline__ Stage<32 / L, ST, R> warp_stage(unsigned char* smem, int cap) {
+    using S = Stage<32 / L, ST, R>;
+    return S(smem + size_t(threadIdx.x >> 5) * size_t(cap * (32 / L)) * (16 * S::kParts), cap, Lanes<L>::vertex());
 }
 
+// One tet from its three other vertices' differences: C into cs, w S D into t, w D D^T into the
+// accumulator's Hessian (unscaled, see finish_acc).
+template <typename R>
+__device__ __forceinline__ void incidence(const R* e0, const R* e1, const R* e2, const R* r0, const R* r1, const R* r2,
+                                          R w, R* cs, R* t, Acc<R>& acc) {
+    const R a[3] = {r1[0] - r0[0], r1[1] - r0[1], r1[2] - r0[2]};
+    const R b[3] = {r2[0] - r0[0], r2[1] - r0[1], r2[2] - r0[2]};
+    const R al[3] = {e1[0] - e0[0], e1[1] - e0[1], e1[2] - e0[2]};
+    const R be[3] = {e2[0] - e0[0], e2[1] - e0[1], e2[2] - e0[2]};
+    const R bd[3] = {b[0] + be[0], b[1] + be[1], b[2] + be[2]};
+    // C = a x be + al x bd, N = a x b
+    const R C0 = (a[1] * be[2] - a[2] * be[1]) + (al[1] * bd[2] - al[2] * bd[1]);
+    const R C1 = (a[2] * be[0] - a[0] * be[2]) + (al[2] * bd[0] - al[0] * bd[2]);
+    const R C2 = (a[0] * be[1] - a[1] * be[0]) + (al[0] * bd[1] - al[1] * bd[0]);
+    const R N0 = a[1] * b[2] - a[2] * b[1], N1 = a[2] * b[0] - a[0] * b[2], N2 = a[0] * b[1] - a[1] * b[0];
+    const R D0 = N0 + C0, D1 = N1 + C1, D2 = N2 + C2;
+    const R p0 = r0[0] + e0[0], p1 = r0[1] + e0[1], p2 = r0[2] + e0[2];
+    const R S = (N0 * e0[0] + N1 * e0[1] + N2 * e0[2]) + (C0 * p0 + C1 * p1 + C2 * p2);
+    const R w0 = w * D0, w1 = w * D1, w2 = w * D2;
+    cs[0] += C0; cs[1] += C1; cs[2] += C2;
+    t[0] += S * w0; t[1] += S * w1; t[2] += S * w2;
+    acc.h00 += w0 * D0;
+    acc.h01 += w0 * D1;
+    acc.h02 += w0 * D2;
+    acc.h11 += w1 * D1;
+    acc.h12 += w1 * D2;
+    acc.h22 += w2 * D2;
+}
+
+// The first records of a lane's share of a segment, loaded ahead of the state reads (they are
+// static data): its first NB neighbours (sub, sub + L, ...) and its first two incidences.
+// Record k of the segment is kSlice * k places after its first.
+template <typename R, int NB>
+struct SegRecs {
+    NbrRec<R> n[NB];
+    IncRec<R> i0, i1;
+    const NbrRec<R>* np;  // the segment's records
+    const IncRec<R>* ip;
+    int nn, ni;           // their numbers (0 for a lane without a vertex)
+};
+template <int L, int RR, typename R, int NB>
+__device__ __forceinline__ void preload(SegRecs<R, NB>& s, const NbrRec<R>* nbr, const IncRec<R>* inc, int4 seg,
+                                        int sub) {
+    s.np = nbr + seg.x;
+    s.ip = inc + seg.y;
+    s.nn = seg.z;
+    s.ni = seg.w;
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+        if (sub + j * L < s.nn) s.n[j] = ld_rec<RR>(s.np + kSlice * (sub + j * L));
+    if (sub < s.ni) s.i0 = ld_rec<RR>(s.ip + kSlice * sub);
+    if (sub + L < s.ni) s.i1 = ld_rec<RR>(s.ip + kSlice * (sub + L));
+}
+
+// Neighbour records a lane holds at a time. ASYNC: the one-ring is copied into the staging area
+// asynchronously, all of a vertex's neighbours (6 or 18 on a 5-tet lattice, about 14 on other
+// meshes) in flight at once without occupying registers, at the price of a second pass over
+// shared memory. Otherwise they are loaded into registers, two per lane at a time (one in
+// the wide groups of small colors, which have one neighbour per lane).
+template <int L, bool ASYNC>
+struct NbrBatch {
+    static constexpr int kN = L >= 16 ? 1 : (!ASYNC ? 2 : (L == 8 ? 3 : (L == 4 ? 5 : 9)));
+};
+
+// One lane's share of one segment: stages the segment's one-ring (neighbours sub, sub + L,
+// ...; a narrow group reads each record twice, for the slot and then for K) in shared memory,
+// adding the linear force on the way, then runs its incidences (sub,
+// sub + L, ...) on the staged differences. Every lane
+// of the warp calls it (lanes without a vertex with empty lists). Each neighbour state is
+// read once per vertex instead of once per incidence, and the incidence loop has no
+// dependent global load.
+template <int L, int RR, bool ASYNC, typename ST, typename R, int NB, typename Fetch>
+__device__ __forceinline__ void accumulate_segment(SegRecs<R, NB>& s, int sub, const Stage<32 / L, ST, R>& st, const Fetch& fetch,
+                                                   const typename ST::U& uo, const float4& Xo, R mu, R lmbd,
+                                                   Acc<R>& acc) {
+    using U = typename ST::U;
+    R kf[3] = {R(0), R(0), R(0)}, cs[3] = {R(0), R(0), R(0)}, t[3] = {R(0), R(0), R(0)};
+    auto take = [&](int k, const U& q, const float4& X, R K) {
+        R e[3];
+        ST::diff(q, uo, e);
+        const R r[3] = {R(X.x) - R(Xo.x), R(X.y) - R(Xo.y), R(X.z) - R(Xo.z)};
+        st.put(k, e, r);
+        kf[0] += K * e[0];
+        kf[1] += K * e[1];
+        kf[2] += K * e[2];
+        acc.S += K;
+    };
+    if constexpr (ASYNC) {
+        for (int k = sub; k < s.nn; k += NB * L) {
+#pragma unroll
+            for (int j = 0; j < NB; ++j)
+                if (k + j * L < s.nn) st.copy(k + j * L, fetch.u, fetch.rest, s.n[j].slot);
+            if (k + NB * L < s.nn) {
+#pragma unroll
+                for (int j = 0; j < NB; ++j)
+                    if (k + (NB + j) * L < s.nn) s.n[j] = ld_rec<RR>(s.np + kSlice * (k + (NB + j) * L));
+            }
+        }
+        cp_async_wait();
+        for (int k = sub; k < s.nn; k += L) {
+            U q;
+            float4 X;
+            st.raw(k, q, X);
+            take(k, q, X, ld_rec<RR == kRecShared ? kRecShared : kRecKept>(s.np + kSlice * k).k);
+        }
+    } else {
+        for (int k = sub; k < s.nn; k += NB * L) {
+            U q[NB];
+            float4 X[NB];
+#pragma unroll
+            for (int j = 0; j < NB; ++j)
+                if (k + j * L < s.nn) fetch(s.n[j].slot, q[j], X[j]);
+#pragma unroll
+            for (int j = 0; j < NB; ++j) {
+                if (k + j * L >= s.nn) break;
+                take(k + j * L, q[j], X[j], s.n[j].k);
+                if (k + (j + NB) * L < s.nn) s.n[j] = ld_rec<RR>(s.np + kSlice * (k + (j + NB) * L));
+            }
+        }
+    }
+    __syncwarp();
+    for (int k = sub; k < s.ni; k += L) {
+        const IncRec<R> cur = s.i0;
+        s.i0 = s.i1;
+        if (k + 2 * L < s.ni) s.i1 = ld_rec<RR>(s.ip + kSlice * (k + 2 * L));
+        R e0[3], e1[3], e2[3], r0[3], r1[3], r2[3];
+        st.get(int(cur.idx & 255u), e0, r0);
+        st.get(int((cur.idx >> 8) & 255u), e1, r1);
+        st.get(int((cur.idx >> 16) & 255u), e2, r2);
+        incidence(e0, e1, e2, r0, r1, r2, cur.w, cs, t, acc);
+    }
+    const R m6 = mu * R(1.0 / 6.0), l6 = lmbd * R(1.0 / 6.0);
+    acc.f0 += l6 * t[0] - m6 * cs[0] - mu * kf[0];
+    acc.f1 += l6 * t[1] - m6 * cs[1] - mu * kf[1];
+    acc.f2 += l6 * t[2] - m6 * cs[2] - mu * kf[2];
+}
+
+// The remaining segments of a vertex with more than kSegNbrs neighbours. Only the 32-lane
+// kernels of scenes with such a vertex (MULTI) hold this loop: it costs registers.
+template <int L, int RR, bool ASYNC, typename ST, typename R, int NB, typename Fetch>
+__device__ __forceinline__ void accumulate_more(SegRecs<R, NB>& rec, const Ptrs<ST, R>& P, const NbrRec<R>* nbr,
+                                                const IncRec<R>* inc, int2 more, int sub, const Stage<32 / L, ST, R>& st,
+                                                const Fetch& fetch, const typename ST::U& uo, const float4& Xo, R mu,
+                                                R lmbd, Acc<R>& acc) {
+    static_assert(L == 32, "one vertex per warp");
+    for (int i = more.x; i < more.y; ++i) {
+        __syncwarp();
+        preload<L, RR>(rec, nbr, inc, P.segs[i], sub);
+        accumulate_segment<L, RR, ASYNC, ST>(rec, sub, st, fetch, uo, Xo, mu, lmbd, acc);
+    }
+}
+
+// The accumulated sums in the units of the force and the Hessian (after the lane reduction).
+template <typename R>
+__device__ __forceinline__ void finish_acc(Acc<R>& a, R mu, R lmbd) {
+    const R l6 = lmbd * R(1.0 / 6.0);
+    a.h00 *= l6; a.h01 *= l6; a.h02 *= l6; a.h11 *= l6; a.h12 *= l6; a.h22 *= l6;
+    a.S *= -mu;
+}
+
+// One halving step of the reduce-scatter below: of n values, this lane keeps the lower or the
+// upper half (rounded up; a missing one counts as zero) and adds its partner's share of it.
+template <int N>
+__device__ __forceinline__ void halve(double* v, int off, bool upper) {
+    constexpr int H = (N + 1) / 2;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        const double lo = v[i], hi = i + H < N ? v[i + H] : 0.0;
+        const double got = __shfl_xor_sync(0xffffffffu, upper ? lo : hi, off);
+        v[i] = (upper ? hi : lo) + got;
+    }
+}
+
+// Sums over the L lanes of a vertex; valid on sub-lane 0.
 template <int L, typename R>
 __device__ __forceinline__ void reduce_group(Acc<R>& a) {
+    constexpr int W = 32 / L;
+    if constexpr (sizeof(R) == 8 && L >= 8) {
+        // FP64 in wide groups: the adds of a butterfly over all ten sums (50 per lane at L = 32, as
+        // many as two thirds of an incidence) cost more than the loop, as the FP64 pipe takes 16 cycles a warp
+        // instruction. Each step halves the sums a lane holds (5, 3, 2, 1, 1 adds), and sub-lane 0
+        // collects them at the end.
+        double v[10] = {a.f0, a.f1, a.f2, a.h00, a.h01, a.h02, a.h11, a.h12, a.h22, a.S};
+        const int sub = Lanes<L>::sub(), vw = Lanes<L>::vertex();
+        // top bits of sub choose the halves: 10 -> 5 -> 3 -> 2 (-> 1)
+        halve<10>(v, 16, (sub & (L / 2)) != 0);
+        halve<5>(v, 8, (sub & (L / 4)) != 0);
+        halve<3>(v, 4, (sub & (L / 8)) != 0);
+        constexpr int kLeft = L >= 16 ? 1 : 2;  // sums held per lane
+        if constexpr (L >= 16) halve<2>(v, 2, (sub & (L / 16)) != 0);
+        if constexpr (L >= 32) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+        // sum k sits on the lane whose choices lead to it: k = 5 b0 + 3 b1 + 2 b2 + b3
+        double out[10];
 #pragma unroll
-    for (int off = L / 2; off > 0; off >>= 1) {
-        a.f0 += __shfl_xor_sync(0xffffffffu, a.f0, off);
-        a.f1 += __shfl_xor_sync(0xffffffffu, a.f1, off);
-        a.f2 += __shfl_xor_sync(0xffffffffu, a.f2, off);
-        a.h00 += __shfl_xor_sync(0xffffffffu, a.h00, off);
-        a.h01 += __shfl_xor_sync(0xffffffffu, a.h01, off);
-        a.h02 += __shfl_xor_sync(0xffffffffu, a.h02, off);
-        a.h11 += __shfl_xor_sync(0xffffffffu, a.h11, off);
-        a.h12 += __shfl_xor_sync(0xffffffffu, a.h12, off);
-        a.h22 += __shfl_xor_sync(0xffffffffu, a.h22, off);
-        a.S += __shfl_xor_sync(0xffffffffu, a.S, off);
+        for (int k = 0; k < 10; ++k) {
+            const int b0 = k >= 5, k1 = k - 5 * b0, b1 = k1 >= 3, k2 = k1 - 3 * b1, b2 = k2 >= 2, k3 = k2 - 2 * b2;
+            int src = b0 * (L / 2) + b1 * (L / 4) + b2 * (L / 8);
+            if (kLeft == 1) src += k3 * (L / 16);
+            out[k] = __shfl_sync(0xffffffffu, kLeft == 1 ? v[0] : v[k3], src * W + vw);
+        }
+        a = Acc<R>{out[0], out[1], out[2], out[3], out[4], out[5], out[6], out[7], out[8], out[9]};
+    } else {
+#pragma unroll
+        for (int off = 16; off >= W; off >>= 1) {
+            a.f0 += __shfl_xor_sync(0xffffffffu, a.f0, off);
+            a.f1 += __shfl_xor_sync(0xffffffffu, a.f1, off);
+            a.f2 += __shfl_xor_sync(0xffffffffu, a.f2, off);
+            a.h00 += __shfl_xor_sync(0xffffffffu, a.h00, off);
+            a.h01 += __shfl_xor_sync(0xffffffffu, a.h01, off);
+            a.h02 += __shfl_xor_sync(0xffffffffu, a.h02, off);
+            a.h11 += __shfl_xor_sync(0xffffffffu, a.h11, off);
+            a.h12 += __shfl_xor_sync(0xffffffffu, a.h12, off);
+            a.h22 += __shfl_xor_sync(0xffffffffu, a.h22, off);
+            a.S += __shfl_xor_sync(0xffffffffu, a.S, off);
+        }
     }
 }
 
@@ -385,8 +610,9 @@ __device__ __forceinline__ void axis_friction(int d, const R* dx, R mu, R lambda
 // ---------------------------------------------------------------------------
 template <typename ST, typename R, bool PROBE>
 __device__ __forceinline__ bool vertex_tail(const Ptrs<ST, R>& P, const Consts<R>& c, int v, const typename ST::U& uo,
-                                            const MeshMat<R>& mat, const Acc<R>& acc, int friction,
-                                            double* probe_out, int beg, int end, typename ST::U* unew = nullptr);
+                                            const float4& Xo, const float3& Fo, const MeshMat<R>& mat,
+                                            const Acc<R>& acc, int friction, double* probe_out,
+                                            typename ST::U* unew = nullptr);
 
 // ---------------------------------------------------------------------------
 // Tet-mesh vertex-face contact (VBDPhysicsCompute.cu:1731-1773, 1812-1930)
@@ -518,68 +744,49 @@ __global__ void __launch_bounds__(128) k_contact_color(Ptrs<ST, R> P, Consts<R> 
     }
 }
 
-// The vertex tail's own inputs (inertia target, start-of-substep state, rest position) into
-// L1 while the incidence loop runs: they do not change during a sweep, and loaded only in
-// the tail their latency would follow the lane reduction on the critical path.
-template <typename ST, typename R>
+// The vertex tail's own inputs into L1 while the incidence loop runs: they do not change during
+// a sweep, and loaded only in the tail their latency would follow the lane reduction on the
+// critical path. Wide groups (few vertices, bound by that path) prefetch what only the vertices
+// at a wall read, too; the others save its 48 bytes per vertex.
+template <int L, typename ST, typename R>
 __device__ __forceinline__ void prefetch_tail(const Ptrs<ST, R>& P, int v) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(P.y + v));
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(P.xprev + v));
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(P.rest + v));
-    if (P.rest_fh) {
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.rest_fh + v));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.rest_fl + v));
+    if constexpr (L >= 16) {
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.xprev + v));
+        if (P.rest_fh) {
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(P.rest_fh + v));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(P.rest_fl + v));
+        }
     }
 }
 
-// How the incidence loop reads neighbour states and records:
-//  kStateStream  states through the read-only cache (written by earlier launches only),
-//                records streamed (read once per launch);
-//  kStateBlock   states with plain loads (written earlier in the same kernel by the same
-//                block, ordered by a block barrier), records kept in the caches (read
-//                every iteration by the persistent sweeps);
-//  kStateGrid    states through L2 only (written earlier in the same kernel by other
-//                blocks, ordered by a grid barrier), records kept.
-enum StateRead { kStateStream = 0, kStateBlock = 1, kStateGrid = 2 };
+// The mesh frame's offset of a vertex, rounded to FP32 (zero without frames).
+template <typename ST, typename R>
+__device__ __forceinline__ float3 frame_offset(const Ptrs<ST, R>& P, int v) {
+    if (!P.frame_F) return make_float3(0.f, 0.f, 0.f);
+    const double4 f = P.frame_F[P.slot_mesh[v]];
+    return make_float3(float(f.x), float(f.y), float(f.z));
+}
 
-// The incidence loop of one lane: records r, r + L, ... below e, the first (`cur`) already
-// loaded; two-stage pipeline (the next record is in flight during this incidence).
-template <int L, typename ST, typename R, int COHERENT>
-__device__ __forceinline__ void accumulate_records(const Ptrs<ST, R>& P, int r, int e, RecRaw<R> cur,
-                                                   const typename ST::U& uo_full, R mu, R lmbd, Acc<R>& acc) {
-    using U = typename ST::U;
-    const U uo = ST::nb(uo_full);
-    while (r < e) {
-        const int rn = r + L;
-        RecRaw<R> nxt;
-        if (rn < e) {
-            if constexpr (COHERENT != kStateStream) nxt.load_kept(P.rec_n, P.rec_a, P.rec_b, P.rec_c, rn);
-            else nxt.load(P.rec_n, P.rec_a, P.rec_b, P.rec_c, rn);
-        }
-        U q0, q1, q2;
-        if constexpr (COHERENT == kStateGrid) {
-            q0 = ST::ldcg(P.u, cur.n.x);
-            q1 = ST::ldcg(P.u, cur.n.y);
-            q2 = ST::ldcg(P.u, cur.n.z);
-        } else if constexpr (COHERENT == kStateBlock) {
-            q0 = ST::ld(P.u, cur.n.x);
-            q1 = ST::ld(P.u, cur.n.y);
-            q2 = ST::ld(P.u, cur.n.z);
-        } else {
-            q0 = ST::ldg(P.u, cur.n.x);
-            q1 = ST::ldg(P.u, cur.n.y);
-            q2 = ST::ldg(P.u, cur.n.z);
-        }
-        R m0[3], m1[3], m2[3];
-        cur.rows(m0, m1, m2);
-        R e0[3], e1[3], e2[3];
-        ST::diff(q0, uo, e0);
-        ST::diff(q1, uo, e1);
-        ST::diff(q2, uo, e2);
-        incidence<R>(e0, e1, e2, m0, m1, m2, mu, lmbd, acc);
-        cur = nxt;
-        r = rn;
+// Whether the vertex can touch the world box: false only where an FP32 estimate of its
+// position is inside by more than the estimate can be off, so that the exact test (which
+// reads the start-of-substep state and, in a mesh frame, X + F as a float pair: 48 bytes
+// more per vertex) runs for the few vertices at the walls. The estimate adds three floats
+// (and rounds the frame offset): its error is below 2^-21 of the sum of their magnitudes.
+// A position that is not finite counts as near.
+template <typename ST, typename R>
+__device__ __forceinline__ bool near_box(const Consts<R>& c, const typename ST::U& uo, const float4& Xo,
+                                         const float3& Fo) {
+    const float4 u = ST::head(uo);
+    const float X[3] = {Xo.x, Xo.y, Xo.z}, F[3] = {Fo.x, Fo.y, Fo.z}, U3[3] = {u.x, u.y, u.z};
+    bool inside = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float x = (X[d] + F[d]) + U3[d];
+        const float m = 4.8e-7f * ((fabsf(X[d]) + fabsf(F[d])) + (fabsf(U3[d]) + fabsf(x)));
+        inside = inside && x - m > c.lo_f[d] + 2.4e-7f * fabsf(c.lo_f[d]) && x + m < c.hi_f[d] - 2.4e-7f * fabsf(c.hi_f[d]);
     }
+    return !inside;
 }
 
 // Bulk prefetch into L2 (no shared memory, no completion to wait for): addr and bytes
@@ -588,128 +795,99 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* addr, uint32_t byte
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(addr), "r"(bytes) : "memory");
 }
 
-// The FP32 records (three 16-byte arrays) of block b of a color launch with blockDim / L
-// vertices per block, prefetched into L2: the block that runs one resident wave later then
-// finds its record stream in L2, and the DRAM reads run ahead of the warps that consume
-// them (a latency-bound sweep keeps more bytes in flight than its warps' registers hold).
+// The record ranges of the vertices [v0, v1): whole slices, from the slice of v0 to the end of
+// the longest list that the slice of v1 - 1 can hold (max_nbr, max_inc per vertex of the
+// color; the arrays are padded by as much).
+struct RecTile {
+    int n0, n1, i0, i1;
+};
+template <typename ST, typename R>
+__device__ __forceinline__ RecTile rec_tile(const Ptrs<ST, R>& P, int v0, int v1, int max_nbr, int max_inc) {
+    const int4 r0 = P.vrec[v0], r1 = P.vrec[v1 - 1];
+    return RecTile{r0.x & ~(kSlice - 1), (r1.x & ~(kSlice - 1)) + kSlice * max_nbr, r0.y & ~(kSlice - 1),
+                   (r1.y & ~(kSlice - 1)) + kSlice * max_inc};
+}
+
+// What the warp `pf` warps on (one resident wave later) will load first, into L2: its records
+// (from their vrec, which this warp loaded ahead), rest positions and tail inputs, and the
+// vrec of the warp as far on again. Every link of a vertex's load chain (vrec, records,
+// neighbours) is then an L2 round trip instead of a DRAM one.
 template <int L, typename ST, typename R>
-__device__ __forceinline__ void prefetch_block_records(const Ptrs<ST, R>& P, int beg, int end, int b) {
-    const int vpb = int(blockDim.x) / L;
-    const long long v0l = (long long)beg + (long long)b * vpb;
-    if (v0l >= end) return;
-    const int v0 = int(v0l), v1 = min(end, v0 + vpb);
-    const int r0 = P.inc_ofs[v0], r1 = P.inc_ofs[v1];
-    if (r1 <= r0) return;
-    const uint32_t bytes = uint32_t(r1 - r0) * 16u;
-    bulk_prefetch_l2(P.rec_n + r0, bytes);
-    bulk_prefetch_l2(P.rec_a + r0, bytes);
-    bulk_prefetch_l2(P.rec_b + r0, bytes);
+__device__ __forceinline__ void prefetch_vertices(const Ptrs<ST, R>& P, int v, int end, int pf, int4 ahead) {
+    const int va = v + pf * Lanes<L>::kW;  // this lane's vertex in that warp
+    if (va >= end) return;
+    if (Lanes<L>::vertex() % kSlice == 0 && Lanes<L>::sub() == 0) {
+        // one lane per slice: the longest list is at most a little longer than its first vertex's
+        bulk_prefetch_l2(P.nbr + (ahead.x & ~(kSlice - 1)), uint32_t(max(ahead.z, 1)) * uint32_t(kSlice * sizeof(NbrRec<R>)));
+        bulk_prefetch_l2(P.inc + (ahead.y & ~(kSlice - 1)), uint32_t(max(ahead.w, 1)) * uint32_t(kSlice * sizeof(IncRec<R>)));
+    }
+    if (Lanes<L>::sub() == L - 1) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(P.rest + va));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(P.y + va));
+        if (va + pf * Lanes<L>::kW < end) asm volatile("prefetch.global.L2 [%0];" ::"l"(P.vrec + va + pf * Lanes<L>::kW));
+    }
 }
 
 // Minimum resident blocks of 256 threads: caps FP32-compute kernels at 64
-// registers (32 warps per SM, no spills); the FP64 kernel keeps its registers.
-template <typename R>
+// registers (32 warps per SM, no spills); the FP64 kernel keeps its registers, as do
+// the wide groups, whose colors are too small to fill the GPU.
+template <int L, typename R>
 struct SolveOcc {
-    static constexpr int kMinBlocks = sizeof(R) == 8 ? 2 : 4;
+    static constexpr int kMinBlocks = sizeof(R) == 8 || L >= 16 ? 2 : 4;
 };
 
-template <int L, typename ST, typename R, bool PROBE>
-__global__ void __launch_bounds__(256, SolveOcc<R>::kMinBlocks)
-    k_solve(Ptrs<ST, R> P, Consts<R> c, int beg, int end, int friction, double* probe_out, int pf) {
+// DEEP (variant 4): asynchronous one-ring copies (narrow groups). MULTI: a scene with a vertex
+// of several segments. pf > 0: prefetch distance in warps.
+// max_nbr: the longest neighbour list of the color, the staging entries per vertex.
+template <int L, typename ST, typename R, bool PROBE, bool DEEP, bool MULTI>
+__global__ void __launch_bounds__(256, SolveOcc<L, R>::kMinBlocks)
+    k_solve(Ptrs<ST, R> P, Consts<R> c, int beg, int end, int friction, double* probe_out, int pf, int max_nbr) {
     using U = typename ST::U;
-    using Sc = typename ST::Sc;
+    constexpr bool kAsync = DEEP && L < 16;
+    constexpr int NB = NbrBatch<L, kAsync>::kN;
+    constexpr int RR = kAsync ? kRecKept : kRecStream;  // neighbour records are read twice
+    extern __shared__ __align__(16) unsigned char smem[];
     pdl_launch_dependents();
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = tid & (L - 1);
-    const int v = beg + tid / L;
+    const int sub = Lanes<L>::sub();
+    const int v = beg + int((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
     const bool valid = v < end;
     Acc<R> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     U uo{};
-    MeshMat<R> mat;
-    int r = 0, e = 0;
-    RecRaw<R> cur;
-    // the records of the block pf blocks ahead (one resident wave later) into L2
-    if constexpr (sizeof(R) == 4 && !PROBE)
-        if (pf > 0 && threadIdx.x == 0) prefetch_block_records<L>(P, beg, end, int(blockIdx.x) + pf);
-    // prologue on static data (records, CSR offsets, materials): overlaps the
-    // previous color's tail when launched as a programmatic dependent
+    MeshMat<R> mat{};
+    float4 Xo = make_float4(0.f, 0.f, 0.f, 0.f);
+    // prologue on static data (records, rest position, materials): overlaps the previous
+    // color's tail when launched as a programmatic dependent
+    int4 seg = make_int4(0, 0, 0, 0);
     if (valid) {
+        seg = P.vrec[v];
+        Xo = __ldg(P.rest + v);
         mat = P.mats[P.slot_mesh[v]];
-        r = P.inc_ofs[v] + lane;
-        e = P.inc_ofs[v + 1];
-        if (r < e) cur.load(P.rec_n, P.rec_a, P.rec_b, P.rec_c, r);
-        if (lane == 0 && !PROBE) prefetch_tail(P, v);
     }
+    SegRecs<R, NB> rec;
+    const Stage<32 / L, ST, R> st = warp_stage<L, ST, R>(smem, max_nbr);
+    if (valid && sub == 0 && !PROBE) prefetch_tail<L>(P, v);
+    float3 Fo = make_float3(0.f, 0.f, 0.f);
+    if constexpr (L >= 16)
+        if (valid && sub == 0) Fo = frame_offset(P, v);
+    preload<L, RR>(rec, P.nbr, P.inc, seg, sub);
+    constexpr bool kPrefetch = sizeof(R) == 4 && !PROBE && !DEEP && L < 16;
+    int4 ahead = make_int4(0, 0, 0, 0);
+    if constexpr (kPrefetch)
+        if (pf > 0 && v + pf * Lanes<L>::kW < end && sub == 0) ahead = P.vrec[v + pf * Lanes<L>::kW];
     pdl_wait();
-    if (valid) {
-        uo = P.u[v];
-        accumulate_records<L, ST, R, kStateStream>(P, r, e, cur, uo, mat.mu, mat.lmbd, acc);
-    }
+    if (valid) uo = P.u[v];
+    const U uon = ST::nb(uo);
+    const FetchGlobal<ST, kStatePlain> fetch{P.u, P.rest};
+    accumulate_segment<L, RR, kAsync, ST>(rec, sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
+    if constexpr (kPrefetch)
+        if (pf > 0) prefetch_vertices<L>(P, v, end, pf, ahead);
+    if constexpr (MULTI)
+        if (valid)
+            accumulate_more<L, RR, kAsync, ST>(rec, P, P.nbr, P.inc, P.vmore[v], sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
     reduce_group<L, R>(acc);
-    if (!valid || lane != 0) return;
-    vertex_tail<ST, R, PROBE>(P, c, v, uo, mat, acc, friction, probe_out, beg, end);
-}
-
-// The same incidence loop with two records in flight beyond the one being computed
-// (`cur` and `nx1` already loaded): more loads outstanding per lane, for colors whose
-// record stream is long enough to need the memory-level parallelism (HBM-bound sweeps).
-template <int L, typename ST, typename R>
-__device__ __forceinline__ void accumulate_records3(const Ptrs<ST, R>& P, int r, int e, RecRaw<R> cur,
-                                                    RecRaw<R> nx1, const typename ST::U& uo_full, R mu, R lmbd,
-                                                    Acc<R>& acc) {
-    using U = typename ST::U;
-    const U uo = ST::nb(uo_full);
-    while (r < e) {
-        const int r2 = r + 2 * L;
-        RecRaw<R> nx2;
-        if (r2 < e) nx2.load(P.rec_n, P.rec_a, P.rec_b, P.rec_c, r2);
-        const U q0 = ST::ldg(P.u, cur.n.x), q1 = ST::ldg(P.u, cur.n.y), q2 = ST::ldg(P.u, cur.n.z);
-        R m0[3], m1[3], m2[3];
-        cur.rows(m0, m1, m2);
-        R e0[3], e1[3], e2[3];
-        ST::diff(q0, uo, e0);
-        ST::diff(q1, uo, e1);
-        ST::diff(q2, uo, e2);
-        incidence<R>(e0, e1, e2, m0, m1, m2, mu, lmbd, acc);
-        cur = nx1;
-        nx1 = nx2;
-        r += L;
-    }
-}
-
-// k_solve with the deeper record pipeline (variant 4): the prologue loads the first two
-// records of each lane before the programmatic-dependency wait. Three resident blocks of
-// 256 threads leave it the registers the second record in flight needs (no spills).
-template <int L, typename ST, typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 2 : 3)
-    k_solve_deep(Ptrs<ST, R> P, Consts<R> c, int beg, int end, int friction) {
-    using U = typename ST::U;
-    pdl_launch_dependents();
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = tid & (L - 1);
-    const int v = beg + tid / L;
-    const bool valid = v < end;
-    Acc<R> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    U uo{};
-    MeshMat<R> mat;
-    int r = 0, e = 0;
-    RecRaw<R> cur, nx1;
-    if (valid) {
-        mat = P.mats[P.slot_mesh[v]];
-        r = P.inc_ofs[v] + lane;
-        e = P.inc_ofs[v + 1];
-        if (r < e) cur.load(P.rec_n, P.rec_a, P.rec_b, P.rec_c, r);
-        if (r + L < e) nx1.load(P.rec_n, P.rec_a, P.rec_b, P.rec_c, r + L);
-        if (lane == 0) prefetch_tail(P, v);
-    }
-    pdl_wait();
-    if (valid) {
-        uo = P.u[v];
-        accumulate_records3<L, ST, R>(P, r, e, cur, nx1, uo, mat.mu, mat.lmbd, acc);
-    }
-    reduce_group<L, R>(acc);
-    if (!valid || lane != 0) return;
-    vertex_tail<ST, R, false>(P, c, v, uo, mat, acc, friction, nullptr, beg, end);
+    if (!valid || sub != 0) return;
+    finish_acc(acc, mat.mu, mat.lmbd);
+    vertex_tail<ST, R, PROBE>(P, c, v, uo, Xo, L >= 16 ? Fo : frame_offset(P, v), mat, acc, friction, probe_out);
 }
 
 // ---- per-vertex tail (lane 0 of a vertex group): damping, inertia, ground and
@@ -717,16 +895,16 @@ __global__ void __launch_bounds__(256, sizeof(R) == 8 ? 2 : 3)
 // The new state goes to P.u[v], or to *unew when given; returns whether the vertex moved.
 template <typename ST, typename R, bool PROBE>
 __device__ __forceinline__ bool vertex_tail(const Ptrs<ST, R>& P, const Consts<R>& c, int v, const typename ST::U& uo,
-                                            const MeshMat<R>& mat, const Acc<R>& acc, int friction,
-                                            double* probe_out, int beg, int end, typename ST::U* unew) {
+                                            const float4& Xo, const float3& Fo, const MeshMat<R>& mat,
+                                            const Acc<R>& acc, int friction, double* probe_out,
+                                            typename ST::U* unew) {
     using U = typename ST::U;
     using Sc = typename ST::Sc;
     R f[3] = {acc.f0, acc.f1, acc.f2};
     R H[6] = {acc.h00 + acc.S, acc.h01, acc.h02, acc.h11 + acc.S, acc.h12, acc.h22 + acc.S};
-    const U xp = P.xprev[v];
-    R dx[3];
-    ST::diff(uo, xp, dx);
     if (mat.kh > R(0) || mat.kd > R(0)) {
+        R dx[3];
+        ST::diff(uo, P.xprev[v], dx);
         // damping Hessian (k_h H_lambda + k_d S I) / dt (VBD_NeoHookean.cpp:562-574)
         R D[6] = {mat.kh * acc.h00 + mat.kd * acc.S, mat.kh * acc.h01, mat.kh * acc.h02,
                   mat.kh * acc.h11 + mat.kd * acc.S, mat.kh * acc.h12, mat.kh * acc.h22 + mat.kd * acc.S};
@@ -758,12 +936,14 @@ __device__ __forceinline__ bool vertex_tail(const Ptrs<ST, R>& P, const Consts<R
         for (int i = 0; i < 6; ++i) H[i] += cs[3 + i];
     }
     // plane ground / world box with friction on each violated axis (VBDPhysics.cpp:2858-2953)
-    if (c.plane) {
+    if (c.plane && near_box<ST, R>(c, uo, Xo, Fo)) {
         // x = X + u, or (X + F) + u in a mesh frame F, X + F held as a float pair per slot
         const bool framed = P.rest_fh != nullptr;
-        const float4 X = framed ? P.rest_fh[v] : P.rest[v];
+        const float4 X = framed ? P.rest_fh[v] : Xo;
         const float4 Xl = framed ? P.rest_fl[v] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float Xc[3] = {X.x, X.y, X.z}, Xlc[3] = {Xl.x, Xl.y, Xl.z};
+        R dx[3];
+        ST::diff(uo, P.xprev[v], dx);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             // below = lo - x, above = x - hi
@@ -819,14 +999,14 @@ __device__ __forceinline__ bool vertex_tail(const Ptrs<ST, R>& P, const Consts<R
 
 // ---------------------------------------------------------------------------
 // TMA-staged solve (FP32 compute). Each block owns vpb = blockDim / L
-// consecutive vertices of the color; their incidence records are one
-// contiguous range [inc_ofs[v0], inc_ofs[v0 + vpb]). Thread 0 stages the range
-// into shared memory with three bulk copies (cp.async.bulk, one per record
-// array) completing on an mbarrier, issued before the programmatic-dependency
-// wait: a block's whole record range is in flight at once, overlapping the
-// previous color's tail, at no register cost. Neighbour positions are gathered
-// as in k_solve. max_rec bounds the records of any block of this launch (the
-// host sizes the dynamic shared memory from it).
+// consecutive vertices of the color; their neighbour and their incidence
+// records are one contiguous range each. Thread 0 stages the ranges into shared
+// memory with two bulk copies (cp.async.bulk) completing on an mbarrier, issued
+// before the programmatic-dependency wait: a block's whole record range is in
+// flight at once, overlapping the previous color's tail, at no register cost.
+// Neighbour positions are gathered as in k_solve. tile_nbr and tile_inc bound the
+// records of any block of this launch (the host sizes the dynamic shared memory
+// from them). Scenes without a vertex of several segments only.
 // ---------------------------------------------------------------------------
 constexpr int kMbarSpinLimit = 1 << 20;
 // Polls of the final drain wait of a block whose first wait ran out, each after a 1 us
@@ -868,78 +1048,66 @@ __device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity) {
     return false;
 }
 
+__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// The copies of a record range (whole slices: 16-byte aligned) on mbarrier `bar` by one thread.
+template <typename ST>
+__device__ __forceinline__ void issue_tile(const Ptrs<ST, float>& P, const RecTile& t, NbrRec<float>* s_nbr,
+                                           IncRec<float>* s_inc, uint32_t bar) {
+    const uint32_t nb = uint32_t(t.n1 - t.n0) * 8u, ib = uint32_t(t.i1 - t.i0) * 8u;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(nb + ib) : "memory");
+    if (nb) bulk_g2s(s_nbr, P.nbr + t.n0, nb, bar);
+    if (ib) bulk_g2s(s_inc, P.inc + t.i0, ib, bar);
+}
+
 template <int L, typename ST>
 __global__ void __launch_bounds__(256, 4)
-    k_solve_tma(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int friction, int max_rec) {
+    k_solve_tma(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int friction, int max_nbr, int max_inc,
+                int tile_nbr, int tile_inc) {
     using U = typename ST::U;
+    constexpr int NB = NbrBatch<L, false>::kN;
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t bar = smem_u32(smem);
-    int4* s_n = reinterpret_cast<int4*>(smem + 16);
-    float4* s_a = reinterpret_cast<float4*>(smem + 16 + 16 * size_t(max_rec));
-    float4* s_b = reinterpret_cast<float4*>(smem + 16 + 32 * size_t(max_rec));
+    NbrRec<float>* s_nbr = reinterpret_cast<NbrRec<float>*>(smem + 16);
+    IncRec<float>* s_inc = reinterpret_cast<IncRec<float>*>(smem + 16 + 8 * size_t(tile_nbr));
+    unsigned char* s_stage = smem + 16 + 8 * (size_t(tile_nbr) + size_t(tile_inc));
     pdl_launch_dependents();
     const int vpb = blockDim.x / L;
     const int v0 = beg + blockIdx.x * vpb;
     const int v1 = min(end, v0 + vpb);
-    const int r0 = P.inc_ofs[v0];
-    const int nrec = min(P.inc_ofs[v1] - r0, max_rec);
+    const RecTile tile = rec_tile(P, v0, v1, max_nbr, max_inc);
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t bytes = uint32_t(nrec) * 16u;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(3u * bytes) : "memory");
-        if (bytes) {
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    smem_u32(s_n)),
-                "l"(P.rec_n + r0), "r"(bytes), "r"(bar)
-                : "memory");
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    smem_u32(s_a)),
-                "l"(P.rec_a + r0), "r"(bytes), "r"(bar)
-                : "memory");
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    smem_u32(s_b)),
-                "l"(P.rec_b + r0), "r"(bytes), "r"(bar)
-                : "memory");
-        }
-    }
-    const int lane = threadIdx.x & (L - 1);
-    const int v = v0 + int(threadIdx.x) / L;
+    if (threadIdx.x == 0) issue_tile(P, tile, s_nbr, s_inc, bar);
+    const int sub = Lanes<L>::sub();
+    const int v = v0 + int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
     const bool valid = v < v1;
-    MeshMat<float> mat;
-    int rb = 0, re = 0;
+    MeshMat<float> mat{};
+    float4 Xo = make_float4(0.f, 0.f, 0.f, 0.f);
+    int4 seg = make_int4(0, 0, 0, 0);
     if (valid) {
+        seg = P.vrec[v];
+        seg.x -= tile.n0;
+        seg.y -= tile.i0;
+        Xo = __ldg(P.rest + v);
         mat = P.mats[P.slot_mesh[v]];
-        rb = P.inc_ofs[v] - r0 + lane;
-        re = min(P.inc_ofs[v + 1] - r0, nrec);
-        if (lane == 0) prefetch_tail(P, v);
+        if (sub == 0) prefetch_tail<L>(P, v);
     }
+    const Stage<32 / L, ST, float> st = warp_stage<L, ST, float>(s_stage, max_nbr);
     pdl_wait();
     U uo{};
     if (valid) uo = P.u[v];
+    const U uon = ST::nb(uo);
     // the block goes on only if every thread saw the records land within the limit
     const bool ok = __syncthreads_and(mbar_wait(bar, 0, c.spin_limit)) != 0;
-    Acc<float> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (valid && ok) {
-        const U uon = ST::nb(uo);
-        for (int r = rb; r < re; r += L) {
-            const int4 n = s_n[r];
-            const float4 a = s_a[r], b = s_b[r];
-            const U q0 = ST::ldg(P.u, n.x), q1 = ST::ldg(P.u, n.y), q2 = ST::ldg(P.u, n.z);
-            const float m0[3] = {a.x, a.y, a.z}, m1[3] = {a.w, b.x, b.y}, m2[3] = {b.z, b.w, f_bits(n.w)};
-            float e0[3], e1[3], e2[3];
-            ST::diff(q0, uon, e0);
-            ST::diff(q1, uon, e1);
-            ST::diff(q2, uon, e2);
-            incidence<float>(e0, e1, e2, m0, m1, m2, mat.mu, mat.lmbd, acc);
-        }
-    }
     if (!ok) {
         // the records did not land within the limit: the block skips its vertices (none
         // moves) and records it, which the host reports as a device-timeout status; thread
@@ -951,9 +1119,105 @@ __global__ void __launch_bounds__(256, 4)
         }
         return;
     }
+    Acc<float> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    SegRecs<float, NB> rec;
+    preload<L, kRecShared>(rec, s_nbr, s_inc, seg, sub);
+    accumulate_segment<L, kRecShared, false, ST>(rec, sub, st, FetchGlobal<ST, kStatePlain>{P.u, P.rest}, uon, Xo, mat.mu, mat.lmbd, acc);
     reduce_group<L, float>(acc);
-    if (!valid || lane != 0) return;
-    vertex_tail<ST, float, false>(P, c, v, uo, mat, acc, friction, nullptr, beg, end);
+    if (!valid || sub != 0) return;
+    finish_acc(acc, mat.mu, mat.lmbd);
+    vertex_tail<ST, float, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr);
+}
+
+// ---------------------------------------------------------------------------
+// Double-buffered TMA pipeline (FP32 compute). A persistent grid walks the color's tiles
+// of vpt = blockDim / L consecutive vertices (tile t of block b: t = b, b + grid, ...). The
+// records of a tile are one contiguous range per array; thread 0 stages the next tile's
+// ranges into the other shared-memory buffer (two cp.async.bulk copies on that buffer's
+// mbarrier) while the block computes the current one, so the record stream of the whole
+// color is in flight ahead of the warps without occupying their registers. Bounded waits as
+// in k_solve_tma: a block whose wait runs out counts a timeout, drains every copy it issued
+// and returns. tile_nbr and tile_inc bound the records of any tile (the host sizes the buffers
+// from them). Scenes without a vertex of several segments only.
+// ---------------------------------------------------------------------------
+template <int L, typename ST>
+__global__ void __launch_bounds__(256)
+    k_solve_pipe(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int friction, int max_nbr, int max_inc,
+                 int tile_nbr, int tile_inc) {
+    using U = typename ST::U;
+    constexpr int NB = NbrBatch<L, false>::kN;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t bar0 = smem_u32(smem);
+    const size_t buf_bytes = 8 * (size_t(tile_nbr) + size_t(tile_inc));
+    auto s_nbr = [&](int b) { return reinterpret_cast<NbrRec<float>*>(smem + 16 + size_t(b) * buf_bytes); };
+    auto s_inc = [&](int b) { return reinterpret_cast<IncRec<float>*>(smem + 16 + size_t(b) * buf_bytes + 8 * size_t(tile_nbr)); };
+    unsigned char* s_stage = smem + 16 + 2 * buf_bytes;
+    const int vpt = int(blockDim.x) / L;
+    const int ntiles = (end - beg + vpt - 1) / vpt;
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    auto tile_of = [&](int t) { return rec_tile(P, beg + t * vpt, min(end, beg + (t + 1) * vpt), max_nbr, max_inc); };
+    // thread 0: the records of tile t into buffer b (records are static: no ordering with
+    // the previous color needed)
+    auto issue = [&](int t, int b) { issue_tile(P, tile_of(t), s_nbr(b), s_inc(b), bar0 + 8u * uint32_t(b)); };
+    if (threadIdx.x == 0 && int(blockIdx.x) < ntiles) issue(int(blockIdx.x), 0);
+    pdl_wait();
+    const int sub = Lanes<L>::sub();
+    const Stage<32 / L, ST, float> st = warp_stage<L, ST, float>(s_stage, max_nbr);
+    int k = 0;
+    for (int t = int(blockIdx.x); t < ntiles; t += int(gridDim.x), ++k) {
+        const int b = k & 1;
+        const uint32_t parity = uint32_t(k >> 1) & 1u;
+        const int tn = t + int(gridDim.x);
+        // the next tile into the other buffer (released by the barrier that ended the last tile)
+        if (threadIdx.x == 0 && tn < ntiles) issue(tn, b ^ 1);
+        const RecTile tile = tile_of(t);
+        const int v0 = beg + t * vpt, v1 = min(end, v0 + vpt);
+        const int v = v0 + int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
+        const bool valid = v < v1;
+        MeshMat<float> mat{};
+        float4 Xo = make_float4(0.f, 0.f, 0.f, 0.f);
+        int4 seg = make_int4(0, 0, 0, 0);
+        U uo{};
+        if (valid) {
+            seg = P.vrec[v];
+            seg.x -= tile.n0;
+            seg.y -= tile.i0;
+            Xo = __ldg(P.rest + v);
+            mat = P.mats[P.slot_mesh[v]];
+            if (sub == 0) prefetch_tail<L>(P, v);
+            uo = P.u[v];
+        }
+        const U uon = ST::nb(uo);
+        const bool ok = __syncthreads_and(mbar_wait(bar0 + 8u * uint32_t(b), parity, c.spin_limit)) != 0;
+        if (!ok) {
+            // this tile's records did not land within the limit: skip the block's remaining
+            // tiles (their vertices do not move), count it, and drain every copy issued (this
+            // tile's and, if issued, the next one's) before the block exits
+            if (threadIdx.x == 0) {
+                atomicAdd(&P.counters[CNT_TIMEOUT], 1ull);
+                bool drained = mbar_drain(bar0 + 8u * uint32_t(b), parity);
+                if (tn < ntiles) drained = mbar_drain(bar0 + 8u * uint32_t(b ^ 1), uint32_t((k + 1) >> 1) & 1u) && drained;
+                if (!drained) atomicAdd(&P.counters[CNT_DRAIN], 1ull);
+            }
+            return;
+        }
+        Acc<float> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+        SegRecs<float, NB> rec;
+        preload<L, kRecShared>(rec, s_nbr(b), s_inc(b), seg, sub);
+        accumulate_segment<L, kRecShared, false, ST>(rec, sub, st, FetchGlobal<ST, kStatePlain>{P.u, P.rest}, uon, Xo, mat.mu, mat.lmbd, acc);
+        reduce_group<L, float>(acc);
+        if (valid && sub == 0) {
+            finish_acc(acc, mat.mu, mat.lmbd);
+            vertex_tail<ST, float, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr);
+        }
+        __syncthreads();  // every read of buffer b done before the next iteration refills it
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -969,143 +1233,55 @@ __global__ void __launch_bounds__(256, 4)
 // are mesh m's color slot ranges in sweep order. MAXB bounds the block size (and so the
 // registers a thread may use: 256 leaves the compiler all it needs, 1024 caps it at 64).
 // ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
-// Double-buffered TMA pipeline (FP32 compute). A persistent grid walks the color's tiles
-// of vpt = blockDim / L consecutive vertices (tile t of block b: t = b, b + grid, ...). The
-// records of a tile are one contiguous range; thread 0 stages the next tile's range into
-// the other shared-memory buffer (three cp.async.bulk copies on that buffer's mbarrier)
-// while the block computes the current one, so the record stream of the whole color is in
-// flight ahead of the warps without occupying their registers. Each lane then prefetches
-// the neighbour states of its next incidence (ids from shared memory) before evaluating the
-// current one: two incidences' gathers in flight per lane. Bounded waits as in k_solve_tma:
-// a block whose wait runs out counts a timeout, drains every copy it issued and returns.
-// max_rec bounds the records of any tile (the host sizes the buffers from it).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
 
-template <int L, typename ST>
-__global__ void __launch_bounds__(256)
-    k_solve_pipe(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int friction, int max_rec) {
+// One vertex group's solve inside a persistent sweep, its state and its neighbours' read with
+// Fetch. Every lane of the warp calls it; v is the group's vertex when valid. cap: staged
+// neighbours per vertex.
+template <int L, bool MULTI, typename ST, typename R, typename Fetch>
+__device__ __forceinline__ void solve_in_sweep(const Ptrs<ST, R>& P, const Consts<R>& c, int v, bool valid, int sub,
+                                               unsigned char* smem, int cap, const Fetch& fetch,
+                                               const typename ST::U& uo, int friction) {
     using U = typename ST::U;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t bar0 = smem_u32(smem);
-    const size_t buf_bytes = 48 * size_t(max_rec);
-    auto s_n = [&](int b) { return reinterpret_cast<int4*>(smem + 16 + size_t(b) * buf_bytes); };
-    auto s_a = [&](int b) { return reinterpret_cast<float4*>(smem + 16 + size_t(b) * buf_bytes + 16 * size_t(max_rec)); };
-    auto s_b = [&](int b) { return reinterpret_cast<float4*>(smem + 16 + size_t(b) * buf_bytes + 32 * size_t(max_rec)); };
-    const int vpt = int(blockDim.x) / L;
-    const int ntiles = (end - beg + vpt - 1) / vpt;
-    pdl_launch_dependents();
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    constexpr bool kAsync = L < 16;
+    constexpr int NB = NbrBatch<L, kAsync>::kN;
+    Acc<R> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    MeshMat<R> mat{};
+    float4 Xo = make_float4(0.f, 0.f, 0.f, 0.f);
+    int4 seg = make_int4(0, 0, 0, 0);
+    if (valid) {
+        seg = __ldg(P.vrec + v);
+        Xo = __ldg(P.rest + v);
+        mat = P.mats[P.slot_mesh[v]];
     }
-    __syncthreads();
-    // thread 0: the records of tile t into buffer b (records are static: no ordering with
-    // the previous color needed)
-    auto issue = [&](int t, int b) {
-        const int v0 = beg + t * vpt, v1 = min(end, v0 + vpt);
-        const int r0 = P.inc_ofs[v0];
-        const uint32_t bytes = uint32_t(min(P.inc_ofs[v1] - r0, max_rec)) * 16u;
-        const uint32_t bar = bar0 + 8u * uint32_t(b);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(3u * bytes) : "memory");
-        if (bytes) {
-            bulk_g2s(s_n(b), P.rec_n + r0, bytes, bar);
-            bulk_g2s(s_a(b), P.rec_a + r0, bytes, bar);
-            bulk_g2s(s_b(b), P.rec_b + r0, bytes, bar);
-        }
-    };
-    if (threadIdx.x == 0 && int(blockIdx.x) < ntiles) issue(int(blockIdx.x), 0);
-    pdl_wait();
-    const int lane = int(threadIdx.x) & (L - 1);
-    int k = 0;
-    for (int t = int(blockIdx.x); t < ntiles; t += int(gridDim.x), ++k) {
-        const int b = k & 1;
-        const uint32_t parity = uint32_t(k >> 1) & 1u;
-        const int tn = t + int(gridDim.x);
-        // the next tile into the other buffer (released by the barrier that ended the last tile)
-        if (threadIdx.x == 0 && tn < ntiles) issue(tn, b ^ 1);
-        const int v0 = beg + t * vpt, v1 = min(end, v0 + vpt);
-        const int r0 = P.inc_ofs[v0];
-        const int nrec = min(P.inc_ofs[v1] - r0, max_rec);
-        const int v = v0 + int(threadIdx.x) / L;
-        const bool valid = v < v1;
-        MeshMat<float> mat;
-        int rb = 0, re = 0;
-        U uo{};
-        if (valid) {
-            mat = P.mats[P.slot_mesh[v]];
-            rb = P.inc_ofs[v] - r0 + lane;
-            re = min(P.inc_ofs[v + 1] - r0, nrec);
-            if (lane == 0) prefetch_tail(P, v);
-            uo = P.u[v];
-        }
-        const bool ok = __syncthreads_and(mbar_wait(bar0 + 8u * uint32_t(b), parity, c.spin_limit)) != 0;
-        if (!ok) {
-            // this tile's records did not land within the limit: skip the block's remaining
-            // tiles (their vertices do not move), count it, and drain every copy issued (this
-            // tile's and, if issued, the next one's) before the block exits
-            if (threadIdx.x == 0) {
-                atomicAdd(&P.counters[CNT_TIMEOUT], 1ull);
-                bool drained = mbar_drain(bar0 + 8u * uint32_t(b), parity);
-                if (tn < ntiles) drained = mbar_drain(bar0 + 8u * uint32_t(b ^ 1), uint32_t((k + 1) >> 1) & 1u) && drained;
-                if (!drained) atomicAdd(&P.counters[CNT_DRAIN], 1ull);
-            }
-            return;
-        }
-        Acc<float> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-        if (valid && rb < re) {
-            const int4* sn = s_n(b);
-            const float4* sa = s_a(b);
-            const float4* sb = s_b(b);
-            const U uon = ST::nb(uo);
-            int4 n = sn[rb];
-            U q0 = ST::ldg(P.u, n.x), q1 = ST::ldg(P.u, n.y), q2 = ST::ldg(P.u, n.z);
-            for (int r = rb; r < re; r += L) {
-                const int rn = r + L;
-                int4 nn = n;
-                U p0 = q0, p1 = q1, p2 = q2;
-                if (rn < re) {  // the next incidence's gathers in flight during this one
-                    nn = sn[rn];
-                    p0 = ST::ldg(P.u, nn.x);
-                    p1 = ST::ldg(P.u, nn.y);
-                    p2 = ST::ldg(P.u, nn.z);
-                }
-                const float4 a = sa[r], bb = sb[r];
-                const float m0[3] = {a.x, a.y, a.z}, m1[3] = {a.w, bb.x, bb.y}, m2[3] = {bb.z, bb.w, f_bits(n.w)};
-                float e0[3], e1[3], e2[3];
-                ST::diff(q0, uon, e0);
-                ST::diff(q1, uon, e1);
-                ST::diff(q2, uon, e2);
-                incidence<float>(e0, e1, e2, m0, m1, m2, mat.mu, mat.lmbd, acc);
-                n = nn;
-                q0 = p0;
-                q1 = p1;
-                q2 = p2;
-            }
-        }
-        reduce_group<L, float>(acc);
-        if (valid && lane == 0) vertex_tail<ST, float, false>(P, c, v, uo, mat, acc, friction, nullptr, beg, end);
-        __syncthreads();  // every read of buffer b done before the next iteration refills it
+    SegRecs<R, NB> rec;
+    const Stage<32 / L, ST, R> st = warp_stage<L, ST, R>(smem, cap);
+    preload<L, kRecKept>(rec, P.nbr, P.inc, seg, sub);
+    if (valid && sub == 0) prefetch_tail<L>(P, v);
+    const U uon = ST::nb(uo);
+    accumulate_segment<L, kRecKept, kAsync, ST>(rec, sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
+    if constexpr (MULTI)
+        if (valid)
+            accumulate_more<L, kRecKept, kAsync, ST>(rec, P, P.nbr, P.inc, P.vmore[v], sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
+    __syncwarp();  // the staging area is written again by the warp's next vertices
+    reduce_group<L, R>(acc);
+    if (valid && sub == 0) {
+        finish_acc(acc, mat.mu, mat.lmbd);
+        vertex_tail<ST, R, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr);
     }
 }
 
-template <int L, typename ST, typename R, int MAXB>
+template <int L, bool MULTI, typename ST, typename R, int MAXB>
 __global__ void __launch_bounds__(MAXB) k_sweep_scenes(Ptrs<ST, R> P, Consts<R> c, const int2* colors,
                                                        const int32_t* scene_ofs, const int32_t* scene_order,
                                                        int32_t nscenes, int32_t iterations, int32_t friction_start,
-                                                       int32_t* work) {
+                                                       int32_t* work, int cap) {
     using U = typename ST::U;
+    extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_scene;
     const int groups = int(blockDim.x) / L;
-    const int g = int(threadIdx.x) / L;
-    const int lane = int(threadIdx.x) & (L - 1);
+    const int g = int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
+    const int sub = Lanes<L>::sub();
+    const FetchGlobal<ST, kStatePlain> fetch{P.u, P.rest};
     for (;;) {
         if (threadIdx.x == 0) s_scene = atomicAdd(work, 1);
         __syncthreads();
@@ -1121,20 +1297,9 @@ __global__ void __launch_bounds__(MAXB) k_sweep_scenes(Ptrs<ST, R> P, Consts<R> 
                 for (int base = rg.x; base < rg.y; base += groups) {
                     const int v = base + g;
                     const bool valid = v < rg.y;
-                    Acc<R> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
                     U uo{};
-                    MeshMat<R> mat;
-                    if (valid) {
-                        mat = P.mats[P.slot_mesh[v]];
-                        const int r = P.inc_ofs[v] + lane, e = P.inc_ofs[v + 1];
-                        RecRaw<R> cur;
-                        if (r < e) cur.load_kept(P.rec_n, P.rec_a, P.rec_b, P.rec_c, r);
-                        if (lane == 0) prefetch_tail(P, v);
-                        uo = ST::ld_own(P.u, v);
-                        accumulate_records<L, ST, R, kStateBlock>(P, r, e, cur, uo, mat.mu, mat.lmbd, acc);
-                    }
-                    reduce_group<L, R>(acc);
-                    if (valid && lane == 0) vertex_tail<ST, R, false>(P, c, v, uo, mat, acc, friction, nullptr, rg.x, rg.y);
+                    if (valid) uo = ST::ld_own(P.u, v);
+                    solve_in_sweep<L, MULTI, ST, R>(P, c, v, valid, sub, smem, cap, fetch, uo, friction);
                 }
                 __syncthreads();  // this color's updates before the next color reads them
             }

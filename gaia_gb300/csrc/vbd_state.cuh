@@ -9,7 +9,7 @@
 //   StDFH : StDF state whose neighbour reads load the FP32 high part only (see below)
 //   StF64 : displacement as FP64                          (32 B per vertex, w = mass)
 //
-// Each trait provides read-only (ldg) and coherent (ld) loads, a - b rounded to the
+// Each trait provides coherent (ld) and L2 (ldcg) loads, a - b rounded to the
 // compute type R, a + d for a delta d in the velocity type, conversions from
 // and to double, and (c - X - u) for the world-box tests.
 #pragma once
@@ -49,17 +49,14 @@ struct StF32 {
     using V = R4<float>;
     using Sc = float;
     static constexpr int kCode = 32;  // gaia_vbd_stats.precision
+    static constexpr int kNbParts = 1;  // 16-byte parts of a state that the incidence loop reads
     __host__ __device__ static U from_d(const double* x, double w) {
         return U{float(x[0]), float(x[1]), float(x[2]), float(w)};
     }
     __device__ static void to_d(const U& u, double* x) { x[0] = u.x; x[1] = u.y; x[2] = u.z; }
     __device__ static Sc mass(const U& u) { return u.w; }
-    __device__ static U ldg(const U* p, int i) {
-        float4 v = __ldg(reinterpret_cast<const float4*>(p) + i);
-        return U{v.x, v.y, v.z, v.w};
-    }
-    // coherent load: for state written earlier in the same kernel by the same block
-    // (ordered by a block barrier)
+    // coherent load: for state written by earlier launches, or earlier in the same kernel by
+    // the same block (ordered by a block barrier)
     __device__ static U ld(const U* p, int i) {
         float4 v = reinterpret_cast<const float4*>(p)[i];
         return U{v.x, v.y, v.z, v.w};
@@ -109,14 +106,10 @@ struct StF64 {
     using V = R4<double>;
     using Sc = double;
     static constexpr int kCode = 64;
+    static constexpr int kNbParts = 2;
     __host__ __device__ static U from_d(const double* x, double w) { return U{x[0], x[1], x[2], w}; }
     __device__ static void to_d(const U& u, double* x) { x[0] = u.x; x[1] = u.y; x[2] = u.z; }
     __device__ static Sc mass(const U& u) { return u.w; }
-    __device__ static U ldg(const U* p, int i) {
-        const double2* q = reinterpret_cast<const double2*>(p + i);
-        double2 a = __ldg(q), b = __ldg(q + 1);
-        return U{a.x, a.y, b.x, b.y};
-    }
     __device__ static U ld(const U* p, int i) {
         const double2* q = reinterpret_cast<const double2*>(p + i);
         double2 a = q[0], b = q[1];
@@ -161,6 +154,7 @@ struct StDF {
     using V = R4<float>;
     using Sc = float;
     static constexpr int kCode = 48;
+    static constexpr int kNbParts = 2;
     __host__ __device__ static U from_d(const double* x, double w) {
         U u;
         u.hx = float(x[0]); u.lx = float(x[0] - double(u.hx));
@@ -176,11 +170,6 @@ struct StDF {
         x[2] = double(u.hz) + double(u.lz);
     }
     __device__ static Sc mass(const U& u) { return u.w; }
-    __device__ static U ldg(const U* p, int i) {
-        const float4* q = reinterpret_cast<const float4*>(p + i);
-        float4 a = __ldg(q), b = __ldg(q + 1);
-        return U{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    }
     __device__ static U ld(const U* p, int i) {
         const float4* q = reinterpret_cast<const float4*>(p + i);
         float4 a = q[0], b = q[1];
@@ -239,10 +228,7 @@ struct StDF {
 // FP32 mode's accumulation of rounded updates.
 struct StDFH : StDF {
     static constexpr int kCode = 40;
-    __device__ static U ldg(const U* p, int i) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p + i));
-        return U{a.x, a.y, a.z, a.w, 0.f, 0.f, 0.f, 0.f};
-    }
+    static constexpr int kNbParts = 1;
     __device__ static U ld(const U* p, int i) {
         const float4 a = reinterpret_cast<const float4*>(p + i)[0];
         return U{a.x, a.y, a.z, a.w, 0.f, 0.f, 0.f, 0.f};
