@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
                     int moved = 0;
                     if (valid && sub == 0) {
                         finish_acc(acc, mat.mu, mat.lmbd);
-                        moved = vertex_tail<ST, R, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr, &un) ? 1 : 0;
+                        moved = vertex_tail<ST, R, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr, nullptr, &un) ? 1 : 0;
                     }
                     const int src = Lanes<L>::vertex();
                     moved = __shfl_sync(0xffffffffu, moved, src);

@@ -152,7 +152,8 @@ struct Ptrs {
     const int4* col_own;
     const int32_t* col_rel;
     const double2* mesh_fric;      // per mesh: frictionDynamic, frictionEpsV
-    R* col_scratch;                // 9 per slot: contact force (3) and Hessian (6) of the solve
+    typename ST::U* snap;          // 2 per slot: states of the vertices with contact records as they
+                                   // were after the previous iteration's solve of their color
     // mesh frames (null when off): per mesh the shift that the substep's initial step takes
     // out of every state of the mesh and the frame offset F (FP64); per slot the reference
     // position X + F as a float pair, which the world-box test uses in place of X
@@ -612,7 +613,7 @@ template <typename ST, typename R, bool PROBE>
 __device__ __forceinline__ bool vertex_tail(const Ptrs<ST, R>& P, const Consts<R>& c, int v, const typename ST::U& uo,
                                             const float4& Xo, const float3& Fo, const MeshMat<R>& mat,
                                             const Acc<R>& acc, int friction, double* probe_out,
-                                            typename ST::U* unew = nullptr);
+                                            const R* con, typename ST::U* unew = nullptr);
 
 // ---------------------------------------------------------------------------
 // Tet-mesh vertex-face contact (VBDPhysicsCompute.cu:1731-1773, 1812-1930)
@@ -634,21 +635,24 @@ struct V3T<double> {
 // (X_q - X_p) + (u_q - u_p). Penalty k * depth along the face normal (interior closest
 // point) or the closest-point direction oriented like the face normal, lagged IPC
 // friction in the frame (edge AB, AB x n); scaled by b = 1 (sp) or -barycentric.
-template <typename ST, typename R>
-__device__ __forceinline__ void contact_term(const Ptrs<ST, R>& P, const Consts<R>& c, int sp, int order, R* f,
-                                             R* H) {
+template <typename ST, typename R, typename Get>
+__device__ __forceinline__ void contact_term(const Ptrs<ST, R>& P, const Consts<R>& c, const Get& state, int sp,
+                                             int order, R* f, R* H) {
     using U = typename ST::U;
     using V = typename V3T<R>::type;
     const int4 fo = P.col_own[sp];
     const int fs[3] = {fo.x, fo.y, fo.z};
-    const U up = P.u[sp];
+    const U up = state(sp);
+    U uf[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) uf[k] = state(fs[k]);
     const float4 Xp = P.rest[sp];
     V q[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float4 Xq = P.rest[fs[k]];
         R d[3];
-        ST::diff(P.u[fs[k]], up, d);
+        ST::diff(uf[k], up, d);
         q[k] = V{R(Xq.x) - R(Xp.x) + d[0], R(Xq.y) - R(Xp.y) + d[1], R(Xq.z) - R(Xp.z) + d[2]};
     }
     const V o{R(0), R(0), R(0)};
@@ -683,7 +687,7 @@ __device__ __forceinline__ void contact_term(const Ptrs<ST, R>& P, const Consts<
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         R dk[3];
-        ST::diff(P.u[fs[k]], P.xprev[fs[k]], dk);
+        ST::diff(uf[k], P.xprev[fs[k]], dk);
         dx[0] -= bk[k] * dk[0];
         dx[1] -= bk[k] * dk[1];
         dx[2] -= bk[k] * dk[2];
@@ -703,44 +707,57 @@ __device__ __forceinline__ void contact_term(const Ptrs<ST, R>& P, const Consts<
     cloth::friction<R>(mu, lambda, ta, tb, u0, u1, epsU, b, f, H);
 }
 
-// accumulateCollisionForceAndHessian (VBDPhysicsCompute.cu:1731-1773) for the vertices
-// with contact records in the slot range [beg, end) of one color, evaluated just before
-// that color's solve kernel: the vertex's own contact, then its relations, summed into
-// its 9 scratch values, which the solve adds between inertia and boundary. Running
-// before the color's solve, every read sees the positions of earlier colors updated and
-// those of this color not yet, which is the reference's Jacobi-within-color update
-// (positionsNew, VBDPhysicsCompute.cu:803-908). `list` holds the slots with records,
-// ascending, so a color's vertices are one sub-range.
-template <typename ST, typename R>
-__global__ void __launch_bounds__(128) k_contact_color(Ptrs<ST, R> P, Consts<R> c, int beg, int end,
-                                                       const int32_t* list, const int32_t* nlist) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int n = *nlist;
-    auto lower = [&](int key) {
-        int lo = 0, hi = n;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (list[mid] < key) lo = mid + 1;
-            else hi = mid;
+// Flags of a solve launch: friction on, and which half of the contact snapshots this iteration
+// writes (it reads the other one).
+enum { kSolveFriction = 1, kSolveParity = 2 };
+
+// accumulateCollisionForceAndHessian (VBDPhysicsCompute.cu:1731-1773) of a vertex with contact
+// records (info != 0): its own contact and its relations, at most five terms, one per lane of
+// its group where the group is wide enough, summed into con (force 3, Hessian 6), which the
+// solve adds between inertia and boundary. The vertices of the running color [beg, end) enter
+// as they were before this launch (their snapshots: a contact partner can share the vertex's
+// color and be updated by this very launch), all others as they are, which is the reference's
+// Jacobi-within-color update (positionsNew, VBDPhysicsCompute.cu:803-908). Evaluated by a
+// kernel of its own before each color, one thread per vertex, the terms of a vertex ran one
+// after another and every color paid a second launch: 14 us per color on four small bodies in
+// contact, 7.5 us with the terms here. Every lane of the warp calls it.
+template <int L, typename ST, typename R>
+__device__ __forceinline__ void contact_sums(const Ptrs<ST, R>& P, const Consts<R>& c, int v, int info, int sub, int beg,
+                                          int end, int flags, R* con) {
+    using U = typename ST::U;
+    const U* before = P.snap + ((flags & kSolveParity) ? 0 : size_t(P.nslots));
+    const auto state = [&](int s) { return s >= beg && s < end ? before[s] : P.u[s]; };
+    for (int j = sub; j < 5; j += L) {
+        if (j == 0) {
+            if (info & 8) contact_term<ST, R>(P, c, state, v, 3, con, con + 3);
+        } else if (j - 1 < (info & 7)) {
+            const int e = P.col_rel[4 * v + j - 1];
+            contact_term<ST, R>(P, c, state, e >> 2, e & 3, con, con + 3);
         }
-        return lo;
-    };
-    const int i0 = lower(beg), i1 = lower(end);
-    for (int i = i0 + int(blockIdx.x * blockDim.x + threadIdx.x); i < i1; i += int(gridDim.x * blockDim.x)) {
-        const int v = list[i];
-        const int info = P.col_info[v];
-        R f[3] = {R(0), R(0), R(0)}, H[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
-        if (info & 8) contact_term<ST, R>(P, c, v, 3, f, H);
-        const int nrel = info & 7;
-        for (int j = 0; j < nrel; ++j) {
-            const int e = P.col_rel[4 * v + j];
-            contact_term<ST, R>(P, c, e >> 2, e & 3, f, H);
-        }
-        R* o = P.col_scratch + 9 * size_t(v);
-        o[0] = f[0]; o[1] = f[1]; o[2] = f[2];
+    }
 #pragma unroll
-        for (int k = 0; k < 6; ++k) o[3 + k] = H[k];
+    for (int off = 16; off >= 32 / L; off >>= 1)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) con[k] += __shfl_xor_sync(0xffffffffu, con[k], off);
+}
+
+// The same as a call: in the narrow groups of large colors few warps take it, and the solve of
+// the others keeps its registers.
+template <int L, typename ST, typename R>
+__device__ __noinline__ void contact_sums_call(const Ptrs<ST, R>& P, const Consts<R>& c, int v, int info, int sub,
+                                               int beg, int end, int flags, R* con) {
+    contact_sums<L, ST, R>(P, c, v, info, sub, beg, end, flags, con);
+}
+
+// The snapshots of the vertices with contact records that the first solve of each color after
+// a detection reads: the current states, into half `half`.
+template <typename ST>
+__global__ void k_contact_snapshot(const typename ST::U* u, typename ST::U* snap, int32_t nslots, int half,
+                                   const int32_t* list, const int32_t* nlist) {
+    const int n = *nlist;
+    for (int i = int(blockIdx.x * blockDim.x + threadIdx.x); i < n; i += int(gridDim.x * blockDim.x)) {
+        const int v = list[i];
+        snap[size_t(half) * nslots + v] = u[v];
     }
 }
 
@@ -828,6 +845,12 @@ __device__ __forceinline__ void prefetch_vertices(const Ptrs<ST, R>& P, int v, i
     }
 }
 
+template <int L, bool PROBE, bool CONTACT, typename ST, typename R>
+__device__ __forceinline__ void finish_vertex(const Ptrs<ST, R>& P, const Consts<R>& c, int v, bool valid, int sub,
+                                              const typename ST::U& uo, const float4& Xo, const float3& Fo,
+                                              const MeshMat<R>& mat, Acc<R>& acc, int info, int beg, int end, int flags,
+                                              double* probe_out);
+
 // Minimum resident blocks of 256 threads: caps FP32-compute kernels at 64
 // registers (32 warps per SM, no spills); the FP64 kernel keeps its registers, as do
 // the wide groups, whose colors are too small to fill the GPU.
@@ -839,9 +862,9 @@ struct SolveOcc {
 // DEEP (variant 4): asynchronous one-ring copies (narrow groups). MULTI: a scene with a vertex
 // of several segments. pf > 0: prefetch distance in warps.
 // max_nbr: the longest neighbour list of the color, the staging entries per vertex.
-template <int L, typename ST, typename R, bool PROBE, bool DEEP, bool MULTI>
+template <int L, typename ST, typename R, bool PROBE, bool DEEP, bool MULTI, bool CONTACT>
 __global__ void __launch_bounds__(256, SolveOcc<L, R>::kMinBlocks)
-    k_solve(Ptrs<ST, R> P, Consts<R> c, int beg, int end, int friction, double* probe_out, int pf, int max_nbr) {
+    k_solve(Ptrs<ST, R> P, Consts<R> c, int beg, int end, int flags, double* probe_out, int pf, int max_nbr) {
     using U = typename ST::U;
     constexpr bool kAsync = DEEP && L < 16;
     constexpr int NB = NbrBatch<L, kAsync>::kN;
@@ -875,7 +898,11 @@ __global__ void __launch_bounds__(256, SolveOcc<L, R>::kMinBlocks)
     if constexpr (kPrefetch)
         if (pf > 0 && v + pf * Lanes<L>::kW < end && sub == 0) ahead = P.vrec[v + pf * Lanes<L>::kW];
     pdl_wait();
-    if (valid) uo = P.u[v];
+    int info = 0;
+    if (valid) {
+        uo = P.u[v];
+        if constexpr (CONTACT) info = P.col_info[v];
+    }
     const U uon = ST::nb(uo);
     const FetchGlobal<ST, kStatePlain> fetch{P.u, P.rest};
     accumulate_segment<L, RR, kAsync, ST>(rec, sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
@@ -885,19 +912,20 @@ __global__ void __launch_bounds__(256, SolveOcc<L, R>::kMinBlocks)
         if (valid)
             accumulate_more<L, RR, kAsync, ST>(rec, P, P.nbr, P.inc, P.vmore[v], sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
     reduce_group<L, R>(acc);
-    if (!valid || sub != 0) return;
-    finish_acc(acc, mat.mu, mat.lmbd);
-    vertex_tail<ST, R, PROBE>(P, c, v, uo, Xo, L >= 16 ? Fo : frame_offset(P, v), mat, acc, friction, probe_out);
+    if constexpr (L < 16)
+        if (valid && sub == 0) Fo = frame_offset(P, v);
+    finish_vertex<L, PROBE, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, beg, end, flags, probe_out);
 }
 
 // ---- per-vertex tail (lane 0 of a vertex group): damping, inertia, ground and
 // friction, 3x3 solve, update ------------------------------------------------------
-// The new state goes to P.u[v], or to *unew when given; returns whether the vertex moved.
+// con: the vertex's contact sums (null: none). The new state goes to P.u[v], or to *unew when
+// given; returns whether the vertex moved.
 template <typename ST, typename R, bool PROBE>
 __device__ __forceinline__ bool vertex_tail(const Ptrs<ST, R>& P, const Consts<R>& c, int v, const typename ST::U& uo,
                                             const float4& Xo, const float3& Fo, const MeshMat<R>& mat,
                                             const Acc<R>& acc, int friction, double* probe_out,
-                                            typename ST::U* unew) {
+                                            const R* con, typename ST::U* unew) {
     using U = typename ST::U;
     using Sc = typename ST::Sc;
     R f[3] = {acc.f0, acc.f1, acc.f2};
@@ -927,13 +955,11 @@ __device__ __forceinline__ bool vertex_tail(const Ptrs<ST, R>& P, const Consts<R
         f[2] += w * dy[2];
         H[0] += w; H[3] += w; H[5] += w;
     }
-    // tet-mesh contact (between inertia and boundary, VBDPhysicsCompute.cu:893-895),
-    // evaluated by k_contact_color just before this color
-    if (P.col_info && P.col_info[v]) {
-        const R* cs = P.col_scratch + 9 * size_t(v);
-        f[0] += cs[0]; f[1] += cs[1]; f[2] += cs[2];
+    // tet-mesh contact (between inertia and boundary, VBDPhysicsCompute.cu:893-895)
+    if (con) {
+        f[0] += con[0]; f[1] += con[1]; f[2] += con[2];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) H[i] += cs[3 + i];
+        for (int i = 0; i < 6; ++i) H[i] += con[3 + i];
     }
     // plane ground / world box with friction on each violated axis (VBDPhysics.cpp:2858-2953)
     if (c.plane && near_box<ST, R>(c, uo, Xo, Fo)) {
@@ -995,6 +1021,36 @@ __device__ __forceinline__ bool vertex_tail(const Ptrs<ST, R>& P, const Consts<R
     if (unew) *unew = ST::add(uo, s0, s1, s2);
     else P.u[v] = ST::add(uo, s0, s1, s2);
     return true;
+}
+
+// The end of a color launch for one vertex group: contact sums (CONTACT: scenes with contact
+// detection), the tail on sub-lane 0 and the vertex's contact snapshot for the next iteration.
+// Every lane of the warp calls it, with the reduced sums.
+template <int L, bool PROBE, bool CONTACT, typename ST, typename R>
+__device__ __forceinline__ void finish_vertex(const Ptrs<ST, R>& P, const Consts<R>& c, int v, bool valid, int sub,
+                                              const typename ST::U& uo, const float4& Xo, const float3& Fo,
+                                              const MeshMat<R>& mat, Acc<R>& acc, int info, int beg, int end, int flags,
+                                              double* probe_out) {
+    if constexpr (CONTACT) {
+        R con[9] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
+        const bool some = __any_sync(0xffffffffu, info != 0);
+        if (some) {
+            if constexpr (L >= 16) contact_sums<L, ST, R>(P, c, v, info, sub, beg, end, flags, con);
+            else contact_sums_call<L, ST, R>(P, c, v, info, sub, beg, end, flags, con);
+        }
+        if (!valid || sub != 0) return;
+        finish_acc(acc, mat.mu, mat.lmbd);
+        typename ST::U un = uo;
+        const bool moved = vertex_tail<ST, R, PROBE>(P, c, v, uo, Xo, Fo, mat, acc, flags & kSolveFriction, probe_out,
+                                                     info ? con : nullptr, &un);
+        if (PROBE) return;
+        if (moved) P.u[v] = un;
+        if (info) P.snap[((flags & kSolveParity) ? size_t(P.nslots) : 0) + v] = moved ? un : uo;
+    } else {
+        if (!valid || sub != 0) return;
+        finish_acc(acc, mat.mu, mat.lmbd);
+        vertex_tail<ST, R, PROBE>(P, c, v, uo, Xo, Fo, mat, acc, flags & kSolveFriction, probe_out, nullptr);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1065,9 +1121,9 @@ __device__ __forceinline__ void issue_tile(const Ptrs<ST, float>& P, const RecTi
     if (ib) bulk_g2s(s_inc, P.inc + t.i0, ib, bar);
 }
 
-template <int L, typename ST>
+template <int L, bool CONTACT, typename ST>
 __global__ void __launch_bounds__(256, 4)
-    k_solve_tma(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int friction, int max_nbr, int max_inc,
+    k_solve_tma(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int flags, int max_nbr, int max_inc,
                 int tile_nbr, int tile_inc) {
     using U = typename ST::U;
     constexpr int NB = NbrBatch<L, false>::kN;
@@ -1104,7 +1160,11 @@ __global__ void __launch_bounds__(256, 4)
     const Stage<32 / L, ST, float> st = warp_stage<L, ST, float>(s_stage, max_nbr);
     pdl_wait();
     U uo{};
-    if (valid) uo = P.u[v];
+    int info = 0;
+    if (valid) {
+        uo = P.u[v];
+        if constexpr (CONTACT) info = P.col_info[v];
+    }
     const U uon = ST::nb(uo);
     // the block goes on only if every thread saw the records land within the limit
     const bool ok = __syncthreads_and(mbar_wait(bar, 0, c.spin_limit)) != 0;
@@ -1124,9 +1184,8 @@ __global__ void __launch_bounds__(256, 4)
     preload<L, kRecShared>(rec, s_nbr, s_inc, seg, sub);
     accumulate_segment<L, kRecShared, false, ST>(rec, sub, st, FetchGlobal<ST, kStatePlain>{P.u, P.rest}, uon, Xo, mat.mu, mat.lmbd, acc);
     reduce_group<L, float>(acc);
-    if (!valid || sub != 0) return;
-    finish_acc(acc, mat.mu, mat.lmbd);
-    vertex_tail<ST, float, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr);
+    const float3 Fo = valid && sub == 0 ? frame_offset(P, v) : make_float3(0.f, 0.f, 0.f);
+    finish_vertex<L, false, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, beg, end, flags, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1140,9 +1199,9 @@ __global__ void __launch_bounds__(256, 4)
 // and returns. tile_nbr and tile_inc bound the records of any tile (the host sizes the buffers
 // from them). Scenes without a vertex of several segments only.
 // ---------------------------------------------------------------------------
-template <int L, typename ST>
+template <int L, bool CONTACT, typename ST>
 __global__ void __launch_bounds__(256)
-    k_solve_pipe(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int friction, int max_nbr, int max_inc,
+    k_solve_pipe(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int flags, int max_nbr, int max_inc,
                  int tile_nbr, int tile_inc) {
     using U = typename ST::U;
     constexpr int NB = NbrBatch<L, false>::kN;
@@ -1184,6 +1243,7 @@ __global__ void __launch_bounds__(256)
         float4 Xo = make_float4(0.f, 0.f, 0.f, 0.f);
         int4 seg = make_int4(0, 0, 0, 0);
         U uo{};
+        int info = 0;
         if (valid) {
             seg = P.vrec[v];
             seg.x -= tile.n0;
@@ -1192,6 +1252,7 @@ __global__ void __launch_bounds__(256)
             mat = P.mats[P.slot_mesh[v]];
             if (sub == 0) prefetch_tail<L>(P, v);
             uo = P.u[v];
+            if constexpr (CONTACT) info = P.col_info[v];
         }
         const U uon = ST::nb(uo);
         const bool ok = __syncthreads_and(mbar_wait(bar0 + 8u * uint32_t(b), parity, c.spin_limit)) != 0;
@@ -1212,10 +1273,8 @@ __global__ void __launch_bounds__(256)
         preload<L, kRecShared>(rec, s_nbr(b), s_inc(b), seg, sub);
         accumulate_segment<L, kRecShared, false, ST>(rec, sub, st, FetchGlobal<ST, kStatePlain>{P.u, P.rest}, uon, Xo, mat.mu, mat.lmbd, acc);
         reduce_group<L, float>(acc);
-        if (valid && sub == 0) {
-            finish_acc(acc, mat.mu, mat.lmbd);
-            vertex_tail<ST, float, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr);
-        }
+        const float3 Fo = valid && sub == 0 ? frame_offset(P, v) : make_float3(0.f, 0.f, 0.f);
+        finish_vertex<L, false, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, beg, end, flags, nullptr);
         __syncthreads();  // every read of buffer b done before the next iteration refills it
     }
 }
@@ -1266,7 +1325,7 @@ __device__ __forceinline__ void solve_in_sweep(const Ptrs<ST, R>& P, const Const
     reduce_group<L, R>(acc);
     if (valid && sub == 0) {
         finish_acc(acc, mat.mu, mat.lmbd);
-        vertex_tail<ST, R, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr);
+        vertex_tail<ST, R, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr, nullptr);
     }
 }
 
