@@ -40,12 +40,12 @@ sys.path.insert(0, ROOT)
 
 METRIC = "VBD vertex-solves/s & steps/s, FP32-mixed vs plain FP64 at <=1e-5 rel pos err"
 # dram__bytes_read.sum + dram__bytes_write.sum per solved incidence of k_solve, measured by
-# ncu: FP32 on 8 color launches of the 100^3 twist (4.8 M incidences each), double-float on
-# colors 0-2 of the 60^3 twist (3 x ~1.01 M incidences); see profiles/
-TRAFFIC_BYTES_PER_INCIDENCE = {"fp32": 54.4, "mixed": 59.9}
+# ncu on 8 color launches each of the 60^3 twist (1.009 M incidences a launch; 21.89 MB FP32,
+# 26.18 MB double-float); see profiles/
+TRAFFIC_BYTES_PER_INCIDENCE = {"fp32": 21.7, "mixed": 25.9}
 # DRAM bytes (read + write) of one k_sweep_scenes launch per solved incidence and iteration:
-# 44.65 GB over 20 iterations of the 512-cube batch's 38.95 M incidences (FP32, mesh frames)
-SCENES_TRAFFIC_BYTES_PER_INCIDENCE_ITERATION = 57.3
+# 1.056 GB over 4 iterations of a 200-cube batch's 15.23 M incidences (FP32, mesh frames)
+SCENES_TRAFFIC_BYTES_PER_INCIDENCE_ITERATION = 17.3
 
 
 def load_peaks() -> tuple[float, str]:
@@ -824,11 +824,11 @@ def main():
         traffic, source = None, None
         if per_inc and sweep_mode == 0:
             traffic = per_inc * ninc / st["num_groups"]
-            source = ("ncu DRAM bytes per incidence (FP32: 100^3 twist launches; double-float: 60^3 twist), times "
+            source = ("ncu DRAM bytes per incidence (60^3 twist launches), times "
                       "this launch's incidences")
         elif sweep_mode == 1 and head["precision"] == "fp32":
             traffic = SCENES_TRAFFIC_BYTES_PER_INCIDENCE_ITERATION * ninc * args.iterations
-            source = ("ncu DRAM bytes of the scene-major sweep per incidence and iteration (512-cube batch, FP32), "
+            source = ("ncu DRAM bytes of the scene-major sweep per incidence and iteration (200-cube batch, FP32), "
                       "times this launch's incidences and iterations")
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "traffic": traffic, "traffic_source": source,

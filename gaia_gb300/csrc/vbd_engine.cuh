@@ -84,7 +84,7 @@ inline int div_up(int64_t a, int64_t b) { return int((a + b - 1) / b); }
 }  // namespace
 
 enum { kSweepMerged = 0, kSweepScenes = 1, kSweepCluster = 2, kSweepGrid = 3 };
-constexpr int kVariantDeep = 4;  // solve variant: k_solve_deep
+constexpr int kVariantDeep = 4;  // solve variant: k_solve with asynchronous one-ring copies
 constexpr int kVariantGrid = 5;  // solve variant: k_sweep_grid
 constexpr int kVariantPrefetch = 6;  // solve variant: k_solve with the next wave's records prefetched into L2
 constexpr int kVariantPipe = 7;      // solve variant: k_solve_pipe, double-buffered TMA tiles on a persistent grid
@@ -2204,7 +2204,7 @@ private:
     bool use_pdl_ = true;
     int small_color_ = 16384;
     int variant_ = 0;          // 0 = register-pipelined k_solve, 1 = TMA-staged k_solve_tma, 2 = k_sweep_scenes,
-                               // 3 = k_sweep_cluster, 4 = k_solve_deep, 5 = k_sweep_grid, 6 = k_solve with L2
+                               // 3 = k_sweep_cluster, 4 = k_solve with DEEP, 5 = k_sweep_grid, 6 = k_solve with L2
                                // prefetch of the next wave's records, 7 = k_solve_pipe
     int mode_ = 0;             // kSweepMerged, kSweepScenes, kSweepCluster or kSweepGrid
     // scene-major mode: per mesh its color slot ranges, in sweep order

@@ -61,9 +61,9 @@ typedef struct {
     int64_t device_bytes;         /* device memory owned by the handle */
     double autotune_ms_per_iteration; /* best measured sweep time per iteration (0 if not tuned) */
     int32_t solve_variant;        /* 0 = register-pipelined solve kernel, 1 = TMA-staged records,
-                                     2 = scene-major persistent sweep, 3 = cluster sweep, 4 = register
-                                     pipeline two records deep, 5 = grid sweep, 6 = register pipeline
-                                     with the records of the next resident wave prefetched into L2,
+                                     2 = scene-major persistent sweep, 3 = cluster sweep, 4 = one-ring
+                                     copied to shared memory asynchronously, 5 = grid sweep, 6 = as 0
+                                     with the data of the next resident wave prefetched into L2,
                                      7 = double-buffered TMA tiles on a persistent grid (of the
                                      largest color) */
     int32_t mesh_frames;          /* 1: states are kept relative to a per-mesh frame offset that
@@ -247,7 +247,7 @@ typedef struct {
 int gaia_vbd_get_output_params(const gaia_vbd* h, gaia_vbd_output_params* out);
 int64_t gaia_vbd_frame(const gaia_vbd* h);
 /* Launch configuration the autotuner chose for merged color g (parallel group g):
- * lanes per vertex, block size, kernel variant (0 registers, 1 TMA-staged), and the
+ * lanes per vertex, block size, kernel variant (stats: solve_variant), and the
  * measured time of one launch in ms (0 when not tuned). Any pointer may be NULL.
  * The reference launches every color with one 32-thread block per vertex
  * (VBDPhysicsCompute.cu:114-123). */
