@@ -13,9 +13,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <memory>
 #include <stdexcept>
@@ -507,6 +509,52 @@ public:
         }
     }
 
+    // The edge weights of one segment in the compute type. FP32: each rounded to the one of its
+    // two neighbouring floats that keeps sum (k - K) r small (r the rest edges), largest first:
+    // the weights of a rigid or linear motion e = A r then sum as the FP64 ones do, although the
+    // terms of a flat one-ring are far larger than their sum.
+    static void round_weights(int n, const double* K, const double (*r)[3], R* k) {
+        for (int i = 0; i < n; ++i) k[i] = R(K[i]);
+        if (sizeof(R) != 4 || n < 2) return;
+        double d0[dev::kSegNbrs][3], d1[dev::kSegNbrs][3], key[dev::kSegNbrs], s[3] = {0, 0, 0};
+        R alt[dev::kSegNbrs];
+        int order[dev::kSegNbrs];
+        for (int i = 0; i < n; ++i) {
+            const R inf = std::numeric_limits<R>::infinity();
+            alt[i] = std::nextafter(k[i], double(k[i]) < K[i] ? inf : -inf);
+            key[i] = 0.0;
+            for (int c = 0; c < 3; ++c) {
+                d0[i][c] = (double(k[i]) - K[i]) * r[i][c];
+                d1[i][c] = (double(alt[i]) - K[i]) * r[i][c];
+                key[i] += (d1[i][c] - d0[i][c]) * (d1[i][c] - d0[i][c]);
+            }
+            order[i] = i;
+        }
+        std::sort(order, order + n, [&](int a, int b) { return key[a] != key[b] ? key[a] > key[b] : a < b; });
+        auto norm = [](const double* a, const double* b, const double* c) {
+            double q = 0.0;
+            for (int j = 0; j < 3; ++j) q += (a[j] - b[j] + c[j]) * (a[j] - b[j] + c[j]);
+            return q;
+        };
+        const double zero[3] = {0, 0, 0};
+        for (int q = 0; q < n; ++q) {
+            const int i = order[q];
+            if (norm(s, zero, d1[i]) < norm(s, zero, d0[i])) {
+                std::swap(k[i], alt[i]);
+                std::swap(d0[i], d1[i]);
+            }
+            for (int c = 0; c < 3; ++c) s[c] += d0[i][c];
+        }
+        for (int pass = 0; pass < 2; ++pass)
+            for (int q = 0; q < n; ++q) {
+                const int i = order[q];
+                if (!(norm(s, d0[i], d1[i]) < 0.99 * norm(s, zero, zero))) continue;
+                for (int c = 0; c < 3; ++c) s[c] += d1[i][c] - d0[i][c];
+                std::swap(k[i], alt[i]);
+                std::swap(d0[i], d1[i]);
+            }
+    }
+
     // The segments of slot s one after another in nbr and inc (done() is called after each).
     template <typename Fn>
     void segments_of(int32_t s, std::vector<dev::NbrRec<R>>& nbr, std::vector<dev::IncRec<R>>& inc, Fn&& done) const {
@@ -514,7 +562,9 @@ public:
         const TetMesh& M = sc_.meshes[m];
         const int v = orig_of_[s] - int32_t(mesh_off_[m]);
         int32_t slots[dev::kSegNbrs];
-        double K[dev::kSegNbrs];
+        double K[dev::kSegNbrs], rest[dev::kSegNbrs][3];
+        R k[dev::kSegNbrs];
+        const float* Xo = &M.X[3 * size_t(v)];
         int n = 0;
         inc.clear();
         auto close = [&] {
@@ -523,14 +573,17 @@ public:
             uint32_t rank[dev::kSegNbrs];
             for (int i = 0; i < n; ++i) order[i] = i;
             std::sort(order, order + n, [&](int a, int b) { return slots[a] < slots[b]; });
+            round_weights(n, K, rest, k);
             nbr.resize(size_t(n));
             for (int i = 0; i < n; ++i) {
                 rank[order[i]] = uint32_t(i);
                 nbr[size_t(i)] = dev::NbrRec<R>{};
                 nbr[size_t(i)].slot = slots[order[i]];
-                nbr[size_t(i)].k = R(K[order[i]]);
+                nbr[size_t(i)].k = k[order[i]];
             }
-            for (auto& q : inc) q.idx = rank[q.idx & 255u] | rank[(q.idx >> 8) & 255u] << 8 | rank[(q.idx >> 16) & 255u] << 16;
+            for (auto& q : inc)
+                q.idx = rank[q.idx & 255u] | rank[(q.idx >> 8) & 255u] << 8 | rank[(q.idx >> 16) & 255u] << 16 |
+                        rank[q.idx >> 24] << 24;
             done();
             n = 0;
             inc.clear();
@@ -547,6 +600,27 @@ public:
             for (int j = 0; j < 4; ++j)
                 if (j != o) others[w++] = j;
             if (o & 1) std::swap(others[0], others[1]);  // keeps det of the rows = det(DmInv)
+            // The face normals are taken at the vertex opposite the face's longest edge, the volume
+            // change at the vertex nearest to o: the parts that cancel in a rotated tet are then
+            // smallest (a rotation of the three vertices keeps the determinant's sign).
+            std::array<double, 3> r[3];
+            for (int i = 0; i < 3; ++i)
+                for (int c = 0; c < 3; ++c)
+                    r[i][c] = double(M.X[3 * size_t(M.tets[4 * size_t(t) + others[i]]) + c]) - double(Xo[c]);
+            auto edge2 = [&](int i, int j) {
+                double q = 0.0;
+                for (int c = 0; c < 3; ++c) q += (r[i][c] - r[j][c]) * (r[i][c] - r[j][c]);
+                return q;
+            };
+            int first = 0, near = 0;
+            for (int i = 1; i < 3; ++i) {
+                if (edge2((i + 1) % 3, (i + 2) % 3) > edge2((first + 1) % 3, (first + 2) % 3)) first = i;
+                auto len2 = [&](int j) { return r[j][0] * r[j][0] + r[j][1] * r[j][1] + r[j][2] * r[j][2]; };
+                if (len2(i) < len2(near)) near = i;
+            }
+            std::rotate(others, others + first, others + 3);
+            std::rotate(r, r + first, r + 3);
+            near = (near - first + 3) % 3;
             int32_t sl[3];
             int at[3], fresh = 0;
             auto find = [&](int32_t x) {
@@ -564,6 +638,7 @@ public:
                 if (at[i] < 0) {
                     at[i] = n;
                     slots[n] = sl[i];
+                    for (int c = 0; c < 3; ++c) rest[n][c] = r[i][c];
                     K[n++] = 0.0;
                 }
                 const double* a = row[o];
@@ -571,7 +646,7 @@ public:
                 K[at[i]] += M.vol[t] * (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]);
             }
             dev::IncRec<R> rec{};
-            rec.idx = uint32_t(at[0]) | uint32_t(at[1]) << 8 | uint32_t(at[2]) << 16;
+            rec.idx = uint32_t(at[0]) | uint32_t(at[1]) << 8 | uint32_t(at[2]) << 16 | uint32_t(at[near]) << 24;
             rec.w = R(1.0 / (6.0 * M.vol[t]));
             inc.push_back(rec);
         }

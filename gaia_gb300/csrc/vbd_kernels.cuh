@@ -32,7 +32,7 @@
 //         FP64 DmInv), the material-free edge weight of the linear part of the force;
 //       IncRec (8 B FP32, 16 B FP64): per incident tet the positions of its three other
 //         vertices in the vertex's neighbour list (8 bits each, in the order whose rows have
-//         determinant det DmInv) and w = 1 / (6 A) = det DmInv.
+//         determinant det DmInv, and the nearest one's again) and w = 1 / (6 A) = det DmInv.
 //     The records of eight consecutive vertices are interleaved (record k of a vertex lies
 //     kSlice places after its record k - 1), so that lanes on neighbouring vertices read
 //     neighbouring records. vrec[s] = (first NbrRec, first IncRec, their numbers). Lists of
@@ -52,6 +52,21 @@
 // dF/dx, VBDPhysicsCompute.cu:2035-2232, VBD_NeoHookean.cpp:379-581: det F is affine in x_o,
 // so the (J - a) d2J/dF2 term contracts to zero). Every difference is formed from small
 // quantities: C = a x de + db x b' with a, b' edges and db, de differences of displacements.
+//
+// Where a tet is rotated, G is not small, and the parts of S, and the sums of K_n e_n and C,
+// are large and cancel. In FP32 they keep what the stored rows of dF/dx gave:
+//   * position 0 is the vertex opposite the longest edge of the face, so that the cross products
+//     are of the two shorter edges, and S is taken at the vertex nearest to o (the fourth
+//     position of IncRec): |N| |e| is then smallest against the tet's volume;
+//   * S is two dot products with their rounding errors, sum K_n e_n a float pair over the
+//     neighbours and over the lanes;
+//   * the K_n are rounded so that the first moment of their rounding errors, sum dK_n r_n,
+//     (nearly) vanishes, and with it their part in any linear motion e = A r.
+// Error of a vertex's step from the elastic force against FP64, on a body of random tets,
+// relative to the rows' (1.0): rotated by 0.3 rad 0.92, flattened to a tenth and rotated by
+// 2 rad 0.92, as with stored rows 0.87 and 0.89 (tests/test_gpu_rotated_ring.py); without any of
+// these 1.60 and 2.02. The 100^3 twist takes 9.4 ms a step with them, 8.1 without (the choice of the
+// positions and the rounding of K_n, which cost nothing, alone: 1.07 and 1.49).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -264,10 +279,12 @@ __device__ __forceinline__ T ld_rec(const T* p) {
 }
 
 // Accumulator of one vertex: force (3), lambda-part of the Hessian (6, upper
-// triangle), and S = sum A mu |m_o|^2 (the isotropic part).
+// triangle), and S = sum A mu |m_o|^2 (the isotropic part). FP32: k + l, sum K e over the
+// neighbours as a float pair (before finish_acc).
 template <typename R>
 struct Acc {
     R f0, f1, f2, h00, h01, h02, h11, h12, h22, S;
+    R k0, k1, k2, l0, l1, l2;
 };
 
 // Where a vertex's one-ring comes from. Global memory: either copied into the staging area
@@ -369,24 +386,54 @@ __device__ __forceinline__ Stage<32 / L, ST, R> warp_stage(unsigned char* smem, 
     return S(smem + size_t(threadIdx.x >> 5) * size_t(cap * (32 / L)) * (16 * S::kParts), cap, Lanes<L>::vertex());
 }
 
+// k + l += x y: l takes the rounding errors of product and sum (two-sum of k and fl(x y), the
+// product's own error coming in with the last term).
+__device__ __forceinline__ void pair_fma(float x, float y, float& k, float& l) {
+    const float s = __fadd_rn(k, __fmul_rn(x, y));
+    const float b = __fsub_rn(s, k);
+    l = __fadd_rn(l, __fadd_rn(__fsub_rn(k, __fsub_rn(s, b)), __fmaf_rn(x, y, -b)));
+    k = s;
+}
+
+// x.y as a float pair s + er.
+__device__ __forceinline__ float dot_pair(const float* x, const float* y, float& er) {
+    float s = __fmul_rn(x[0], y[0]);
+    er = __fmaf_rn(x[0], y[0], -s);
+#pragma unroll
+    for (int c = 1; c < 3; ++c) pair_fma(x[c], y[c], s, er);
+    return s;
+}
+
+// N.e + C.p, which cancel where the tet is rotated.
+template <typename R>
+__device__ __forceinline__ R volume_change(const R* N, const R* e, const R* C, const R* p) {
+    if constexpr (sizeof(R) == 4) {
+        float en, ec;
+        const float n = dot_pair(N, e, en), c = dot_pair(C, p, ec);
+        return __fadd_rn(__fadd_rn(n, c), __fadd_rn(en, ec));
+    } else {
+        return (N[0] * e[0] + N[1] * e[1] + N[2] * e[2]) + (C[0] * p[0] + C[1] * p[1] + C[2] * p[2]);
+    }
+}
+
 // One tet from its three other vertices' differences: C into cs, w S D into t, w D D^T into the
-// accumulator's Hessian (unscaled, see finish_acc).
+// accumulator's Hessian (unscaled, see finish_acc). es, rs: the vertex at the shortest rest edge.
 template <typename R>
 __device__ __forceinline__ void incidence(const R* e0, const R* e1, const R* e2, const R* r0, const R* r1, const R* r2,
-                                          R w, R* cs, R* t, Acc<R>& acc) {
+                                          const R* es, const R* rs, R w, R* cs, R* t, Acc<R>& acc) {
     const R a[3] = {r1[0] - r0[0], r1[1] - r0[1], r1[2] - r0[2]};
     const R b[3] = {r2[0] - r0[0], r2[1] - r0[1], r2[2] - r0[2]};
     const R al[3] = {e1[0] - e0[0], e1[1] - e0[1], e1[2] - e0[2]};
     const R be[3] = {e2[0] - e0[0], e2[1] - e0[1], e2[2] - e0[2]};
     const R bd[3] = {b[0] + be[0], b[1] + be[1], b[2] + be[2]};
     // C = a x be + al x bd, N = a x b
-    const R C0 = (a[1] * be[2] - a[2] * be[1]) + (al[1] * bd[2] - al[2] * bd[1]);
-    const R C1 = (a[2] * be[0] - a[0] * be[2]) + (al[2] * bd[0] - al[0] * bd[2]);
-    const R C2 = (a[0] * be[1] - a[1] * be[0]) + (al[0] * bd[1] - al[1] * bd[0]);
+    const R C0 = a[1] * be[2] - a[2] * be[1] + al[1] * bd[2] - al[2] * bd[1];
+    const R C1 = a[2] * be[0] - a[0] * be[2] + al[2] * bd[0] - al[0] * bd[2];
+    const R C2 = a[0] * be[1] - a[1] * be[0] + al[0] * bd[1] - al[1] * bd[0];
     const R N0 = a[1] * b[2] - a[2] * b[1], N1 = a[2] * b[0] - a[0] * b[2], N2 = a[0] * b[1] - a[1] * b[0];
     const R D0 = N0 + C0, D1 = N1 + C1, D2 = N2 + C2;
-    const R p0 = r0[0] + e0[0], p1 = r0[1] + e0[1], p2 = r0[2] + e0[2];
-    const R S = (N0 * e0[0] + N1 * e0[1] + N2 * e0[2]) + (C0 * p0 + C1 * p1 + C2 * p2);
+    const R N[3] = {N0, N1, N2}, C[3] = {C0, C1, C2}, p[3] = {rs[0] + es[0], rs[1] + es[1], rs[2] + es[2]};
+    const R S = volume_change(N, es, C, p);
     const R w0 = w * D0, w1 = w * D1, w2 = w * D2;
     cs[0] += C0; cs[1] += C1; cs[2] += C2;
     t[0] += S * w0; t[1] += S * w1; t[2] += S * w2;
@@ -451,9 +498,15 @@ __device__ __forceinline__ void accumulate_segment(SegRecs<R, NB>& s, int sub, c
         ST::diff(q, uo, e);
         const R r[3] = {R(X.x) - R(Xo.x), R(X.y) - R(Xo.y), R(X.z) - R(Xo.z)};
         st.put(k, e, r);
-        kf[0] += K * e[0];
-        kf[1] += K * e[1];
-        kf[2] += K * e[2];
+        if constexpr (sizeof(R) == 4) {
+            pair_fma(K, e[0], acc.k0, acc.l0);
+            pair_fma(K, e[1], acc.k1, acc.l1);
+            pair_fma(K, e[2], acc.k2, acc.l2);
+        } else {
+            kf[0] += K * e[0];
+            kf[1] += K * e[1];
+            kf[2] += K * e[2];
+        }
         acc.S += K;
     };
     if constexpr (ASYNC) {
@@ -498,7 +551,13 @@ __device__ __forceinline__ void accumulate_segment(SegRecs<R, NB>& s, int sub, c
         st.get(int(cur.idx & 255u), e0, r0);
         st.get(int((cur.idx >> 8) & 255u), e1, r1);
         st.get(int((cur.idx >> 16) & 255u), e2, r2);
-        incidence(e0, e1, e2, r0, r1, r2, cur.w, cs, t, acc);
+        if constexpr (sizeof(R) == 4) {
+            R es[3], rs[3];
+            st.get(int(cur.idx >> 24), es, rs);
+            incidence(e0, e1, e2, r0, r1, r2, es, rs, cur.w, cs, t, acc);
+        } else {
+            incidence(e0, e1, e2, r0, r1, r2, e0, r0, cur.w, cs, t, acc);
+        }
     }
     const R m6 = mu * R(1.0 / 6.0), l6 = lmbd * R(1.0 / 6.0);
     acc.f0 += l6 * t[0] - m6 * cs[0] - mu * kf[0];
@@ -527,6 +586,11 @@ __device__ __forceinline__ void finish_acc(Acc<R>& a, R mu, R lmbd) {
     const R l6 = lmbd * R(1.0 / 6.0);
     a.h00 *= l6; a.h01 *= l6; a.h02 *= l6; a.h11 *= l6; a.h12 *= l6; a.h22 *= l6;
     a.S *= -mu;
+    if constexpr (sizeof(R) == 4) {
+        a.f0 -= mu * (a.k0 + a.l0);
+        a.f1 -= mu * (a.k1 + a.l1);
+        a.f2 -= mu * (a.k2 + a.l2);
+    }
 }
 
 // One halving step of the reduce-scatter below: of n values, this lane keeps the lower or the
@@ -583,6 +647,18 @@ __device__ __forceinline__ void reduce_group(Acc<R>& a) {
             a.h12 += __shfl_xor_sync(0xffffffffu, a.h12, off);
             a.h22 += __shfl_xor_sync(0xffffffffu, a.h22, off);
             a.S += __shfl_xor_sync(0xffffffffu, a.S, off);
+            if constexpr (sizeof(R) == 4) {
+                auto join = [&](float& k, float& l) {
+                    const float ko = __shfl_xor_sync(0xffffffffu, k, off), lo = __shfl_xor_sync(0xffffffffu, l, off);
+                    float s, e;
+                    two_sum(k, ko, s, e);
+                    k = s;
+                    l = __fadd_rn(__fadd_rn(l, lo), e);
+                };
+                join(a.k0, a.l0);
+                join(a.k1, a.l1);
+                join(a.k2, a.l2);
+            }
         }
     }
 }
