@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/gaia_vbd.h"
+#include "launch_shape.hpp"
 #include "scene.hpp"
 #include "state_io.hpp"
 #include "tet_cd.hpp"
@@ -1444,7 +1445,6 @@ public:
     void enqueue_scenes_sweep(int L, int B) {
         if (nscenes_ == 0 || sc_.p.iterations == 0) return;
         GAIA_CUDA(cudaMemsetAsync(d_scene_work_.p, 0, sizeof(int32_t), st_));
-        while (B > 64 && stage_bytes(max_nbr_all_, 32, B) > kTmaSmemMax) B /= 2;
         if (multi_seg_) {
             launch_scenes_l<32, true>(B);
             return;
@@ -1662,10 +1662,10 @@ public:
         GAIA_CUDA(cudaMemsetAsync(d_scene_work_.p, 0, sizeof(int32_t), st_));
         // more lanes per vertex, then fewer threads, where the staging areas do not fit beside the scene
         auto fits = [&](int l) { return f->bytes + stage_bytes(max_nbr_all_, l, B) <= cluster_budget_; };
+        if (f->lean) L = 32;
         while (L < 32 && !fits(L)) L *= 2;
-        while (B > 64 && !fits(L)) B /= 2;
+        while (B > kMinBlock && !fits(L)) B = smaller_block(B);
         if (f->lean) {
-            while (B > 64 && f->bytes + stage_bytes(max_nbr_all_, 32, B) > cluster_budget_) B /= 2;
             if (multi_seg_) launch_cluster_l<32, true, true>(*f, B);
             else launch_cluster_l<32, false, true>(*f, B);
             return;
