@@ -22,11 +22,11 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
-#include <thread>
 #include <tuple>
 #include <vector>
 
 #include "../../include/gaia_vbd.h"
+#include "host_threads.hpp"
 #include "launch_shape.hpp"
 #include "scene.hpp"
 #include "state_io.hpp"
@@ -453,10 +453,7 @@ public:
                 }
             }
         };
-        std::vector<std::thread> th;
-        for (int k = 1; k < nt; ++k) th.emplace_back(work, k);
-        work(0);
-        for (auto& t : th) t.join();
+        run_parts(nt, work);
         size_t nn = 0, ni = 0;
         for (auto& q : part) {
             nn += q.nbr.size();
