@@ -73,8 +73,8 @@ struct ClusterScenes {
     int32_t pos_cap;           // states each block's shared copy holds
     int32_t nbr_cap, inc_cap;  // neighbour and incidence records each block holds
     int32_t stage_cap;         // staging entries per vertex
-    const int4* ranges;        // per color and rank: its records in the global arrays (colors of all
-                               // scenes, C per color): first and last + 1 NbrRec and IncRec
+    const int4* ranges;        // per color and rank: its record rows in the global arrays (colors of all
+                               // scenes, C per color): first and last + 1 of NbrRec and IncRec
 };
 
 // A state broadcast from lane src of the warp (every field of the trait's state type).
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
             beg = min(rg.y, rg.x + rank * per);
             end = min(rg.y, beg + per);
         };
-        // per color, where the chunk's records start in the shared arrays, less their global number
+        // per color, the row where the chunk's records start in the shared arrays, less their global one
         if (!LEAN && threadIdx.x == 0) {
             int2 base = make_int2(0, 0);
             for (int ci = c0; ci < c1; ++ci) {
@@ -157,12 +157,16 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
         for (int ci = c0; !LEAN && ci < c1; ++ci) {
             const int4 r = S.ranges[ci * C + rank];
             const int2 sb = s_rec_base[ci - c0];
-            for (int i = r.x + int(threadIdx.x); i < r.y; i += blockDim.x) {
-                NbrRec<R> n = P.nbr[i];
+            const NbrRec<R>* gn = P.nbr + record_index(r.x, 0);
+            const IncRec<R>* gi = P.inc + record_index(r.z, 0);
+            NbrRec<R>* dn = snbr + (sb.x + r.x) * kSlice;
+            IncRec<R>* di = sinc + (sb.y + r.z) * kSlice;
+            for (int i = int(threadIdx.x); i < (r.y - r.x) * kSlice; i += blockDim.x) {
+                NbrRec<R> n = gn[i];
                 n.slot = loc(n.slot);
-                snbr[sb.x + i] = n;
+                dn[i] = n;
             }
-            for (int i = r.z + int(threadIdx.x); i < r.w; i += blockDim.x) sinc[sb.y + i] = P.inc[i];
+            for (int i = int(threadIdx.x); i < (r.w - r.z) * kSlice; i += blockDim.x) di[i] = gi[i];
         }
         cluster.sync();  // every copy staged before any block writes into another's
         for (int it = 0; it < S.iterations; ++it) {
@@ -171,8 +175,8 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
                 int beg, end;
                 chunk(ci, beg, end);
                 const int2 sb = LEAN ? make_int2(0, 0) : s_rec_base[ci - c0];
-                const NbrRec<R>* nbr = LEAN ? P.nbr : snbr + sb.x;
-                const IncRec<R>* inc = LEAN ? P.inc : sinc + sb.y;
+                const NbrRec<R>* nbr = LEAN ? P.nbr : snbr + ptrdiff_t(sb.x) * kSlice;
+                const IncRec<R>* inc = LEAN ? P.inc : sinc + ptrdiff_t(sb.y) * kSlice;
                 for (int base = beg; base < end; base += groups) {
                     const int v = base + g;
                     const bool valid = v < end;

@@ -370,8 +370,7 @@ public:
         for (int32_t s = 0; s < nactive_; ++s) {
             const int m = slot_mesh_[s], v = orig_of_[s] - int32_t(mesh_off_[m]);
             total += meshes[m].nbr_ofs[v + 1] - meshes[m].nbr_ofs[v];
-            if (total > int64_t(INT32_MAX) / 2) throw std::runtime_error("too many incidences");
-            inc_ofs_[s + 1] = int32_t(total);
+            inc_ofs_[s + 1] = checked_count(total);
         }
         ninc_ = int32_t(total);
         std::vector<int2> slices;  // slot ranges
@@ -401,8 +400,9 @@ public:
             std::vector<dev::IncRec<R>> inc;
             // the lists of one segment into place: every kSlice-th record from the segment's first
             auto place = [&](int4 seg) {
-                for (int i = 0; i < seg.z; ++i) out.nbr[size_t(seg.x + dev::kSlice * i)] = nbr[size_t(i)];
-                for (int i = 0; i < seg.w; ++i) out.inc[size_t(seg.y + dev::kSlice * i)] = inc[size_t(i)];
+                const int at = dev::place_of(seg.z);
+                for (size_t i = 0; i < nbr.size(); ++i) out.nbr[dev::record_index(seg.x + int(i), at)] = nbr[i];
+                for (size_t i = 0; i < inc.size(); ++i) out.inc[dev::record_index(seg.y + int(i), at)] = inc[i];
             };
             std::vector<std::vector<dev::NbrRec<R>>> ln(dev::kSlice);
             std::vector<std::vector<dev::IncRec<R>>> li(dev::kSlice);
@@ -420,35 +420,37 @@ public:
                             mn = std::max(mn, nbr.size());
                             mi = std::max(mi, inc.size());
                         } else {
-                            extra.push_back({s, make_int4(0, 0, int(nbr.size()), int(inc.size()))});
+                            extra.push_back({s, make_int4(0, 0, dev::pack_nbrs(int(nbr.size()), 0), int(inc.size()))});
                             extra_lists.emplace_back(nbr, inc);
                         }
                         first = false;
                     });
                 }
-                const size_t nb = out.nbr.size(), ib = out.inc.size();
+                // rows of this part so far
+                const int nb = checked_count(int64_t(out.nbr.size() / dev::kSlice));
+                const int ib = checked_count(int64_t(out.inc.size() / dev::kSlice));
                 size_t en = 0, ei = 0;
                 for (auto& e : extra_lists) {
                     en += e.first.size();
                     ei += e.second.size();
                 }
-                out.nbr.resize(nb + dev::kSlice * (mn + en));
-                out.inc.resize(ib + dev::kSlice * (mi + ei));
+                out.nbr.resize(out.nbr.size() + dev::kSlice * (mn + en));
+                out.inc.resize(out.inc.size() + dev::kSlice * (mi + ei));
                 for (int32_t s = rg.x; s < rg.y; ++s) {
                     nbr = ln[size_t(s - rg.x)];
                     inc = li[size_t(s - rg.x)];
-                    vrec_[size_t(s)] = make_int4(int(nb) + (s - rg.x), int(ib) + (s - rg.x), int(nbr.size()), int(inc.size()));
+                    vrec_[size_t(s)] = make_int4(nb, ib, dev::pack_nbrs(int(nbr.size()), s - rg.x), int(inc.size()));
                     place(vrec_[size_t(s)]);
                 }
-                int n1 = int(nb + dev::kSlice * mn), i1 = int(ib + dev::kSlice * mi);
+                int n1 = nb + int(mn), i1 = ib + int(mi);
                 for (size_t e = 0; e < extra.size(); ++e) {
                     nbr = extra_lists[e].first;
                     inc = extra_lists[e].second;
                     extra[e].r.x = n1;
                     extra[e].r.y = i1;
                     place(extra[e].r);
-                    n1 += dev::kSlice * int(nbr.size());
-                    i1 += dev::kSlice * int(inc.size());
+                    n1 += int(nbr.size());
+                    i1 += int(inc.size());
                     out.more.push_back(extra[e]);
                 }
             }
@@ -459,7 +461,8 @@ public:
             nn += q.nbr.size();
             ni += q.inc.size();
         }
-        if (std::max(nn, ni) > size_t(INT32_MAX) / 2) throw std::runtime_error("too many incidences");
+        nbr_end_ = checked_count(int64_t(nn / dev::kSlice));
+        inc_end_ = checked_count(int64_t(ni / dev::kSlice));
         // the parts end to end, padded for the copies of whole slices that run past the last list
         max_nbr_all_ = max_inc_all_ = 2;
         h_nbr_.clear();
@@ -470,7 +473,7 @@ public:
         std::vector<Seg> more;
         for (int k = 0; k < nt; ++k) {
             Part& q = part[size_t(k)];
-            const int n0 = int(h_nbr_.size()), i0 = int(h_inc_.size());
+            const int n0 = int(h_nbr_.size() / dev::kSlice), i0 = int(h_inc_.size() / dev::kSlice);
             if (range(k) < range(k + 1))
                 for (int32_t s = slices[range(k)].x; s < slices[range(k + 1) - 1].y; ++s) {
                     vrec_[size_t(s)].x += n0;
@@ -484,13 +487,11 @@ public:
             h_nbr_.insert(h_nbr_.end(), q.nbr.begin(), q.nbr.end());
             h_inc_.insert(h_inc_.end(), q.inc.begin(), q.inc.end());
         }
-        nbr_end_ = int(h_nbr_.size());
-        inc_end_ = int(h_inc_.size());
         for (const int4& r : vrec_) {
-            max_nbr_all_ = std::max(max_nbr_all_, (r.z + 1) & ~1);
+            max_nbr_all_ = std::max(max_nbr_all_, (dev::nbrs_of(r.z) + 1) & ~1);
             max_inc_all_ = std::max(max_inc_all_, r.w);
         }
-        for (const Seg& e : more) max_nbr_all_ = std::max(max_nbr_all_, (e.r.z + 1) & ~1);
+        for (const Seg& e : more) max_nbr_all_ = std::max(max_nbr_all_, (dev::nbrs_of(e.r.z) + 1) & ~1);
         h_nbr_.resize(h_nbr_.size() + size_t(dev::kSlice) * max_nbr_all_, dev::NbrRec<R>{});
         h_inc_.resize(h_inc_.size() + size_t(dev::kSlice) * max_inc_all_, dev::IncRec<R>{});
         multi_seg_ = !more.empty();
@@ -660,7 +661,7 @@ public:
         if (it != lists_cache_.end()) return it->second;
         int2 m = make_int2(2, 1);
         for (int v = beg; v < end; ++v) {
-            m.x = std::max(m.x, (vrec_[size_t(v)].z + 1) & ~1);
+            m.x = std::max(m.x, (dev::nbrs_of(vrec_[size_t(v)].z) + 1) & ~1);
             m.y = std::max(m.y, vrec_[size_t(v)].w);
         }
         return lists_cache_[key] = m;
@@ -936,9 +937,8 @@ public:
         int2 m = make_int2(0, 0);
         for (int v0 = beg; v0 < end; v0 += vpb) {
             const int4 r0 = vrec_[size_t(v0)], r1 = vrec_[size_t(std::min(end, v0 + vpb) - 1)];
-            const int mask = ~(dev::kSlice - 1);
-            m.x = std::max(m.x, (r1.x & mask) + dev::kSlice * lists.x - (r0.x & mask));
-            m.y = std::max(m.y, (r1.y & mask) + dev::kSlice * lists.y - (r0.y & mask));
+            m.x = std::max(m.x, dev::kSlice * (r1.x + lists.x - r0.x));
+            m.y = std::max(m.y, dev::kSlice * (r1.y + lists.y - r0.y));
         }
         maxrec_cache_[key] = m;
         return m;
@@ -1526,8 +1526,8 @@ public:
                     int64_t nbr = 0, inc = 0;
                     for (int32_t ci = scene_ofs_[m]; ci < scene_ofs_[m + 1]; ++ci) {
                         const int4 q = rg[size_t(ci) * C + r];
-                        nbr += q.y - q.x;
-                        inc += q.w - q.z;
+                        nbr += int64_t(dev::kSlice) * (q.y - q.x);
+                        inc += int64_t(dev::kSlice) * (q.w - q.z);
                     }
                     nbr_cap = std::max(nbr_cap, nbr);
                     inc_cap = std::max(inc_cap, inc);
@@ -1587,14 +1587,13 @@ public:
         return most;
     }
 
-    // Records of every color's chunk of every rank in a cluster of C blocks (C per color): the
-    // chunks are whole slices, so a chunk's records end where the next slice's begin.
+    // Record rows of every color's chunk of every rank in a cluster of C blocks (C per color): the
+    // chunks are whole slices, so a chunk's rows end where the next slice's begin.
     std::vector<int4> cluster_ranges(int C) const {
         std::vector<int4> out;
-        const int mask = ~(dev::kSlice - 1);
         auto at = [&](int v) {
             if (v >= nactive_) return make_int2(nbr_end_, inc_end_);
-            return make_int2(vrec_[size_t(v)].x & mask, vrec_[size_t(v)].y & mask);
+            return make_int2(vrec_[size_t(v)].x, vrec_[size_t(v)].y);
         };
         for (const int2 c : scene_colors_) {
             const int per = dev::cluster_chunk(c.y - c.x, C);

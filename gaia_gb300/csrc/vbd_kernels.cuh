@@ -33,10 +33,11 @@
 //       IncRec (8 B FP32, 16 B FP64): per incident tet the positions of its three other
 //         vertices in the vertex's neighbour list (8 bits each, in the order whose rows have
 //         determinant det DmInv, and the nearest one's again) and w = 1 / (6 A) = det DmInv.
-//     The records of eight consecutive vertices are interleaved (record k of a vertex lies
-//     kSlice places after its record k - 1), so that lanes on neighbouring vertices read
-//     neighbouring records. vrec[s] = (first NbrRec, first IncRec, their numbers). Lists of
-//     more than kSegNbrs neighbours are cut into segments, the further ones in vmore.
+//     The records of eight consecutive vertices are interleaved in rows (record k of a vertex
+//     lies kSlice places after its record k - 1), so that lanes on neighbouring vertices read
+//     neighbouring records. vrec[s] = (first rows, numbers and place in the row, see
+//     record_index.hpp). Lists of more than kSegNbrs neighbours are cut into segments, the
+//     further ones in vmore.
 //
 // Per vertex the Neo-Hookean block is evaluated in closed form from differences of rest
 // positions, r = X_n - X_o, and of displacements, e = u_n - u_o. With (0, 1, 2) the tet's
@@ -73,6 +74,7 @@
 #include <string.h>
 
 #include "cloth_dev.cuh"
+#include "record_index.hpp"
 #include "vbd_state.cuh"
 
 namespace gaia {
@@ -118,8 +120,6 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 enum { CNT_FP64_SOLVES = 0, CNT_FAILED_SOLVES = 1, CNT_NONFINITE = 2, CNT_TIMEOUT = 3, CNT_DRAIN = 4, CNT_N = 8 };
 
 // One-ring and incidence records (see the top of the file), each one vector load.
-constexpr int kSegNbrs = 128;  // neighbours per segment at most (8-bit positions)
-constexpr int kSlice = 8;      // vertices whose records are interleaved
 template <typename R>
 struct NbrRec;
 template <>
@@ -153,7 +153,7 @@ struct Ptrs {
     typename ST::U* xprev;
     typename ST::V* vel;
     typename ST::V* vprev;
-    const int4* vrec;          // per slot: first NbrRec, first IncRec, number of each
+    const int4* vrec;          // per slot: first rows of its records and their numbers
     const int2* vmore;         // per slot its further segments [x, y) in segs; null: there are none
     const int4* segs;          // the further segments, as vrec
     const NbrRec<R>* nbr;
@@ -459,9 +459,9 @@ struct SegRecs {
 template <int L, int RR, typename R, int NB>
 __device__ __forceinline__ void preload(SegRecs<R, NB>& s, const NbrRec<R>* nbr, const IncRec<R>* inc, int4 seg,
                                         int sub) {
-    s.np = nbr + seg.x;
-    s.ip = inc + seg.y;
-    s.nn = seg.z;
+    s.np = nbr + record_index(seg.x, place_of(seg.z));
+    s.ip = inc + record_index(seg.y, place_of(seg.z));
+    s.nn = nbrs_of(seg.z);
     s.ni = seg.w;
 #pragma unroll
     for (int j = 0; j < NB; ++j)
@@ -888,7 +888,7 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* addr, uint32_t byte
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(addr), "r"(bytes) : "memory");
 }
 
-// The record ranges of the vertices [v0, v1): whole slices, from the slice of v0 to the end of
+// The record rows of the vertices [v0, v1): whole slices, from the slice of v0 to the end of
 // the longest list that the slice of v1 - 1 can hold (max_nbr, max_inc per vertex of the
 // color; the arrays are padded by as much).
 struct RecTile {
@@ -897,8 +897,7 @@ struct RecTile {
 template <typename ST, typename R>
 __device__ __forceinline__ RecTile rec_tile(const Ptrs<ST, R>& P, int v0, int v1, int max_nbr, int max_inc) {
     const int4 r0 = P.vrec[v0], r1 = P.vrec[v1 - 1];
-    return RecTile{r0.x & ~(kSlice - 1), (r1.x & ~(kSlice - 1)) + kSlice * max_nbr, r0.y & ~(kSlice - 1),
-                   (r1.y & ~(kSlice - 1)) + kSlice * max_inc};
+    return RecTile{r0.x, r1.x + max_nbr, r0.y, r1.y + max_inc};
 }
 
 // What the warp `pf` warps on (one resident wave later) will load first, into L2: its records
@@ -911,8 +910,8 @@ __device__ __forceinline__ void prefetch_vertices(const Ptrs<ST, R>& P, int v, i
     if (va >= end) return;
     if (Lanes<L>::vertex() % kSlice == 0 && Lanes<L>::sub() == 0) {
         // one lane per slice: the longest list is at most a little longer than its first vertex's
-        bulk_prefetch_l2(P.nbr + (ahead.x & ~(kSlice - 1)), uint32_t(max(ahead.z, 1)) * uint32_t(kSlice * sizeof(NbrRec<R>)));
-        bulk_prefetch_l2(P.inc + (ahead.y & ~(kSlice - 1)), uint32_t(max(ahead.w, 1)) * uint32_t(kSlice * sizeof(IncRec<R>)));
+        bulk_prefetch_l2(P.nbr + record_index(ahead.x, 0), uint32_t(max(nbrs_of(ahead.z), 1)) * uint32_t(kSlice * sizeof(NbrRec<R>)));
+        bulk_prefetch_l2(P.inc + record_index(ahead.y, 0), uint32_t(max(ahead.w, 1)) * uint32_t(kSlice * sizeof(IncRec<R>)));
     }
     if (Lanes<L>::sub() == L - 1) {
         asm volatile("prefetch.global.L2 [%0];" ::"l"(P.rest + va));
@@ -1191,10 +1190,10 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 template <typename ST>
 __device__ __forceinline__ void issue_tile(const Ptrs<ST, float>& P, const RecTile& t, NbrRec<float>* s_nbr,
                                            IncRec<float>* s_inc, uint32_t bar) {
-    const uint32_t nb = uint32_t(t.n1 - t.n0) * 8u, ib = uint32_t(t.i1 - t.i0) * 8u;
+    const uint32_t nb = uint32_t(t.n1 - t.n0) * uint32_t(8 * kSlice), ib = uint32_t(t.i1 - t.i0) * uint32_t(8 * kSlice);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(nb + ib) : "memory");
-    if (nb) bulk_g2s(s_nbr, P.nbr + t.n0, nb, bar);
-    if (ib) bulk_g2s(s_inc, P.inc + t.i0, ib, bar);
+    if (nb) bulk_g2s(s_nbr, P.nbr + record_index(t.n0, 0), nb, bar);
+    if (ib) bulk_g2s(s_inc, P.inc + record_index(t.i0, 0), ib, bar);
 }
 
 template <int L, bool CONTACT, typename ST>
