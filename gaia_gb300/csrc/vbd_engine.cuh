@@ -656,6 +656,10 @@ public:
     // vertex) and incidences.
     int2 max_lists(int beg, int end) {
         if (multi_seg_) return make_int2(max_nbr_all_, max_inc_all_);
+        if (end - beg == 1) {  // a probed vertex: any of the scene's, so not kept
+            const int4 r = vrec_[size_t(beg)];
+            return make_int2(std::max(2, (dev::nbrs_of(r.z) + 1) & ~1), std::max(1, r.w));
+        }
         const auto key = std::make_pair(beg, end);
         auto it = lists_cache_.find(key);
         if (it != lists_cache_.end()) return it->second;
