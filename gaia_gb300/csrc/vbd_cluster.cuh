@@ -65,16 +65,24 @@ struct FetchClusterLean {
 };
 
 struct ClusterScenes {
-    const int2* colors;        // slot ranges of the scenes' colors (scene-major slot layout)
+    const int4* colors;        // slot ranges of the scenes' colors (scene-major slot layout): first,
+                               // first of the vertices with long lists, end
     const int32_t* scene_ofs;  // colors of scene m: colors[scene_ofs[m] .. scene_ofs[m + 1])
     const int32_t* scene_order;
     const int4* scene_slots;   // per scene: active slots [x, y), fixed slots [z, w)
     int32_t nscenes, iterations, friction_start;
     int32_t pos_cap;           // states each block's shared copy holds
     int32_t nbr_cap, inc_cap;  // neighbour and incidence records each block holds
-    int32_t stage_cap;         // staging entries per vertex
-    const int4* ranges;        // per color and rank: its record rows in the global arrays (colors of all
-                               // scenes, C per color): first and last + 1 of NbrRec and IncRec
+    SweepStage stage;
+    const int4* ranges;        // per color, rank and kind of list (short, long): its record rows in the global
+                               // arrays (colors of all scenes, 2 C per color): first and last + 1 of NbrRec
+                               // and IncRec
+};
+
+// A compile-time number as an argument.
+template <int N>
+struct IntC {
+    static constexpr int value = N;
 };
 
 // A state broadcast from lane src of the warp (every field of the trait's state type).
@@ -90,12 +98,69 @@ __device__ __forceinline__ typename ST::U shfl_state(typename ST::U u, int src) 
     return u;
 }
 
-// LEAN: only the states in shared memory (nbr_cap and inc_cap 0), for a scene whose records
-// and rest positions do not fit beside them.
-template <int L, bool MULTI, bool LEAN, typename ST, typename R>
-__global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> c, ClusterScenes S, int32_t* work) {
+// One block's chunk [beg, end) of a color's short or long lists: solved, and every new state
+// written into all copies. nbr, inc: the records that vrec's rows count from.
+template <int L, bool MULTI, bool LEAN, typename ST, typename R, typename Fetch>
+__device__ __forceinline__ void cluster_range(const Ptrs<ST, R>& P, const Consts<R>& c, cg::cluster_group& cluster, int C,
+                                              int beg, int end, const int4& sl, typename ST::U* spos, const float4* srest,
+                                              const NbrRec<R>* nbr, const IncRec<R>* inc, unsigned char* stage, int cap,
+                                              int warp_bytes, const Fetch& fetch, int friction) {
     using U = typename ST::U;
     constexpr int NB = L >= 16 ? 1 : 2;
+    constexpr int RR = LEAN ? kRecKept : kRecShared;
+    const int groups = int(blockDim.x) / L;
+    const int g = int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
+    const int sub = Lanes<L>::sub();
+    for (int base = beg; base < end; base += groups) {
+        const int v = base + g;
+        const bool valid = v < end;
+        Acc<R> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+        U uo{};
+        MeshMat<R> mat{};
+        float4 Xo = make_float4(0.f, 0.f, 0.f, 0.f);
+        int4 seg = make_int4(0, 0, 0, 0);
+        if (valid) {
+            if (sub == 0) prefetch_tail<L>(P, v);
+            seg = P.vrec[v];
+            mat = P.mats[P.slot_mesh[v]];
+            uo = spos[v - sl.x];
+            Xo = LEAN ? __ldg(P.rest + v) : srest[v - sl.x];
+        }
+        const U uon = ST::nb(uo);
+        SegRecs<R, NB> rec;
+        const Stage<32 / L, ST, R> st = warp_stage<L, ST, R>(stage, cap, size_t(warp_bytes));
+        preload<L, RR>(rec, nbr, inc, seg, sub);
+        accumulate_segment<L, RR, false, ST>(rec, sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
+        if constexpr (MULTI)
+            if (valid)
+                accumulate_more<L, RR, false, ST>(rec, P, nbr, inc, P.vmore[v], sub, st, fetch, uon, Xo, mat.mu, mat.lmbd,
+                                                  acc);
+        __syncwarp();
+        reduce_group<L, R>(acc);
+        // lane 0 solves; the group's lanes then write the new state into the C
+        // copies, one remote store each, instead of lane 0 writing all of them
+        U un{};
+        int moved = 0;
+        if (valid && sub == 0) {
+            finish_acc(acc, mat.mu, mat.lmbd);
+            moved = vertex_tail<ST, R, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr, nullptr, &un) ? 1 : 0;
+        }
+        const int src = Lanes<L>::vertex();
+        moved = __shfl_sync(0xffffffffu, moved, src);
+        un = shfl_state<ST>(un, src);
+        if (valid && moved) {
+            const int lv = v - sl.x;
+            for (int r = sub; r < C; r += L) *cluster.map_shared_rank(&spos[lv], r) = un;
+        }
+    }
+}
+
+// LEAN: only the states in shared memory (nbr_cap and inc_cap 0), for a scene whose records
+// and rest positions do not fit beside them. LONG: there are vertices with long lists.
+template <int L, bool LONG, bool LEAN, typename ST, typename R>
+__global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> c, ClusterScenes S, int32_t* work) {
+    using U = typename ST::U;
+    constexpr int kKinds = LONG ? 2 : 1;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = int(cluster.block_rank());
     const int C = int(cluster.num_blocks());
@@ -106,10 +171,7 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
     IncRec<R>* sinc = reinterpret_cast<IncRec<R>*>(snbr + S.nbr_cap);
     unsigned char* stage = reinterpret_cast<unsigned char*>(sinc + S.inc_cap);
     __shared__ int s_scene;
-    __shared__ int2 s_rec_base[kClusterMaxColors + 1];
-    const int groups = int(blockDim.x) / L;
-    const int g = int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
-    const int sub = Lanes<L>::sub();
+    __shared__ int2 s_rec_base[2 * kClusterMaxColors];
     for (;;) {
         // rank 0 takes the next scene and hands it to every block of the cluster
         if (rank == 0 && threadIdx.x == 0) {
@@ -128,23 +190,25 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
             if constexpr (LEAN) return FetchClusterLean<ST>{spos, P.rest, sl};
             else return FetchCluster<ST>{spos, srest};
         }();
-        constexpr int RR = LEAN ? kRecKept : kRecShared;
-        // this block's chunk of color ci: [beg, end)
-        auto chunk = [&](int ci, int& beg, int& end) {
-            const int2 rg = S.colors[ci];
-            const int per = cluster_chunk(rg.y - rg.x, C);
-            beg = min(rg.y, rg.x + rank * per);
-            end = min(rg.y, beg + per);
+        // this block's chunk of the short (kind 0) or long lists of color ci: [beg, end)
+        auto chunk = [&](int ci, int kind, int& beg, int& end) {
+            const int4 rg = S.colors[ci];
+            const int lo = kind ? rg.y : rg.x, hi = kind ? rg.z : rg.y;
+            const int per = cluster_chunk(hi - lo, C);
+            beg = min(hi, lo + rank * per);
+            end = min(hi, beg + per);
         };
-        // per color, the row where the chunk's records start in the shared arrays, less their global one
+        auto rows = [&](int ci, int kind) { return S.ranges[2 * (ci * C + rank) + kind]; };
+        // per chunk, the row where its records start in the shared arrays, less their global one
         if (!LEAN && threadIdx.x == 0) {
             int2 base = make_int2(0, 0);
-            for (int ci = c0; ci < c1; ++ci) {
-                const int4 r = S.ranges[ci * C + rank];
-                s_rec_base[ci - c0] = make_int2(base.x - r.x, base.y - r.z);
-                base.x += r.y - r.x;
-                base.y += r.w - r.z;
-            }
+            for (int ci = c0; ci < c1; ++ci)
+                for (int k = 0; k < kKinds; ++k) {
+                    const int4 r = rows(ci, k);
+                    s_rec_base[2 * (ci - c0) + k] = make_int2(base.x - r.x, base.y - r.z);
+                    base.x += r.y - r.x;
+                    base.y += r.w - r.z;
+                }
         }
         // stage: all the scene's states and rest positions, this block's records
         const int nloc = na + (sl.w - sl.z);
@@ -154,9 +218,10 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
             if (!LEAN) srest[i] = P.rest[s];
         }
         __syncthreads();
-        for (int ci = c0; !LEAN && ci < c1; ++ci) {
-            const int4 r = S.ranges[ci * C + rank];
-            const int2 sb = s_rec_base[ci - c0];
+        for (int q = kKinds * c0; !LEAN && q < kKinds * c1; ++q) {
+            const int ci = q / kKinds, k = q % kKinds;
+            const int4 r = rows(ci, k);
+            const int2 sb = s_rec_base[2 * (ci - c0) + k];
             const NbrRec<R>* gn = P.nbr + record_index(r.x, 0);
             const IncRec<R>* gi = P.inc + record_index(r.z, 0);
             NbrRec<R>* dn = snbr + (sb.x + r.x) * kSlice;
@@ -172,60 +237,24 @@ __global__ void __launch_bounds__(256) k_sweep_cluster(Ptrs<ST, R> P, Consts<R> 
         for (int it = 0; it < S.iterations; ++it) {
             const int friction = it >= S.friction_start ? 1 : 0;
             for (int ci = c0; ci < c1; ++ci) {
-                int beg, end;
-                chunk(ci, beg, end);
-                const int2 sb = LEAN ? make_int2(0, 0) : s_rec_base[ci - c0];
-                const NbrRec<R>* nbr = LEAN ? P.nbr : snbr + ptrdiff_t(sb.x) * kSlice;
-                const IncRec<R>* inc = LEAN ? P.inc : sinc + ptrdiff_t(sb.y) * kSlice;
-                for (int base = beg; base < end; base += groups) {
-                    const int v = base + g;
-                    const bool valid = v < end;
-                    Acc<R> acc = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-                    U uo{};
-                    MeshMat<R> mat{};
-                    float4 Xo = make_float4(0.f, 0.f, 0.f, 0.f);
-                    int4 seg = make_int4(0, 0, 0, 0);
-                    if (valid) {
-                        if (sub == 0) prefetch_tail<L>(P, v);
-                        seg = P.vrec[v];
-                        mat = P.mats[P.slot_mesh[v]];
-                        uo = spos[v - sl.x];
-                        Xo = LEAN ? __ldg(P.rest + v) : srest[v - sl.x];
-                    }
-                    const U uon = ST::nb(uo);
-                    SegRecs<R, NB> rec;
-                    const Stage<32 / L, ST, R> st = warp_stage<L, ST, R>(stage, S.stage_cap);
-                    preload<L, RR>(rec, nbr, inc, seg, sub);
-                    accumulate_segment<L, RR, false, ST>(rec, sub, st, fetch, uon, Xo, mat.mu, mat.lmbd, acc);
-                    if constexpr (MULTI)
-                        if (valid)
-                            accumulate_more<L, RR, false, ST>(rec, P, nbr, inc, P.vmore[v], sub, st, fetch, uon, Xo, mat.mu, mat.lmbd,
-                                                       acc);
-                    __syncwarp();
-                    reduce_group<L, R>(acc);
-                    // lane 0 solves; the group's lanes then write the new state into the C
-                    // copies, one remote store each, instead of lane 0 writing all of them
-                    U un{};
-                    int moved = 0;
-                    if (valid && sub == 0) {
-                        finish_acc(acc, mat.mu, mat.lmbd);
-                        moved = vertex_tail<ST, R, false>(P, c, v, uo, Xo, frame_offset(P, v), mat, acc, friction, nullptr, nullptr, &un) ? 1 : 0;
-                    }
-                    const int src = Lanes<L>::vertex();
-                    moved = __shfl_sync(0xffffffffu, moved, src);
-                    un = shfl_state<ST>(un, src);
-                    if (valid && moved) {
-                        const int lv = v - sl.x;
-                        for (int r = sub; r < C; r += L) *cluster.map_shared_rank(&spos[lv], r) = un;
-                    }
-                }
+                auto solve = [&](auto lanes, auto multi, int kind, int cap) {
+                    int beg, end;
+                    chunk(ci, kind, beg, end);
+                    const int2 sb = LEAN ? make_int2(0, 0) : s_rec_base[2 * (ci - c0) + kind];
+                    const NbrRec<R>* nbr = LEAN ? P.nbr : snbr + ptrdiff_t(sb.x) * kSlice;
+                    const IncRec<R>* inc = LEAN ? P.inc : sinc + ptrdiff_t(sb.y) * kSlice;
+                    cluster_range<lanes.value, multi.value, LEAN, ST, R>(P, c, cluster, C, beg, end, sl, spos, srest, nbr, inc,
+                                                                         stage, cap, S.stage.warp_bytes, fetch, friction);
+                };
+                solve(IntC<L>{}, IntC<0>{}, 0, S.stage.cap);
+                if constexpr (LONG) solve(IntC<32>{}, IntC<1>{}, 1, S.stage.cap_long);
                 cluster.sync();  // this color's states in every copy before the next color
             }
         }
         // the owned vertices back to global memory
-        for (int ci = c0; ci < c1; ++ci) {
+        for (int q = kKinds * c0; q < kKinds * c1; ++q) {
             int beg, end;
-            chunk(ci, beg, end);
+            chunk(q / kKinds, q % kKinds, beg, end);
             for (int v = beg + int(threadIdx.x); v < end; v += blockDim.x) P.u[v] = spos[v - sl.x];
         }
         cluster.sync();  // no block stages the next scene while another still reads this one

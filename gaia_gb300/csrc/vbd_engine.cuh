@@ -222,7 +222,10 @@ public:
         slot_of_.assign(nslots_, -1);
         int32_t slot = 0;
         group_beg_.clear();
+        group_mid_.clear();
         group_end_.clear();
+        find_long_lists();
+        deal_ofs_.assign(1, 0);
         scene_colors_.clear();
         scene_ofs_.assign(1, 0);
         if (mode_ == kSweepScenes || mode_ == kSweepCluster) {
@@ -240,19 +243,27 @@ public:
                 for (auto& verts : per[size_t(m)]) {
                     if (verts.empty()) continue;
                     const int32_t beg = slot;
-                    for (int32_t v : verts) slot_of_[mesh_off_[m] + v] = slot++;
-                    scene_colors_.push_back(make_int2(beg, slot));
+                    for (int32_t v : verts)
+                        deal_ofs_.push_back(deal_ofs_.back() + meshes[m].nbr_ofs[v + 1] - meshes[m].nbr_ofs[v]);
+                    for (int32_t v : verts)
+                        if (!is_long(m, v)) slot_of_[mesh_off_[m] + v] = slot++;
+                    const int32_t mid = slot;
+                    for (int32_t v : verts)
+                        if (is_long(m, v)) slot_of_[mesh_off_[m] + v] = slot++;
+                    scene_colors_.push_back(make_int4(beg, mid, slot, 0));
                 }
                 scene_ofs_.push_back(int32_t(scene_colors_.size()));
             }
         } else {
             for (auto& g : sc_.groups) {
                 group_beg_.push_back(slot);
-                for (size_t i = 0; i + 1 < g.size(); i += 2) {
-                    int m = g[i], v = g[i + 1];
-                    if (!meshes[m].fixed[v]) slot_of_[mesh_off_[m] + v] = slot++;
+                for (int part = 0; part < 2; ++part) {
+                    for (size_t i = 0; i + 1 < g.size(); i += 2) {
+                        int m = g[i], v = g[i + 1];
+                        if (!meshes[m].fixed[v] && is_long(m, v) == (part == 1)) slot_of_[mesh_off_[m] + v] = slot++;
+                    }
+                    (part ? group_end_ : group_mid_).push_back(slot);
                 }
-                group_end_.push_back(slot);
             }
         }
         nactive_ = slot;
@@ -357,9 +368,55 @@ public:
         c_.spin_limit = p.waitPollLimit >= 0 ? p.waitPollLimit : dev::kMbarSpinLimit;
     }
 
+    // Vertices with long neighbour lists come last in their color and are solved a warp per
+    // vertex, in a launch of their own where the others take fewer lanes: the staging areas of a
+    // launch are sized by its longest list, and only that form holds lists of more than kSegNbrs.
+    // Long is more than 32 neighbours (a tet mesh has about 14, a 5-tet lattice up to 18), or 64
+    // or kSegNbrs where more than a 32nd of the vertices would be long. Vertices of up to
+    // kFewTets tets are not counted out: 42 tets hold at most 126 neighbours, and about 23 where
+    // they share faces. A step of a 40^3 lattice at 4 lanes (FP32, 10 iterations) takes 1.15 times
+    // as long with one hub of 202 neighbours beside it; when such a vertex changed the whole scene
+    // over to a warp per vertex, 1.57 times.
+    static constexpr int kFewTets = 42;
+    void find_long_lists() {
+        const auto& meshes = sc_.meshes;
+        std::vector<std::vector<uint8_t>> over(meshes.size());  // 1: > 32, 2: > 64, 3: > kSegNbrs neighbours
+        int64_t count[4] = {0, 0, 0, 0}, active = 0;
+        std::vector<int32_t> nb;
+        for (size_t m = 0; m < meshes.size(); ++m) {
+            const TetMesh& M = meshes[m];
+            for (int32_t v = 0; v < M.nv; ++v) {
+                if (M.fixed[v]) continue;
+                ++active;
+                if (M.nbr_ofs[v + 1] - M.nbr_ofs[v] <= kFewTets) continue;
+                nb.clear();
+                for (int q = M.nbr_ofs[v]; q < M.nbr_ofs[v + 1]; ++q)
+                    for (int j = 0; j < 4; ++j)
+                        if (j != M.nbr_order[q]) nb.push_back(M.tets[4 * size_t(M.nbr_tet[q]) + j]);
+                std::sort(nb.begin(), nb.end());
+                const int64_t n = std::unique(nb.begin(), nb.end()) - nb.begin();
+                const int k = n > dev::kSegNbrs ? 3 : (n > 64 ? 2 : (n > 32 ? 1 : 0));
+                if (!k) continue;
+                if (over[m].empty()) over[m].assign(size_t(M.nv), 0);
+                over[m][size_t(v)] = uint8_t(k);
+                ++count[k];
+            }
+        }
+        int line = 1;
+        if (32 * (count[1] + count[2] + count[3]) > active) line = 32 * (count[2] + count[3]) > active ? 3 : 2;
+        any_long_ = false;
+        for (auto& o : over)
+            for (auto& k : o) {
+                k = k >= line ? 1 : 0;
+                any_long_ = any_long_ || k;
+            }
+        long_ = std::move(over);
+    }
+    bool is_long(int m, int v) const { return !long_[size_t(m)].empty() && long_[size_t(m)][size_t(v)]; }
+
     // One-ring and incidence records of the active slots (layout in vbd_kernels.cuh), the host
     // threads taking contiguous ranges of slices; a color (of the merged sweep, or of one
-    // scene) starts a slice. Neighbours are listed by slot, so that the k-th neighbours of
+    // scene) starts a slice, and so do its long lists. Neighbours are listed by slot, so that the k-th neighbours of
     // consecutive vertices of a regular mesh are consecutive too; incidences keep the mesh's
     // ascending tet order, and a segment closes when the next tet's vertices would take it
     // past kSegNbrs neighbours.
@@ -378,9 +435,15 @@ public:
             for (int v = beg; v < end; v += dev::kSlice) slices.push_back(make_int2(v, std::min(end, v + dev::kSlice)));
         };
         if (mode_ == kSweepScenes || mode_ == kSweepCluster)
-            for (int2 c : scene_colors_) cut(c.x, c.y);
+            for (int4 c : scene_colors_) {
+                cut(c.x, c.y);
+                cut(c.y, c.z);
+            }
         else
-            for (size_t g = 0; g < group_beg_.size(); ++g) cut(group_beg_[g], group_end_[g]);
+            for (size_t g = 0; g < group_beg_.size(); ++g) {
+                cut(group_beg_[g], group_mid_[g]);
+                cut(group_mid_[g], group_end_[g]);
+            }
         struct Seg {
             int32_t slot;                // its vertex
             int4 r;                      // as vrec
@@ -464,7 +527,7 @@ public:
         nbr_end_ = checked_count(int64_t(nn / dev::kSlice));
         inc_end_ = checked_count(int64_t(ni / dev::kSlice));
         // the parts end to end, padded for the copies of whole slices that run past the last list
-        max_nbr_all_ = max_inc_all_ = 2;
+        max_nbr_all_ = max_nbr_short_ = max_inc_all_ = 2;
         h_nbr_.clear();
         h_inc_.clear();
         h_nbr_.reserve(nn + size_t(dev::kSlice) * 1024);
@@ -487,8 +550,11 @@ public:
             h_nbr_.insert(h_nbr_.end(), q.nbr.begin(), q.nbr.end());
             h_inc_.insert(h_inc_.end(), q.inc.begin(), q.inc.end());
         }
-        for (const int4& r : vrec_) {
-            max_nbr_all_ = std::max(max_nbr_all_, (dev::nbrs_of(r.z) + 1) & ~1);
+        for (int32_t q = 0; q < nactive_; ++q) {
+            const int4 r = vrec_[size_t(q)];
+            const int n = (dev::nbrs_of(r.z) + 1) & ~1;
+            max_nbr_all_ = std::max(max_nbr_all_, n);
+            if (!long_slot(q)) max_nbr_short_ = std::max(max_nbr_short_, n);
             max_inc_all_ = std::max(max_inc_all_, r.w);
         }
         for (const Seg& e : more) max_nbr_all_ = std::max(max_nbr_all_, (dev::nbrs_of(e.r.z) + 1) & ~1);
@@ -496,7 +562,7 @@ public:
         h_inc_.resize(h_inc_.size() + size_t(dev::kSlice) * max_inc_all_, dev::IncRec<R>{});
         multi_seg_ = !more.empty();
         vmore_.clear();
-        if (multi_seg_) {
+        if (any_long_) {  // (the sweeps read it for every long list)
             vmore_.assign(size_t(nactive_), make_int2(0, 0));
             std::stable_sort(more.begin(), more.end(), [](const Seg& a, const Seg& b) { return a.slot < b.slot; });
             for (size_t i = 0; i < more.size(); ++i) {
@@ -655,11 +721,6 @@ public:
     // Longest lists in the slot range [beg, end): neighbours (even: the staging entries per
     // vertex) and incidences.
     int2 max_lists(int beg, int end) {
-        if (multi_seg_) return make_int2(max_nbr_all_, max_inc_all_);
-        if (end - beg == 1) {  // a probed vertex: any of the scene's, so not kept
-            const int4 r = vrec_[size_t(beg)];
-            return make_int2(std::max(2, (dev::nbrs_of(r.z) + 1) & ~1), std::max(1, r.w));
-        }
         const auto key = std::make_pair(beg, end);
         auto it = lists_cache_.find(key);
         if (it != lists_cache_.end()) return it->second;
@@ -667,17 +728,35 @@ public:
         for (int v = beg; v < end; ++v) {
             m.x = std::max(m.x, (dev::nbrs_of(vrec_[size_t(v)].z) + 1) & ~1);
             m.y = std::max(m.y, vrec_[size_t(v)].w);
+            if (several_segments(v)) m.x = dev::kSegNbrs;
         }
-        return lists_cache_[key] = m;
+        if (end - beg > 1) lists_cache_[key] = m;  // (a single vertex is a probed one: any of the scene's)
+        return m;
+    }
+    bool several_segments(int slot) const { return multi_seg_ && vmore_[size_t(slot)].y > vmore_[size_t(slot)].x; }
+    bool long_slot(int slot) const {
+        const int m = slot_mesh_[size_t(slot)];
+        return is_long(m, orig_of_[size_t(slot)] - int32_t(mesh_off_[m]));
     }
     // Bytes of the staging areas of a block of B threads.
     static size_t stage_bytes(int cap, int L, int B) {
         return size_t(B / L) * size_t(cap) * (16 * dev::Stage<1, ST, R>::kParts);
     }
-    // Fewest lanes per vertex, at least L, whose staging fits the shared memory of a block
-    // (32 where a vertex has several segments: those kernels take one vertex per warp).
+    // The same for a persistent sweep: L lanes per vertex, a warp per vertex for the long lists.
+    dev::SweepStage sweep_stage(int L) const {
+        dev::SweepStage S;
+        S.cap = max_nbr_short_;
+        S.cap_long = any_long_ ? max_nbr_all_ : 0;
+        S.warp_bytes = int(std::max(stage_bytes(S.cap, L, 32), stage_bytes(S.cap_long, 32, 32)));
+        return S;
+    }
+    size_t sweep_stage_bytes(int L, int B) const { return size_t(B / 32) * size_t(sweep_stage(L).warp_bytes); }
+    int fit_sweep_lanes(int L, int B) const {
+        while (L < 32 && sweep_stage_bytes(L, B) > kTmaSmemMax) L *= 2;
+        return L;
+    }
+    // Fewest lanes per vertex, at least L, whose staging fits the shared memory of a block.
     int fit_lanes(int L, int B, int beg, int end) {
-        if (multi_seg_) return 32;
         while (L < 32 && stage_bytes(max_lists(beg, end).x, L, B) > kTmaSmemMax) L *= 2;
         return L;
     }
@@ -887,12 +966,12 @@ public:
     // the previous kernel in the stream (its static-data prologue overlaps that
     // kernel's tail; k_solve waits on griddepcontrol before reading positions).
     template <bool PROBE, bool DEEP, int L, bool MULTI = false>
-    void launch_solve_l(int B, int beg, int end, int friction, double* probe, bool pdl, bool prefetch) {
-        if (cd_.enabled()) launch_solve_c<PROBE, DEEP, L, MULTI, true>(B, beg, end, friction, probe, pdl, prefetch);
-        else launch_solve_c<PROBE, DEEP, L, MULTI, false>(B, beg, end, friction, probe, pdl, prefetch);
+    void launch_solve_l(int B, int beg, int end, int2 color, int flags, double* probe, bool pdl, bool prefetch) {
+        if (cd_.enabled()) launch_solve_c<PROBE, DEEP, L, MULTI, true>(B, beg, end, color, flags, probe, pdl, prefetch);
+        else launch_solve_c<PROBE, DEEP, L, MULTI, false>(B, beg, end, color, flags, probe, pdl, prefetch);
     }
     template <bool PROBE, bool DEEP, int L, bool MULTI, bool CONTACT>
-    void launch_solve_c(int B, int beg, int end, int friction, double* probe, bool pdl, bool prefetch) {
+    void launch_solve_c(int B, int beg, int end, int2 color, int flags, double* probe, bool pdl, bool prefetch) {
         const int cap = max_lists(beg, end).x;
         const size_t smem = stage_bytes(cap, L, B);
         auto kern = dev::k_solve<L, ST, R, PROBE, DEEP, MULTI, CONTACT>;
@@ -909,7 +988,7 @@ public:
         cfg.numAttrs = pdl ? 1 : 0;
         // the prefetching variant fetches for the warps one resident wave ahead
         const int pf = prefetch ? std::max(1, blocks_per_sm(kern, B, smem)) * sm_count() * (B / 32) : 0;
-        GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, friction, probe, pf, cap));
+        GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, color, flags, probe, pf, cap));
     }
 
     template <typename K>
@@ -949,7 +1028,7 @@ public:
     }
 
     template <int L>
-    bool launch_solve_tma_l(int B, int beg, int end, int friction, bool pdl) {
+    bool launch_solve_tma_l(int B, int beg, int end, int2 color, int flags, bool pdl) {
         if constexpr (sizeof(R) != 4) {
             return false;
         } else {
@@ -970,14 +1049,14 @@ public:
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = pdl ? attr : nullptr;
             cfg.numAttrs = pdl ? 1 : 0;
-            GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, friction, lists.x, lists.y, mr.x, mr.y));
+            GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, color, flags, lists.x, lists.y, mr.x, mr.y));
             return true;
         }
     }
 
     // Double-buffered TMA pipeline on a persistent grid (FP32 compute, both tile buffers fit).
     template <int L>
-    bool launch_solve_pipe_l(int B, int beg, int end, int friction, bool pdl) {
+    bool launch_solve_pipe_l(int B, int beg, int end, int2 color, int flags, bool pdl) {
         if constexpr (sizeof(R) != 4) {
             return false;
         } else {
@@ -1001,59 +1080,73 @@ public:
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = pdl ? attr : nullptr;
             cfg.numAttrs = pdl ? 1 : 0;
-            GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, friction, lists.x, lists.y, mr.x, mr.y));
+            GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, beg, end, color, flags, lists.x, lists.y, mr.x, mr.y));
             return true;
         }
     }
 
-    bool launch_solve_pipe(int L, int B, int beg, int end, int friction, bool pdl) {
+    bool launch_solve_pipe(int L, int B, int beg, int end, int2 color, int flags, bool pdl) {
         switch (L) {
-            case 2: return launch_solve_pipe_l<2>(B, beg, end, friction, pdl);
-            case 4: return launch_solve_pipe_l<4>(B, beg, end, friction, pdl);
-            case 8: return launch_solve_pipe_l<8>(B, beg, end, friction, pdl);
-            case 16: return launch_solve_pipe_l<16>(B, beg, end, friction, pdl);
-            default: return launch_solve_pipe_l<32>(B, beg, end, friction, pdl);
+            case 2: return launch_solve_pipe_l<2>(B, beg, end, color, flags, pdl);
+            case 4: return launch_solve_pipe_l<4>(B, beg, end, color, flags, pdl);
+            case 8: return launch_solve_pipe_l<8>(B, beg, end, color, flags, pdl);
+            case 16: return launch_solve_pipe_l<16>(B, beg, end, color, flags, pdl);
+            default: return launch_solve_pipe_l<32>(B, beg, end, color, flags, pdl);
         }
     }
 
     // TMA-staged launch if this engine computes in FP32 and the block's records fit.
-    bool launch_solve_tma(int L, int B, int beg, int end, int friction, bool pdl) {
+    bool launch_solve_tma(int L, int B, int beg, int end, int2 color, int flags, bool pdl) {
         switch (L) {
-            case 2: return launch_solve_tma_l<2>(B, beg, end, friction, pdl);
-            case 4: return launch_solve_tma_l<4>(B, beg, end, friction, pdl);
-            case 8: return launch_solve_tma_l<8>(B, beg, end, friction, pdl);
-            case 16: return launch_solve_tma_l<16>(B, beg, end, friction, pdl);
-            default: return launch_solve_tma_l<32>(B, beg, end, friction, pdl);
+            case 2: return launch_solve_tma_l<2>(B, beg, end, color, flags, pdl);
+            case 4: return launch_solve_tma_l<4>(B, beg, end, color, flags, pdl);
+            case 8: return launch_solve_tma_l<8>(B, beg, end, color, flags, pdl);
+            case 16: return launch_solve_tma_l<16>(B, beg, end, color, flags, pdl);
+            default: return launch_solve_tma_l<32>(B, beg, end, color, flags, pdl);
         }
     }
 
     template <bool PROBE, bool DEEP>
-    void launch_solve_reg(int L, int B, int beg, int end, int friction, double* probe, bool pdl, bool prefetch) {
+    void launch_solve_reg(int L, int B, int beg, int end, int2 color, int flags, double* probe, bool pdl, bool prefetch) {
         B = std::min(B, 256);  // the probe of an engine whose schedule runs larger blocks
-        if (multi_seg_) {
-            launch_solve_l<PROBE, false, 32, true>(B, beg, end, friction, probe, pdl, prefetch);
-            return;
-        }
         switch (fit_lanes(L, B, beg, end)) {
-            case 2: launch_solve_l<PROBE, DEEP, 2>(B, beg, end, friction, probe, pdl, prefetch); break;
-            case 4: launch_solve_l<PROBE, DEEP, 4>(B, beg, end, friction, probe, pdl, prefetch); break;
-            case 8: launch_solve_l<PROBE, DEEP, 8>(B, beg, end, friction, probe, pdl, prefetch); break;
-            case 16: launch_solve_l<PROBE, false, 16>(B, beg, end, friction, probe, pdl, prefetch); break;
-            default: launch_solve_l<PROBE, false, 32>(B, beg, end, friction, probe, pdl, prefetch); break;
+            case 2: launch_solve_l<PROBE, DEEP, 2>(B, beg, end, color, flags, probe, pdl, prefetch); break;
+            case 4: launch_solve_l<PROBE, DEEP, 4>(B, beg, end, color, flags, probe, pdl, prefetch); break;
+            case 8: launch_solve_l<PROBE, DEEP, 8>(B, beg, end, color, flags, probe, pdl, prefetch); break;
+            case 16: launch_solve_l<PROBE, false, 16>(B, beg, end, color, flags, probe, pdl, prefetch); break;
+            default: launch_solve_l<PROBE, false, 32>(B, beg, end, color, flags, probe, pdl, prefetch); break;
         }
     }
 
+    // Vertices of any list length, a warp each.
     template <bool PROBE>
-    void launch_solve(int L, int B, int beg, int end, int friction, double* probe, bool pdl = false,
-                      int variant = 0) {
+    void launch_solve_wide(int B, int beg, int end, int2 color, int flags, double* probe, bool pdl) {
+        B = std::min(B, 256);
+        if (multi_seg_) launch_solve_l<PROBE, false, 32, true>(B, beg, end, color, flags, probe, pdl, false);
+        else launch_solve_l<PROBE, false, 32>(B, beg, end, color, flags, probe, pdl, false);
+    }
+
+    // The vertices [beg, end), none of them with a long list, of a color.
+    void launch_solve(int L, int B, int beg, int end, int2 color, int flags, bool pdl, int variant) {
+        if (variant == 1 && launch_solve_tma(L, B, beg, end, color, flags, pdl)) return;
+        if (variant == kVariantPipe && launch_solve_pipe(L, B, beg, end, color, flags, pdl)) return;
+        if (variant == kVariantDeep) launch_solve_reg<false, true>(L, B, beg, end, color, flags, nullptr, pdl, false);
+        else launch_solve_reg<false, false>(L, B, beg, end, color, flags, nullptr, pdl, variant == kVariantPrefetch);
+    }
+
+    // One color's solve. Its long lists take a launch of their own, unless all its vertices take a
+    // warp each anyway: a launch more costs as much as a small color (about 2.5 us).
+    void launch_color(size_t g, int L, int B, int flags, bool pdl, int variant) {
+        const int beg = group_beg_[g], mid = group_mid_[g], end = group_end_[g];
+        const int2 color = make_int2(beg, end);
         if (end <= beg) return;
-        if constexpr (PROBE) {
-            launch_solve_reg<true, false>(L, B, beg, end, friction, probe, pdl, false);
+        if (mid == end) {
+            launch_solve(L, B, beg, end, color, flags, pdl, variant);
+        } else if (mid == beg || (L == 32 && variant != 1 && variant != kVariantPipe)) {
+            launch_solve_wide<false>(B, beg, end, color, flags, nullptr, pdl);
         } else {
-            if (variant == 1 && !multi_seg_ && launch_solve_tma(L, B, beg, end, friction, pdl)) return;
-            if (variant == kVariantPipe && !multi_seg_ && launch_solve_pipe(L, B, beg, end, friction, pdl)) return;
-            if (variant == kVariantDeep) launch_solve_reg<false, true>(L, B, beg, end, friction, probe, pdl, false);
-            else launch_solve_reg<false, false>(L, B, beg, end, friction, probe, pdl, variant == kVariantPrefetch);
+            launch_solve(L, B, beg, mid, color, flags, pdl, variant);
+            launch_solve_wide<false>(B, mid, end, color, flags, nullptr, use_pdl_);
         }
     }
 
@@ -1126,8 +1219,7 @@ public:
             const int n = group_end_[g] - group_beg_[g];
             if (n <= 0) continue;
             const ColorCfg& cc = ccfg_[g];
-            launch_solve<false>(cc.L, cc.B, group_beg_[g], group_end_[g], flags, nullptr, use_pdl_ && after_solve,
-                                cc.variant);
+            launch_color(g, cc.L, cc.B, flags, use_pdl_ && after_solve, cc.variant);
             after_solve = true;
         }
         if (accel) {
@@ -1295,10 +1387,10 @@ public:
 
     // Time per launch of one color's solve over `reps` launches in a row, as the sweep's graph
     // chains them (programmatic dependent launch).
-    float time_color(int L, int B, int beg, int end, int variant, int reps) {
-        launch_solve<false>(L, B, beg, end, 1, nullptr, false, variant);  // warm-up
+    float time_color(size_t g, int L, int B, int variant, int reps) {
+        launch_color(g, L, B, dev::kSolveFriction, false, variant);  // warm-up
         GAIA_CUDA(cudaEventRecord(ev_a_, st_));
-        for (int r = 0; r < reps; ++r) launch_solve<false>(L, B, beg, end, 1, nullptr, use_pdl_, variant);
+        for (int r = 0; r < reps; ++r) launch_color(g, L, B, dev::kSolveFriction, use_pdl_, variant);
         GAIA_CUDA(cudaEventRecord(ev_b_, st_));
         GAIA_CUDA(cudaEventSynchronize(ev_b_));
         float ms = 0.f;
@@ -1358,7 +1450,7 @@ public:
                     for (int B : Bs) {
                         if (block_ && B != block_) continue;
                         if (chain && !block_ && B != 128) continue;
-                        const float ms = time_color(L, B, beg, end, var, reps);
+                        const float ms = time_color(g, L, B, var, reps);
                         if (ms < best.ms) best = ColorCfg{L, B, var, ms};
                         tried.push_back(ColorCfg{L, B, var, ms});
                     }
@@ -1372,7 +1464,7 @@ public:
                 best.ms = 1e30f;
                 for (ColorCfg& t : tried) t.ms = 1e30f;
                 for (int round = 0; round < 3; ++round)
-                    for (ColorCfg& t : tried) t.ms = std::min(t.ms, time_color(t.L, t.B, beg, end, t.variant, 2 * reps));
+                    for (ColorCfg& t : tried) t.ms = std::min(t.ms, time_color(g, t.L, t.B, t.variant, 2 * reps));
                 for (const ColorCfg& t : tried)
                     if (t.ms < best.ms) best = t;
             }
@@ -1405,7 +1497,7 @@ public:
         std::vector<int64_t> work(size_t(nmesh_), 0);
         for (int m = 0; m < nmesh_; ++m)
             for (int32_t ci = scene_ofs_[m]; ci < scene_ofs_[m + 1]; ++ci)
-                work[size_t(m)] += inc_ofs_[scene_colors_[ci].y] - inc_ofs_[scene_colors_[ci].x];
+                work[size_t(m)] += inc_ofs_[scene_colors_[ci].z] - inc_ofs_[scene_colors_[ci].x];
         std::vector<int32_t> order;
         for (int m = 0; m < nmesh_; ++m)
             if (scene_ofs_[m + 1] > scene_ofs_[m]) order.push_back(m);
@@ -1423,34 +1515,29 @@ public:
         GAIA_CUDA(cudaStreamSynchronize(st_));
     }
 
-    template <int L, int MAXB, bool MULTI>
+    template <int L, int MAXB, bool LONG>
     void launch_scenes_lb(int B) {
-        auto kern = dev::k_sweep_scenes<L, MULTI, ST, R, MAXB>;
-        const int cap = max_nbr_all_;
-        const size_t smem = stage_bytes(cap, L, B);
+        auto kern = dev::k_sweep_scenes<L, LONG, ST, R, MAXB>;
+        const size_t smem = sweep_stage_bytes(L, B);
         allow_smem(kern, smem);
         const int per_sm = blocks_per_sm(kern, B, smem);
         const int grid = std::max(1, std::min(nscenes_, std::max(per_sm, 1) * num_sms_));
         kern<<<grid, B, smem, st_>>>(ptrs(), c_, d_scene_colors_.p, d_scene_ofs_.p, d_scene_order_.p, nscenes_,
-                                     sc_.p.iterations, sc_.p.frictionStartIter, d_scene_work_.p, cap);
+                                     sc_.p.iterations, sc_.p.frictionStartIter, d_scene_work_.p, sweep_stage(L));
         GAIA_CUDA(cudaGetLastError());
     }
 
-    template <int L, bool MULTI = false>
+    template <int L>
     void launch_scenes_l(int B) {
-        if (B <= 256) launch_scenes_lb<L, 256, MULTI>(B);
-        else launch_scenes_lb<L, 1024, MULTI>(B);
+        if (B <= 256) any_long_ ? launch_scenes_lb<L, 256, true>(B) : launch_scenes_lb<L, 256, false>(B);
+        else any_long_ ? launch_scenes_lb<L, 1024, true>(B) : launch_scenes_lb<L, 1024, false>(B);
     }
 
     // One substep's iterations: reset the work counter, one persistent launch.
     void enqueue_scenes_sweep(int L, int B) {
         if (nscenes_ == 0 || sc_.p.iterations == 0) return;
         GAIA_CUDA(cudaMemsetAsync(d_scene_work_.p, 0, sizeof(int32_t), st_));
-        if (multi_seg_) {
-            launch_scenes_l<32, true>(B);
-            return;
-        }
-        switch (fit_lanes(L, B, 0, nactive_)) {
+        switch (fit_sweep_lanes(L, B)) {
             case 2: launch_scenes_l<2>(B); break;
             case 4: launch_scenes_l<4>(B); break;
             case 8: launch_scenes_l<8>(B); break;
@@ -1505,7 +1592,7 @@ public:
             int32_t a0 = 0, a1 = 0;
             if (scene_ofs_[m + 1] > scene_ofs_[m]) {
                 a0 = scene_colors_[scene_ofs_[m]].x;
-                a1 = scene_colors_[scene_ofs_[m + 1] - 1].y;
+                a1 = scene_colors_[scene_ofs_[m + 1] - 1].z;
             }
             int64_t nf = 0;
             for (int v = 0; v < sc_.meshes[m].nv; ++v) nf += sc_.meshes[m].fixed[v] ? 1 : 0;
@@ -1529,9 +1616,11 @@ public:
                 for (int r = 0; r < C; ++r) {
                     int64_t nbr = 0, inc = 0;
                     for (int32_t ci = scene_ofs_[m]; ci < scene_ofs_[m + 1]; ++ci) {
-                        const int4 q = rg[size_t(ci) * C + r];
-                        nbr += int64_t(dev::kSlice) * (q.y - q.x);
-                        inc += int64_t(dev::kSlice) * (q.w - q.z);
+                        for (int kind = 0; kind < 2; ++kind) {
+                            const int4 q = rg[2 * (size_t(ci) * C + r) + kind];
+                            nbr += int64_t(dev::kSlice) * (q.y - q.x);
+                            inc += int64_t(dev::kSlice) * (q.w - q.z);
+                        }
                     }
                     nbr_cap = std::max(nbr_cap, nbr);
                     inc_cap = std::max(inc_cap, inc);
@@ -1540,7 +1629,7 @@ public:
             nbr_cap = (nbr_cap + 1) & ~int64_t(1);
             inc_cap = (inc_cap + 1) & ~int64_t(1);
             // states, rest positions and records; the staging areas come on top (per lanes and block)
-            const size_t min_stage = stage_bytes(max_nbr_all_, 32, 64);
+            const size_t min_stage = sweep_stage_bytes(32, kMinBlock);
             const size_t lean = sizeof(S4) * size_t(pos_cap);
             const size_t bytes = lean + sizeof(float4) * size_t(pos_cap) + sizeof(dev::NbrRec<R>) * size_t(nbr_cap) +
                                  sizeof(dev::IncRec<R>) * size_t(inc_cap);
@@ -1573,17 +1662,17 @@ public:
     }
 
     // Incidences of the fullest block of a cluster of C blocks when each color's vertices are
-    // dealt out evenly.
+    // dealt out evenly, in the order of the color.
     int64_t cluster_incidences(int C) const {
         int64_t most = 0;
         for (int m = 0; m < nmesh_; ++m) {
             std::vector<int64_t> per_rank(size_t(C), 0);
             for (int32_t ci = scene_ofs_[m]; ci < scene_ofs_[m + 1]; ++ci) {
-                const int2 rg = scene_colors_[ci];
-                const int per = (rg.y - rg.x + C - 1) / C;
+                const int4 rg = scene_colors_[ci];
+                const int per = (rg.z - rg.x + C - 1) / C;
                 for (int r = 0; r < C; ++r) {
-                    const int beg = std::min(rg.y, rg.x + r * per), end = std::min(rg.y, beg + per);
-                    per_rank[size_t(r)] += inc_ofs_[end] - inc_ofs_[beg];
+                    const int beg = std::min(rg.z, rg.x + r * per), end = std::min(rg.z, beg + per);
+                    per_rank[size_t(r)] += deal_ofs_[size_t(end)] - deal_ofs_[size_t(beg)];
                 }
             }
             for (int64_t x : per_rank) most = std::max(most, x);
@@ -1591,22 +1680,24 @@ public:
         return most;
     }
 
-    // Record rows of every color's chunk of every rank in a cluster of C blocks (C per color): the
-    // chunks are whole slices, so a chunk's rows end where the next slice's begin.
+    // Record rows of every color's chunks (short and long lists) of every rank in a cluster of C
+    // blocks (2 C per color): the chunks are whole slices, so a chunk's rows end where the next
+    // slice's begin.
     std::vector<int4> cluster_ranges(int C) const {
         std::vector<int4> out;
         auto at = [&](int v) {
             if (v >= nactive_) return make_int2(nbr_end_, inc_end_);
             return make_int2(vrec_[size_t(v)].x, vrec_[size_t(v)].y);
         };
-        for (const int2 c : scene_colors_) {
-            const int per = dev::cluster_chunk(c.y - c.x, C);
-            for (int r = 0; r < C; ++r) {
-                const int beg = std::min(c.y, c.x + r * per), end = std::min(c.y, beg + per);
-                const int2 a = at(beg), b = at(end);
-                out.push_back(beg < end ? make_int4(a.x, b.x, a.y, b.y) : make_int4(0, 0, 0, 0));
-            }
-        }
+        for (const int4 c : scene_colors_)
+            for (int r = 0; r < C; ++r)
+                for (int kind = 0; kind < 2; ++kind) {
+                    const int lo = kind ? c.y : c.x, hi = kind ? c.z : c.y;
+                    const int per = dev::cluster_chunk(hi - lo, C);
+                    const int beg = std::min(hi, lo + r * per), end = std::min(hi, beg + per);
+                    const int2 a = at(beg), b = at(end);
+                    out.push_back(beg < end ? make_int4(a.x, b.x, a.y, b.y) : make_int4(0, 0, 0, 0));
+                }
         return out;
     }
 
@@ -1616,11 +1707,15 @@ public:
         return nullptr;
     }
 
-    template <int L, bool MULTI = false, bool LEAN = false>
+    template <int L, bool LEAN = false>
     void launch_cluster_l(const ClusterFit& f, int B) {
-        auto kern = dev::k_sweep_cluster<L, MULTI, LEAN, ST, R>;
-        const int cap = max_nbr_all_;
-        const size_t smem = f.bytes + stage_bytes(cap, L, B);
+        if (any_long_) launch_cluster_k<L, true, LEAN>(f, B);
+        else launch_cluster_k<L, false, LEAN>(f, B);
+    }
+    template <int L, bool LONG, bool LEAN>
+    void launch_cluster_k(const ClusterFit& f, int B) {
+        auto kern = dev::k_sweep_cluster<L, LONG, LEAN, ST, R>;
+        const size_t smem = f.bytes + sweep_stage_bytes(L, B);
         GAIA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cluster_budget_)));
         if (f.C > 8) GAIA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t cfg = {};
@@ -1650,7 +1745,7 @@ public:
         S.pos_cap = f.pos_cap;
         S.nbr_cap = f.nbr_cap;
         S.inc_cap = f.inc_cap;
-        S.stage_cap = cap;
+        S.stage = sweep_stage(L);
         S.ranges = cluster_range_bufs_.at(f.C)->p;
         GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, S, d_scene_work_.p));
     }
@@ -1661,16 +1756,11 @@ public:
         if (!f) throw std::runtime_error("clusterSize: scenes do not fit a cluster of " + std::to_string(C) + " blocks");
         GAIA_CUDA(cudaMemsetAsync(d_scene_work_.p, 0, sizeof(int32_t), st_));
         // more lanes per vertex, then fewer threads, where the staging areas do not fit beside the scene
-        auto fits = [&](int l) { return f->bytes + stage_bytes(max_nbr_all_, l, B) <= cluster_budget_; };
+        auto fits = [&](int l) { return f->bytes + sweep_stage_bytes(l, B) <= cluster_budget_; };
         if (f->lean) L = 32;
         while (L < 32 && !fits(L)) L *= 2;
         while (B > kMinBlock && !fits(L)) B = smaller_block(B);
         if (f->lean) {
-            if (multi_seg_) launch_cluster_l<32, true, true>(*f, B);
-            else launch_cluster_l<32, false, true>(*f, B);
-            return;
-        }
-        if (multi_seg_) {
             launch_cluster_l<32, true>(*f, B);
             return;
         }
@@ -1737,12 +1827,16 @@ public:
 
     // ---- grid sweep (vbd_grid.cuh) -----------------------------------------------------
     void setup_grid() {
-        std::vector<int2> colors;
+        std::vector<int4> colors;
         for (size_t g = 0; g < group_beg_.size(); ++g)
-            if (group_end_[g] > group_beg_[g]) colors.push_back(make_int2(group_beg_[g], group_end_[g]));
+            if (group_end_[g] > group_beg_[g]) colors.push_back(make_int4(group_beg_[g], group_mid_[g], group_end_[g], 0));
         grid_ncolors_ = int32_t(colors.size());
         grid_max_color_ = 0;
-        for (const int2& c : colors) grid_max_color_ = std::max(grid_max_color_, c.y - c.x);
+        grid_max_long_ = 0;
+        for (const int4& c : colors) {
+            grid_max_color_ = std::max(grid_max_color_, c.y - c.x);
+            grid_max_long_ = std::max(grid_max_long_, c.z - c.y);
+        }
         d_grid_colors_.upload(colors, &bytes_, st_);
         d_grid_bar_.alloc(2, &bytes_);
         int dev = 0, coop = 0;
@@ -1755,16 +1849,21 @@ public:
 
     // Blocks of the grid sweep: enough for the largest color at one vertex per group, at most
     // as many as are resident at once (the cooperative launch requires it).
-    template <int L, bool MULTI>
+    template <int L, bool LONG>
     int grid_blocks(int B, size_t smem) {
-        const int per_sm = blocks_per_sm(dev::k_sweep_grid<L, MULTI, ST, R>, B, smem);
+        const int per_sm = blocks_per_sm(dev::k_sweep_grid<L, LONG, ST, R>, B, smem);
         if (per_sm < 1) throw std::runtime_error("grid sweep: no block of this size fits on an SM");
-        const int need = std::max(1, int(div_up(int64_t(grid_max_color_) * L, B)));
+        const int need = std::max(1, int(div_up(std::max(int64_t(grid_max_color_) * L, int64_t(grid_max_long_) * 32), B)));
         return std::min(need, per_sm * num_sms_);
     }
 
-    template <int L, bool MULTI = false>
+    template <int L>
     void launch_grid_l(int B) {
+        if (any_long_) launch_grid_k<L, true>(B);
+        else launch_grid_k<L, false>(B);
+    }
+    template <int L, bool LONG>
+    void launch_grid_k(int B) {
         dev::GridSweep G;
         G.colors = d_grid_colors_.p;
         G.ncolors = grid_ncolors_;
@@ -1777,25 +1876,20 @@ public:
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const int cap = max_nbr_all_;
-        const size_t smem = stage_bytes(cap, L, B);
-        allow_smem(dev::k_sweep_grid<L, MULTI, ST, R>, smem);
-        cfg.gridDim = dim3(unsigned(grid_blocks<L, MULTI>(B, smem)));
+        const size_t smem = sweep_stage_bytes(L, B);
+        allow_smem(dev::k_sweep_grid<L, LONG, ST, R>, smem);
+        cfg.gridDim = dim3(unsigned(grid_blocks<L, LONG>(B, smem)));
         cfg.blockDim = dim3(unsigned(B));
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st_;
-        GAIA_CUDA(cudaLaunchKernelEx(&cfg, dev::k_sweep_grid<L, MULTI, ST, R>, ptrs(), c_, G, cap));
+        GAIA_CUDA(cudaLaunchKernelEx(&cfg, dev::k_sweep_grid<L, LONG, ST, R>, ptrs(), c_, G, sweep_stage(L)));
     }
 
     // One substep's iterations: the barrier's counter and flag zeroed, one cooperative launch.
     void enqueue_grid_sweep(int L, int B) {
         if (grid_ncolors_ == 0 || sc_.p.iterations == 0) return;
         GAIA_CUDA(cudaMemsetAsync(d_grid_bar_.p, 0, 2 * sizeof(uint32_t), st_));
-        if (multi_seg_) {
-            launch_grid_l<32, true>(B);
-            return;
-        }
-        switch (fit_lanes(L, B, 0, nactive_)) {
+        switch (fit_sweep_lanes(L, B)) {
             case 2: launch_grid_l<2>(B); break;
             case 4: launch_grid_l<4>(B); break;
             case 8: launch_grid_l<8>(B); break;
@@ -2228,7 +2322,10 @@ public:
         int32_t s = slot_of_[off + v];
         if (s >= nactive_) throw std::invalid_argument("vertex is fixed (not solved)");
         if (cd_.enabled()) enqueue_contact_snapshot(0);
-        launch_solve<true>(lanes_, block_, s, s + 1, friction ? dev::kSolveFriction : 0, d_probe_.p);
+        const int flags = friction ? dev::kSolveFriction : 0;
+        const int2 own = make_int2(s, s + 1);
+        if (long_slot(s)) launch_solve_wide<true>(block_, s, s + 1, own, flags, d_probe_.p, false);
+        else launch_solve_reg<true, false>(lanes_, block_, s, s + 1, own, flags, d_probe_.p, false, false);
         double h[12];
         GAIA_CUDA(cudaMemcpyAsync(h, d_probe_.p, sizeof(h), cudaMemcpyDeviceToHost, st_));
         GAIA_CUDA(cudaStreamSynchronize(st_));
@@ -2288,18 +2385,19 @@ private:
                                // prefetch of the next wave's records, 7 = k_solve_pipe
     int mode_ = 0;             // kSweepMerged, kSweepScenes, kSweepCluster or kSweepGrid
     // scene-major mode: per mesh its color slot ranges, in sweep order
-    std::vector<int2> scene_colors_;
+    std::vector<int64_t> deal_ofs_;   // incidences before each vertex, in the order of the colors
+    std::vector<int4> scene_colors_;  // first slot, first of the long lists, end
     std::vector<int32_t> scene_ofs_;
     int32_t nscenes_ = 0;
     int scene_L_ = 8, scene_B_ = 512, scene_C_ = 8, num_sms_ = 1;
-    DevBuf<int2> d_scene_colors_;
+    DevBuf<int4> d_scene_colors_;
     DevBuf<int32_t> d_scene_ofs_, d_scene_order_, d_scene_work_;
     std::vector<ClusterFit> cluster_fits_;
     size_t cluster_budget_ = 0;  // dynamic shared memory of a cluster's block
     std::map<int, std::unique_ptr<DevBuf<int4>>> cluster_range_bufs_;
     DevBuf<int4> d_scene_slots_;
     // grid mode: the merged colors' slot ranges, the barrier's counter and abort flag
-    DevBuf<int2> d_grid_colors_;
+    DevBuf<int4> d_grid_colors_;
     // mesh frames: per mesh the reference slot, the FP64 offset, this substep's shift, the planes
     bool frames_ = false;
     DevBuf<int32_t> d_frame_ref_;
@@ -2307,7 +2405,7 @@ private:
     DevBuf<float4> d_frame_shift_;
     DevBuf<float4> d_rest_fh_, d_rest_fl_;
     DevBuf<uint32_t> d_grid_bar_;
-    int32_t grid_ncolors_ = 0, grid_max_color_ = 0;
+    int32_t grid_ncolors_ = 0, grid_max_color_ = 0, grid_max_long_ = 0;
     int variant_fixed_ = -1;   // from PhysicsParams solveVariant (-1 = autotune)
     std::map<std::pair<int, int>, int2> maxrec_cache_;
     std::map<std::tuple<const void*, int, size_t>, int> occ_cache_;  // (kernel, block, shared bytes) -> blocks per SM
@@ -2321,14 +2419,16 @@ private:
     size_t bytes_ = 0;
     dev::Consts<R> c_{};
     std::vector<int64_t> mesh_off_;
-    std::vector<int32_t> slot_of_, orig_of_, slot_mesh_, inc_ofs_, group_beg_, group_end_;
+    std::vector<int32_t> slot_of_, orig_of_, slot_mesh_, inc_ofs_, group_beg_, group_mid_, group_end_;
+    std::vector<std::vector<uint8_t>> long_;  // per mesh (empty: none) its vertices with long lists
+    bool any_long_ = false;
     // one-ring and incidence records
     std::vector<dev::NbrRec<R>> h_nbr_;
     std::vector<dev::IncRec<R>> h_inc_;
     std::vector<int4> vrec_, segs_;
     std::vector<int2> vmore_;
     bool multi_seg_ = false;  // some vertex has more than kSegNbrs neighbours
-    int max_nbr_all_ = 2, max_inc_all_ = 1, nbr_end_ = 0, inc_end_ = 0;
+    int max_nbr_all_ = 2, max_nbr_short_ = 2, max_inc_all_ = 1, nbr_end_ = 0, inc_end_ = 0;
     std::map<std::pair<int, int>, int2> lists_cache_;
     std::vector<S4> h_pos_;
     std::vector<V4> h_vel_;

@@ -26,7 +26,7 @@ namespace gaia {
 namespace dev {
 
 struct GridSweep {
-    const int2* colors;  // slot ranges of the merged colors, in sweep order
+    const int4* colors;  // slot ranges of the merged colors, in sweep order (first, first long list, end)
     int32_t ncolors, iterations, friction_start;
     uint32_t* bar;       // [0] arrivals (monotonic within a launch), [1] abort flag; zeroed before each launch
 };
@@ -63,27 +63,22 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t target, int
     return s_ok != 0;
 }
 
-template <int L, bool MULTI, typename ST, typename R>
-__global__ void __launch_bounds__(256) k_sweep_grid(Ptrs<ST, R> P, Consts<R> c, GridSweep G, int cap) {
-    using U = typename ST::U;
+template <int L, bool LONG, typename ST, typename R>
+__global__ void __launch_bounds__(256) k_sweep_grid(Ptrs<ST, R> P, Consts<R> c, GridSweep G, SweepStage S) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int per_block = int(blockDim.x) / L;
-    const int ngroups = int(gridDim.x) * per_block;
-    const int gid = int(blockIdx.x) * per_block + int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
-    const int sub = Lanes<L>::sub();
+    const int per_block = int(blockDim.x >> 5);
+    const int warps = int(gridDim.x) * per_block;
+    const int w = int(blockIdx.x) * per_block + int(threadIdx.x >> 5);
     const FetchGlobal<ST, kStateGrid> fetch{P.u, P.rest};
     uint32_t target = 0;
     for (int it = 0; it < G.iterations; ++it) {
         const int friction = it >= G.friction_start ? 1 : 0;
         for (int ci = 0; ci < G.ncolors; ++ci) {
-            const int2 rg = G.colors[ci];
-            for (int base = rg.x; base < rg.y; base += ngroups) {
-                const int v = base + gid;
-                const bool valid = v < rg.y;
-                U uo{};
-                if (valid) uo = ST::ldcg_own(P.u, v);
-                solve_in_sweep<L, MULTI, ST, R>(P, c, v, valid, sub, smem, cap, fetch, uo, friction);
-            }
+            const int4 rg = G.colors[ci];
+            sweep_range<L, false, true, ST, R>(P, c, rg.x, rg.y, w, warps, smem, S.cap, S.warp_bytes, fetch, friction);
+            if constexpr (LONG)
+                sweep_range<32, true, true, ST, R>(P, c, rg.y, rg.z, w, warps, smem, S.cap_long, S.warp_bytes, fetch,
+                                                   friction);
             if (it + 1 == G.iterations && ci + 1 == G.ncolors) break;  // the kernel's end orders the last color
             target += gridDim.x;
             if (!grid_barrier(G.bar, target, c.spin_limit, P.counters)) return;

@@ -378,12 +378,16 @@ struct Stage {
     }
 };
 
-// The staging area of this lane's vertex: the warps' areas follow each other, `cap` entries per
-// vertex.
+// The staging area of this lane's vertex: the warps' areas (warp_bytes each) follow each other,
+// `cap` entries per vertex.
+template <int L, typename ST, typename R>
+__device__ __forceinline__ Stage<32 / L, ST, R> warp_stage(unsigned char* smem, int cap, size_t warp_bytes) {
+    using S = Stage<32 / L, ST, R>;
+    return S(smem + size_t(threadIdx.x >> 5) * warp_bytes, cap, Lanes<L>::vertex());
+}
 template <int L, typename ST, typename R>
 __device__ __forceinline__ Stage<32 / L, ST, R> warp_stage(unsigned char* smem, int cap) {
-    using S = Stage<32 / L, ST, R>;
-    return S(smem + size_t(threadIdx.x >> 5) * size_t(cap * (32 / L)) * (16 * S::kParts), cap, Lanes<L>::vertex());
+    return warp_stage<L, ST, R>(smem, cap, size_t(cap * (32 / L)) * (16 * Stage<32 / L, ST, R>::kParts));
 }
 
 // k + l += x y: l takes the rounding errors of product and sum (two-sum of k and fl(x y), the
@@ -566,7 +570,7 @@ __device__ __forceinline__ void accumulate_segment(SegRecs<R, NB>& s, int sub, c
 }
 
 // The remaining segments of a vertex with more than kSegNbrs neighbours. Only the 32-lane
-// kernels of scenes with such a vertex (MULTI) hold this loop: it costs registers.
+// solves of the long lists (MULTI) hold this loop: it costs registers.
 template <int L, int RR, bool ASYNC, typename ST, typename R, int NB, typename Fetch>
 __device__ __forceinline__ void accumulate_more(SegRecs<R, NB>& rec, const Ptrs<ST, R>& P, const NbrRec<R>* nbr,
                                                 const IncRec<R>* inc, int2 more, int sub, const Stage<32 / L, ST, R>& st,
@@ -934,12 +938,13 @@ struct SolveOcc {
     static constexpr int kMinBlocks = sizeof(R) == 8 || L >= 16 ? 2 : 4;
 };
 
-// DEEP (variant 4): asynchronous one-ring copies (narrow groups). MULTI: a scene with a vertex
-// of several segments. pf > 0: prefetch distance in warps.
-// max_nbr: the longest neighbour list of the color, the staging entries per vertex.
+// [beg, end): the color or the part of it that this launch solves; color: all of it.
+// DEEP (variant 4): asynchronous one-ring copies (narrow groups). MULTI: vertices of several
+// segments among them. pf > 0: prefetch distance in warps.
+// max_nbr: the longest neighbour list of the launch, the staging entries per vertex.
 template <int L, typename ST, typename R, bool PROBE, bool DEEP, bool MULTI, bool CONTACT>
 __global__ void __launch_bounds__(256, SolveOcc<L, R>::kMinBlocks)
-    k_solve(Ptrs<ST, R> P, Consts<R> c, int beg, int end, int flags, double* probe_out, int pf, int max_nbr) {
+    k_solve(Ptrs<ST, R> P, Consts<R> c, int beg, int end, int2 color, int flags, double* probe_out, int pf, int max_nbr) {
     using U = typename ST::U;
     constexpr bool kAsync = DEEP && L < 16;
     constexpr int NB = NbrBatch<L, kAsync>::kN;
@@ -989,7 +994,7 @@ __global__ void __launch_bounds__(256, SolveOcc<L, R>::kMinBlocks)
     reduce_group<L, R>(acc);
     if constexpr (L < 16)
         if (valid && sub == 0) Fo = frame_offset(P, v);
-    finish_vertex<L, PROBE, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, beg, end, flags, probe_out);
+    finish_vertex<L, PROBE, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, color.x, color.y, flags, probe_out);
 }
 
 // ---- per-vertex tail (lane 0 of a vertex group): damping, inertia, ground and
@@ -1137,7 +1142,7 @@ __device__ __forceinline__ void finish_vertex(const Ptrs<ST, R>& P, const Consts
 // flight at once, overlapping the previous color's tail, at no register cost.
 // Neighbour positions are gathered as in k_solve. tile_nbr and tile_inc bound the
 // records of any block of this launch (the host sizes the dynamic shared memory
-// from them). Scenes without a vertex of several segments only.
+// from them). Vertices of one segment only.
 // ---------------------------------------------------------------------------
 constexpr int kMbarSpinLimit = 1 << 20;
 // Polls of the final drain wait of a block whose first wait ran out, each after a 1 us
@@ -1198,7 +1203,7 @@ __device__ __forceinline__ void issue_tile(const Ptrs<ST, float>& P, const RecTi
 
 template <int L, bool CONTACT, typename ST>
 __global__ void __launch_bounds__(256, 4)
-    k_solve_tma(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int flags, int max_nbr, int max_inc,
+    k_solve_tma(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int2 color, int flags, int max_nbr, int max_inc,
                 int tile_nbr, int tile_inc) {
     using U = typename ST::U;
     constexpr int NB = NbrBatch<L, false>::kN;
@@ -1260,7 +1265,7 @@ __global__ void __launch_bounds__(256, 4)
     accumulate_segment<L, kRecShared, false, ST>(rec, sub, st, FetchGlobal<ST, kStatePlain>{P.u, P.rest}, uon, Xo, mat.mu, mat.lmbd, acc);
     reduce_group<L, float>(acc);
     const float3 Fo = valid && sub == 0 ? frame_offset(P, v) : make_float3(0.f, 0.f, 0.f);
-    finish_vertex<L, false, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, beg, end, flags, nullptr);
+    finish_vertex<L, false, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, color.x, color.y, flags, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1272,11 +1277,11 @@ __global__ void __launch_bounds__(256, 4)
 // color is in flight ahead of the warps without occupying their registers. Bounded waits as
 // in k_solve_tma: a block whose wait runs out counts a timeout, drains every copy it issued
 // and returns. tile_nbr and tile_inc bound the records of any tile (the host sizes the buffers
-// from them). Scenes without a vertex of several segments only.
+// from them). Vertices of one segment only.
 // ---------------------------------------------------------------------------
 template <int L, bool CONTACT, typename ST>
 __global__ void __launch_bounds__(256)
-    k_solve_pipe(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int flags, int max_nbr, int max_inc,
+    k_solve_pipe(Ptrs<ST, float> P, Consts<float> c, int beg, int end, int2 color, int flags, int max_nbr, int max_inc,
                  int tile_nbr, int tile_inc) {
     using U = typename ST::U;
     constexpr int NB = NbrBatch<L, false>::kN;
@@ -1349,7 +1354,7 @@ __global__ void __launch_bounds__(256)
         accumulate_segment<L, kRecShared, false, ST>(rec, sub, st, FetchGlobal<ST, kStatePlain>{P.u, P.rest}, uon, Xo, mat.mu, mat.lmbd, acc);
         reduce_group<L, float>(acc);
         const float3 Fo = valid && sub == 0 ? frame_offset(P, v) : make_float3(0.f, 0.f, 0.f);
-        finish_vertex<L, false, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, beg, end, flags, nullptr);
+        finish_vertex<L, false, CONTACT>(P, c, v, valid, sub, uo, Xo, Fo, mat, acc, info, color.x, color.y, flags, nullptr);
         __syncthreads();  // every read of buffer b done before the next iteration refills it
     }
 }
@@ -1373,7 +1378,7 @@ __global__ void __launch_bounds__(256)
 // neighbours per vertex.
 template <int L, bool MULTI, typename ST, typename R, typename Fetch>
 __device__ __forceinline__ void solve_in_sweep(const Ptrs<ST, R>& P, const Consts<R>& c, int v, bool valid, int sub,
-                                               unsigned char* smem, int cap, const Fetch& fetch,
+                                               unsigned char* smem, int cap, int warp_bytes, const Fetch& fetch,
                                                const typename ST::U& uo, int friction) {
     using U = typename ST::U;
     constexpr bool kAsync = L < 16;
@@ -1388,7 +1393,7 @@ __device__ __forceinline__ void solve_in_sweep(const Ptrs<ST, R>& P, const Const
         mat = P.mats[P.slot_mesh[v]];
     }
     SegRecs<R, NB> rec;
-    const Stage<32 / L, ST, R> st = warp_stage<L, ST, R>(smem, cap);
+    const Stage<32 / L, ST, R> st = warp_stage<L, ST, R>(smem, cap, size_t(warp_bytes));
     preload<L, kRecKept>(rec, P.nbr, P.inc, seg, sub);
     if (valid && sub == 0) prefetch_tail<L>(P, v);
     const U uon = ST::nb(uo);
@@ -1404,17 +1409,36 @@ __device__ __forceinline__ void solve_in_sweep(const Ptrs<ST, R>& P, const Const
     }
 }
 
-template <int L, bool MULTI, typename ST, typename R, int MAXB>
-__global__ void __launch_bounds__(MAXB) k_sweep_scenes(Ptrs<ST, R> P, Consts<R> c, const int2* colors,
+// The staging areas of a persistent sweep: entries per vertex of the short lists (L lanes per
+// vertex) and of the long ones (a warp per vertex), and the bytes per warp that hold either.
+struct SweepStage {
+    int32_t cap, cap_long, warp_bytes;
+};
+
+// The vertices [beg, end) of one color in turn over `warps` warps, this one being number `w`.
+template <int L, bool MULTI, bool GRID, typename ST, typename R, typename Fetch>
+__device__ __forceinline__ void sweep_range(const Ptrs<ST, R>& P, const Consts<R>& c, int beg, int end, int w, int warps,
+                                            unsigned char* smem, int cap, int warp_bytes, const Fetch& fetch,
+                                            int friction) {
+    const int g = w * Lanes<L>::kW + Lanes<L>::vertex();
+    for (int base = beg; base < end; base += warps * Lanes<L>::kW) {
+        const int v = base + g;
+        const bool valid = v < end;
+        typename ST::U uo{};
+        if (valid) uo = GRID ? ST::ldcg_own(P.u, v) : ST::ld_own(P.u, v);
+        solve_in_sweep<L, MULTI, ST, R>(P, c, v, valid, Lanes<L>::sub(), smem, cap, warp_bytes, fetch, uo, friction);
+    }
+}
+
+// colors: (first slot, first slot of the vertices with long lists, end). LONG: there are such.
+template <int L, bool LONG, typename ST, typename R, int MAXB>
+__global__ void __launch_bounds__(MAXB) k_sweep_scenes(Ptrs<ST, R> P, Consts<R> c, const int4* colors,
                                                        const int32_t* scene_ofs, const int32_t* scene_order,
                                                        int32_t nscenes, int32_t iterations, int32_t friction_start,
-                                                       int32_t* work, int cap) {
-    using U = typename ST::U;
+                                                       int32_t* work, SweepStage S) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_scene;
-    const int groups = int(blockDim.x) / L;
-    const int g = int(threadIdx.x >> 5) * Lanes<L>::kW + Lanes<L>::vertex();
-    const int sub = Lanes<L>::sub();
+    const int w = int(threadIdx.x >> 5), warps = int(blockDim.x >> 5);
     const FetchGlobal<ST, kStatePlain> fetch{P.u, P.rest};
     for (;;) {
         if (threadIdx.x == 0) s_scene = atomicAdd(work, 1);
@@ -1427,14 +1451,11 @@ __global__ void __launch_bounds__(MAXB) k_sweep_scenes(Ptrs<ST, R> P, Consts<R> 
         for (int it = 0; it < iterations; ++it) {
             const int friction = it >= friction_start ? 1 : 0;
             for (int ci = c0; ci < c1; ++ci) {
-                const int2 rg = colors[ci];
-                for (int base = rg.x; base < rg.y; base += groups) {
-                    const int v = base + g;
-                    const bool valid = v < rg.y;
-                    U uo{};
-                    if (valid) uo = ST::ld_own(P.u, v);
-                    solve_in_sweep<L, MULTI, ST, R>(P, c, v, valid, sub, smem, cap, fetch, uo, friction);
-                }
+                const int4 rg = colors[ci];
+                sweep_range<L, false, false, ST, R>(P, c, rg.x, rg.y, w, warps, smem, S.cap, S.warp_bytes, fetch, friction);
+                if constexpr (LONG)
+                    sweep_range<32, true, false, ST, R>(P, c, rg.y, rg.z, w, warps, smem, S.cap_long, S.warp_bytes, fetch,
+                                                        friction);
                 __syncthreads();  // this color's updates before the next color reads them
             }
         }
