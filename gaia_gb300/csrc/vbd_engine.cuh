@@ -164,8 +164,8 @@ public:
         variant_fixed_ = sc_.p.solveVariant;
         if (variant_fixed_ != -1 && variant_fixed_ != 0 && variant_fixed_ != 1 && variant_fixed_ != kVariantDeep &&
             variant_fixed_ != kVariantPrefetch && variant_fixed_ != kVariantPipe)
-            throw std::runtime_error("solveVariant must be -1 (autotune), 0 (registers), 1 (TMA-staged), 4 (registers, "
-                                     "deeper record pipeline), 6 (registers, next wave's records prefetched into L2) or "
+            throw std::runtime_error("solveVariant must be -1 (autotune), 0 (registers), 1 (TMA-staged), 4 (one-ring "
+                                     "copied asynchronously), 6 (registers, next wave's data prefetched into L2) or "
                                      "7 (double-buffered TMA tiles on a persistent grid)");
         // the FP64 engine has neither the TMA variants nor the record prefetch
         if ((variant_fixed_ == 1 || variant_fixed_ == kVariantPrefetch || variant_fixed_ == kVariantPipe) &&
@@ -298,7 +298,6 @@ public:
             dev::MeshMat<R> mm{};
             mm.mu = R(o.miu);
             mm.lmbd = R(o.lmbd);
-            mm.a = R(1.0 + o.miu / o.lmbd);
             mm.kh = R(o.dampingHydrostatic);
             mm.kd = R(o.dampingDeviatoric);
             mm.exp_damp = R(std::pow(o.exponentialVelDamping, sc_.p.dt));  // VBDPhysics.cpp:794-807
@@ -1027,6 +1026,12 @@ public:
         return m;
     }
 
+    // Shared memory of the TMA variants: `buffers` record tiles beside the staging areas.
+    size_t tma_bytes(int L, int B, int beg, int end, int buffers) {
+        const int2 mr = max_records(beg, end, B / L);
+        return 16 + 8 * size_t(buffers) * (size_t(mr.x) + size_t(mr.y)) + stage_bytes(max_lists(beg, end).x, L, B);
+    }
+
     template <int L>
     bool launch_solve_tma_l(int B, int beg, int end, int2 color, int flags, bool pdl) {
         if constexpr (sizeof(R) != 4) {
@@ -1035,7 +1040,7 @@ public:
             const int vpb = B / L;
             const int2 mr = max_records(beg, end, vpb);
             const int2 lists = max_lists(beg, end);
-            const size_t smem = 16 + 8 * (size_t(mr.x) + size_t(mr.y)) + stage_bytes(lists.x, L, B);
+            const size_t smem = tma_bytes(L, B, beg, end, 1);
             if (smem > kTmaSmemMax) return false;
             auto kern = cd_.enabled() ? dev::k_solve_tma<L, true, ST> : dev::k_solve_tma<L, false, ST>;
             allow_smem(kern, smem);
@@ -1063,7 +1068,7 @@ public:
             const int vpt = B / L;
             const int2 mr = max_records(beg, end, vpt);
             const int2 lists = max_lists(beg, end);
-            const size_t smem = 16 + 2 * 8 * (size_t(mr.x) + size_t(mr.y)) + stage_bytes(lists.x, L, B);
+            const size_t smem = tma_bytes(L, B, beg, end, 2);
             if (smem > kTmaSmemMax) return false;
             auto kern = cd_.enabled() ? dev::k_solve_pipe<L, true, ST> : dev::k_solve_pipe<L, false, ST>;
             allow_smem(kern, smem);
@@ -1165,8 +1170,26 @@ public:
         ccfg_.assign(group_beg_.size(), ColorCfg{});
         for (size_t g = 0; g < group_beg_.size(); ++g) {
             const int n = group_end_[g] - group_beg_[g];
-            ccfg_[g] = ColorCfg{n <= small_color_ ? 32 : L, B, variant, 0.f};
+            ccfg_[g] = effective(g, ColorCfg{n <= small_color_ ? 32 : L, B, variant, 0.f});
         }
+    }
+
+    // The shape that a configuration of color g runs with: more lanes per vertex, or the register
+    // variant, where its shared memory does not fit a block; a warp per vertex for long lists.
+    ColorCfg effective(size_t g, ColorCfg c) {
+        const int beg = group_beg_[g], mid = group_mid_[g];
+        if (group_end_[g] <= beg) return c;
+        if (mid <= beg) {
+            c.L = 32;
+            c.variant = 0;
+            return c;
+        }
+        if (c.variant == 1 || c.variant == kVariantPipe) {
+            if (sizeof(R) == 4 && tma_bytes(c.L, c.B, beg, mid, c.variant == 1 ? 1 : 2) <= kTmaSmemMax) return c;
+            c.variant = 0;
+        }
+        c.L = fit_lanes(c.L, c.B, beg, mid);
+        return c;
     }
 
     void enqueue_init(bool rebuild) {
@@ -1448,11 +1471,12 @@ public:
                     // 1183 with 8, while the timing here puts 2 lanes first (10.8 against 11.7 us).
                     if (sizeof(R) == 4 && cd_.enabled() && !lanes_ && L == 2) continue;
                     for (int B : Bs) {
-                        if (block_ && B != block_) continue;
                         if (chain && !block_ && B != 128) continue;
+                        const ColorCfg run = effective(g, ColorCfg{L, B, var, 0.f});
+                        if (!lanes_ && run.L != L) continue;  // another candidate runs so
                         const float ms = time_color(g, L, B, var, reps);
-                        if (ms < best.ms) best = ColorCfg{L, B, var, ms};
-                        tried.push_back(ColorCfg{L, B, var, ms});
+                        tried.push_back(ColorCfg{run.L, run.B, run.variant, ms});
+                        if (ms < best.ms) best = tried.back();
                     }
                 }
             }
@@ -1560,6 +1584,7 @@ public:
             if (lanes_ && L != lanes_) continue;
             for (int B : Bs) {
                 if (block_ && B != block_) continue;
+                if (!lanes_ && fit_sweep_lanes(L, B) != L) continue;  // another candidate runs so
                 enqueue_scenes_sweep(L, B);  // warm-up
                 GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
                 GAIA_CUDA(cudaEventRecord(ev_a_, st_));
@@ -1750,16 +1775,21 @@ public:
         GAIA_CUDA(cudaLaunchKernelEx(&cfg, kern, ptrs(), c_, S, d_scene_work_.p));
     }
 
+    // The shape that a cluster sweep of L lanes per vertex and B threads runs with: more lanes, then
+    // fewer threads, where the staging areas do not fit beside the scene.
+    void fit_cluster(const ClusterFit& f, int& L, int& B) const {
+        auto fits = [&](int l) { return f.bytes + sweep_stage_bytes(l, B) <= cluster_budget_; };
+        if (f.lean || L == 2) L = 32;  // (the kernel has no form of two lanes)
+        while (L < 32 && !fits(L)) L *= 2;
+        while (B > kMinBlock && !fits(L)) B = smaller_block(B);
+    }
+
     void enqueue_cluster_sweep(int C, int L, int B) {
         if (nscenes_ == 0 || sc_.p.iterations == 0) return;
         const ClusterFit* f = cluster_fit(C);
         if (!f) throw std::runtime_error("clusterSize: scenes do not fit a cluster of " + std::to_string(C) + " blocks");
         GAIA_CUDA(cudaMemsetAsync(d_scene_work_.p, 0, sizeof(int32_t), st_));
-        // more lanes per vertex, then fewer threads, where the staging areas do not fit beside the scene
-        auto fits = [&](int l) { return f->bytes + sweep_stage_bytes(l, B) <= cluster_budget_; };
-        if (f->lean) L = 32;
-        while (L < 32 && !fits(L)) L *= 2;
-        while (B > kMinBlock && !fits(L)) B = smaller_block(B);
+        fit_cluster(*f, L, B);
         if (f->lean) {
             launch_cluster_l<32, true>(*f, B);
             return;
@@ -1786,6 +1816,9 @@ public:
                 if (lanes_ && L != lanes_) continue;
                 for (int B : {128, 256}) {
                     if (block_ && B != block_) continue;
+                    int l = L, b = B;
+                    fit_cluster(f, l, b);
+                    if ((!lanes_ && l != L) || (!block_ && b != B && b == 128)) continue;  // another candidate runs so
                     enqueue_cluster_sweep(f.C, L, B);  // warm-up
                     GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
                     GAIA_CUDA(cudaEventRecord(ev_a_, st_));
@@ -1819,6 +1852,7 @@ public:
         }
         if (!cluster_fit(scene_C_))
             throw std::runtime_error("clusterSize: scenes do not fit a cluster of " + std::to_string(scene_C_) + " blocks");
+        fit_cluster(*cluster_fit(scene_C_), scene_L_, scene_B_);
         lanes_ = scene_L_;
         block_ = scene_B_;
         variant_ = 3;
@@ -1910,6 +1944,7 @@ public:
             if (lanes_ && L != lanes_) continue;
             for (int B : {128, 256}) {
                 if (block_ && B != block_) continue;
+                if (!lanes_ && fit_sweep_lanes(L, B) != L) continue;  // another candidate runs so
                 enqueue_grid_sweep(L, B);  // warm-up
                 GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
                 GAIA_CUDA(cudaEventRecord(ev_a_, st_));
@@ -1938,6 +1973,7 @@ public:
             scene_L_ = lanes_ ? lanes_ : 16;
             scene_B_ = block_ ? block_ : 256;
         }
+        scene_L_ = fit_sweep_lanes(scene_L_, scene_B_);
         lanes_ = scene_L_;
         block_ = scene_B_;
         variant_ = kVariantGrid;
@@ -1949,6 +1985,7 @@ public:
             scene_L_ = lanes_ ? lanes_ : 8;
             scene_B_ = block_ ? block_ : 512;
         }
+        scene_L_ = fit_sweep_lanes(scene_L_, scene_B_);
         lanes_ = scene_L_;
         block_ = scene_B_;
         variant_ = 2;

@@ -82,8 +82,8 @@ namespace dev {
 
 template <typename R>
 struct MeshMat {
-    R mu, lmbd, a, kh, kd, exp_damp, const_damp, pad;
-    int32_t init_type, pad2, pad3, pad4;
+    R mu, lmbd, kh, kd, exp_damp, const_damp;
+    int32_t init_type, pad;
 };
 
 template <typename R>
@@ -196,8 +196,6 @@ struct DeformVerts {
 // ---------------------------------------------------------------------------
 // small math
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float f_bits(int v) { return __int_as_float(v); }
-
 // Symmetric 3x3 solve by LDL^T (the same algorithm as the oracle's
 // solve3x3_ldlt), with one reciprocal per pivot instead of two divisions (three IEEE
 // divisions instead of six on the vertex's serial path; in FP64 a division is a dozen
