@@ -1658,13 +1658,14 @@ public:
             const size_t lean = sizeof(S4) * size_t(pos_cap);
             const size_t bytes = lean + sizeof(float4) * size_t(pos_cap) + sizeof(dev::NbrRec<R>) * size_t(nbr_cap) +
                                  sizeof(dev::IncRec<R>) * size_t(inc_cap);
-            // an explicit "cluster" keeps the limit it is documented with: the states and 48 bytes
-            // (FP64: 96) per owned incidence in each block
-            if (sc_.p.sweepMode == "cluster" && lean + (sizeof(R) == 8 ? 96 : 48) * size_t(cluster_incidences(C)) > budget)
-                ok = false;
+            // The limit of the mode, the same whether it is asked for or timed by the autotuner (whose
+            // pick can then be asked for): the states and 48 bytes (FP64: 96) per owned incidence in
+            // each block. The records take less, at most about a third of it on a lattice, but every
+            // scene within the limit is accepted: the lean form holds the states only.
+            if (lean + (sizeof(R) == 8 ? 96 : 48) * size_t(cluster_incidences(C)) > budget) ok = false;
             if (ok && bytes + min_stage <= budget)
                 cluster_fits_.push_back({C, int32_t(pos_cap), int32_t(nbr_cap), int32_t(inc_cap), bytes, false});
-            else if (ok && sc_.p.sweepMode == "cluster" && lean + min_stage <= budget)
+            else if (ok && lean + min_stage <= budget)
                 cluster_fits_.push_back({C, int32_t(pos_cap), 0, 0, lean, true});
         }
         cluster_budget_ = budget;

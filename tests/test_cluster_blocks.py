@@ -76,3 +76,29 @@ def test_cluster_block_beside_a_large_scene(tmp_path, gaia_lib, block):
         phys.close()
         assert st["sweep_mode"] == {"merged": 0, "cluster": 2}[mode]
     np.testing.assert_array_equal(x["merged"], x["cluster"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cluster,fits", [(4, False), (8, True)])
+def test_autotuner_times_the_cluster_sizes_that_can_be_asked_for(tmp_path, gaia_lib, cluster, fits):
+    """A 9^3 cube in FP64: 4 blocks are past the mode's limit of states and incidences per block,
+    8 are not, for the explicit mode and for the autotuner alike."""
+    from gaia_gb300 import VBDPhysics, scenes
+    from gaia_gb300._lib import GaiaError
+
+    X, T = scenes.lattice_cube((9, 9, 9), 0.01)[:2]
+    tp, cp = scenes._write_mesh(str(tmp_path), "cube", X, T)
+    mp, pp = scenes._write_json(str(tmp_path), [scenes.model_entry(tp, cp)],
+                                scenes.physics_params(1.0 / 300.0, 4, precision="fp64"), collision=scenes.NO_CONTACT)
+    timed = {}
+    for mode in ("cluster", "auto"):
+        phys = VBDPhysics()
+        phys.loadRunningparameters(mp, scenes.set_precision(pp, "fp64", out_path="%s.%s.json" % (pp, mode), sweepMode=mode,
+                                                            clusterSize=cluster))
+        try:
+            phys.initialize()
+            timed[mode] = mode == "cluster" or phys.stats()["sweep_ms_cluster"] > 0
+        except GaiaError:
+            timed[mode] = False
+        phys.close()
+    assert timed == {"cluster": fits, "auto": fits}
