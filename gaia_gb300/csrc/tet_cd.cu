@@ -705,6 +705,21 @@ __global__ void k_rel(Dev D, const unsigned long long* keys, int32_t n, uint8_t*
     if (rank == 3 || last) info[s] = uint8_t(info[s] | (rank + 1));
 }
 
+__global__ void k_sample_records(Dev D, int nf, uint8_t* info, int4* own, int32_t* rel) {
+    const int i = 32 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= D.nsv || nf <= 0) return;
+    const int slot = D.sv[i].x;
+    const int g0 = int((long long)(i) * nf / D.nsv);  // meshes and their faces are in the vertices' order
+    for (int k = 0; k < 16; ++k) {
+        const int4 f = D.faces[(g0 + k) % nf];
+        if (f.x == slot || f.y == slot || f.z == slot) continue;
+        own[slot] = f;
+        for (int j = 0; j < 4; ++j) rel[4 * size_t(slot) + j] = (slot << 2) | 3;
+        info[slot] = 8 | 4;
+        return;
+    }
+}
+
 }  // namespace
 
 struct Detector::Impl {
@@ -870,6 +885,23 @@ void Detector::reset(cudaStream_t st) {
     TCD_CUDA(cudaMemsetAsync(I.pen, 0, std::max(nsv_, 1), st));
     TCD_CUDA(cudaMemsetAsync(I.info, 0, std::max(nslots_, 1), st));
     TCD_CUDA(cudaMemsetAsync(I.nlist, 0, sizeof(int32_t), st));
+}
+
+void Detector::clear_records(cudaStream_t st) {
+    if (!enabled() || !d_) return;
+    TCD_CUDA(cudaMemsetAsync(d_->info, 0, std::max(nslots_, 1), st));
+    TCD_CUDA(cudaMemsetAsync(d_->nlist, 0, sizeof(int32_t), st));
+}
+
+void Detector::sample_records(cudaStream_t st) {
+    if (!enabled() || !d_ || nsv_ == 0 || nf_ == 0) return;
+    Impl& I = *d_;
+    clear_records(st);
+    k_sample_records<<<blocks((nsv_ + 31) / 32, 256), 256, 0, st>>>(I.D, nf_, I.info, I.own, I.rel);
+    TCD_CUDA(cudaGetLastError());
+    size_t sb = I.select_tmp_bytes;
+    TCD_CUDA(cub::DeviceSelect::Flagged(I.select_tmp, sb, thrust::counting_iterator<int32_t>(0), I.info, I.list,
+                                        I.nlist, nslots_, st));
 }
 
 Records Detector::records() const {

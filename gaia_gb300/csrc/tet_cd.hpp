@@ -80,6 +80,10 @@ public:
     void build(const float4* xf, cudaStream_t st);
     // Clears every result and record (a state reset).
     void reset(cudaStream_t st);
+    // Records as if every 32nd surface vertex were in contact with a nearby face and with four
+    // others (for timing solves before there are contacts), and none again.
+    void sample_records(cudaStream_t st);
+    void clear_records(cudaStream_t st);
     // Enqueues one detection pass (see the reference order in tet_cd.cu): at the start
     // of a substep (intermediate = false) or between iterations. rebuild = rebuild the
     // face hierarchy (otherwise refit); the tet hierarchy is refitted only when some tet

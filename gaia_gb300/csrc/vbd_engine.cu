@@ -151,7 +151,7 @@ int gaia_vbd_initialize(gaia_vbd* h) {
                 }
                 const double t = e->measure_sweep_ms();
                 h->sweep_ms[mode] = t;
-                if (t < tbest) {
+                if (t < 0.97 * tbest) {  // more than the timings of one schedule differ: handles pick alike
                     tbest = t;
                     best = std::move(e);
                 }

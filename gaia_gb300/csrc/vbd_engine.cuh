@@ -1357,6 +1357,7 @@ public:
     }
 
     void run_steps(int n) override {
+        stepped_ = true;
         for (int k = 0; k < n; ++k)
             for (int sub = 0; sub < sc_.p.numSubsteps; ++sub) {
                 if (sub == 0) start_step_log();
@@ -1379,6 +1380,7 @@ public:
             if (total_ms) *total_ms = tot;
             return;
         }
+        stepped_ = true;
         // per-substep sweep events: [start, end] pairs recorded around the sweep graph
         int nsub = n * sc_.p.numSubsteps;
         std::vector<cudaEvent_t> ev(2 * size_t(nsub));
@@ -1408,8 +1410,7 @@ public:
         if (sweep_ms) *sweep_ms = sw;
     }
 
-    // Time per launch of one color's solve over `reps` launches in a row, as the sweep's graph
-    // chains them (programmatic dependent launch).
+    // Time per launch of one color's solve over `reps` launches in a row.
     float time_color(size_t g, int L, int B, int variant, int reps) {
         launch_color(g, L, B, dev::kSolveFriction, false, variant);  // warm-up
         GAIA_CUDA(cudaEventRecord(ev_a_, st_));
@@ -1421,84 +1422,193 @@ public:
         return ms / reps;
     }
 
-    // Autotuner: per merged color, every (kernel variant, lanes per vertex, block
-    // size) is timed on that color's kernel alone (CUDA events around repeated
-    // launches on the current state, positions restored afterwards) and the
-    // fastest is kept. Fixed lanesPerVertex / blockSize / solveVariant
-    // parameters restrict the search.
+    // The state that solves are timed on, put back when it goes out of scope. Before the first step
+    // that is the rest state with every vertex moved a little and, for the merged colors (walls):
+    // the world box raised past the lowest vertices, and contact records on a few where detection
+    // is on. At rest no vertex has a force, and the vertices at a wall or in contact are the ones
+    // a launch waits for. Later it is the state as it stands.
+    class TuneState {
+    public:
+        TuneState(Engine& e, bool walls) : e_(e), c_(e.c_) {
+            const size_t bytes = size_t(e.nslots_) * sizeof(S4);
+            save_.alloc(e.nslots_, nullptr);
+            start_.alloc(e.nslots_, nullptr);
+            GAIA_CUDA(cudaMemcpyAsync(save_.p, e.d_pos_.p, bytes, cudaMemcpyDeviceToDevice, e.st_));
+            if (!e.stepped_) {
+                dev::k_perturb<ST, R><<<div_up(e.nactive_, 256), 256, 0, e.st_>>>(e.ptrs());
+                GAIA_CUDA(cudaGetLastError());
+                if (walls) raise_floor();
+                sampled_ = walls && e.cd_.enabled();
+                if (sampled_) e.cd_.sample_records(e.st_);
+            }
+            GAIA_CUDA(cudaMemcpyAsync(start_.p, e.d_pos_.p, bytes, cudaMemcpyDeviceToDevice, e.st_));
+        }
+        ~TuneState() {
+            e_.c_ = c_;
+            (void)cudaMemcpyAsync(e_.d_pos_.p, save_.p, size_t(e_.nslots_) * sizeof(S4), cudaMemcpyDeviceToDevice, e_.st_);
+            (void)cudaMemsetAsync(e_.d_counters_.p, 0, dev::CNT_N * sizeof(unsigned long long), e_.st_);
+            if (sampled_) try {
+                    e_.cd_.clear_records(e_.st_);
+                } catch (...) {
+                }
+            (void)cudaStreamSynchronize(e_.st_);
+        }
+        TuneState(const TuneState&) = delete;
+        TuneState& operator=(const TuneState&) = delete;
+        const S4* state() const { return start_.p; }
+
+    private:
+        // The wall that gravity points to, a hundredth of the scene's height past the first vertices.
+        void raise_floor() {
+            if (!e_.c_.plane) return;
+            int d = 0;
+            for (int k = 1; k < 3; ++k)
+                if (std::fabs(c_.g[k]) > std::fabs(c_.g[d])) d = k;
+            auto comp = [d](const float4& x) { return d == 0 ? x.x : (d == 1 ? x.y : x.z); };
+            float lo = std::numeric_limits<float>::infinity(), hi = -lo;
+            for (int32_t s = 0; s < e_.nactive_; ++s) {
+                lo = std::min(lo, comp(e_.h_rest_[size_t(s)]));
+                hi = std::max(hi, comp(e_.h_rest_[size_t(s)]));
+            }
+            if (c_.g[d] > 0) {
+                e_.c_.hi[d] = double(hi) - 0.01 * (double(hi) - lo);
+                e_.c_.hi_f[d] = float(e_.c_.hi[d]);
+            } else {
+                e_.c_.lo[d] = double(lo) + 0.01 * (double(hi) - lo);
+                e_.c_.lo_f[d] = float(e_.c_.lo[d]);
+            }
+        }
+        Engine& e_;
+        const dev::Consts<R> c_;
+        DevBuf<S4> save_, start_;
+        bool sampled_ = false;
+    };
+
+    // How much faster a shape has to be timed than one before it to take its place: more than the
+    // timings of one shape differ, so that handles of a scene pick alike (lanes per vertex decide
+    // the order of the sums, and so the last bits of the results).
+    static constexpr float kFaster = 0.97f;
+
+    // One substep's color launches of `iters` iterations, as the sweep's graph chains them.
+    void enqueue_chain(const std::vector<ColorCfg>& cfg, int iters) {
+        if (cd_.enabled()) enqueue_contact_snapshot(0);
+        bool after_solve = false;
+        for (int it = 0; it < iters; ++it)
+            for (size_t g = 0; g < group_beg_.size(); ++g) {
+                if (group_end_[g] <= group_beg_[g]) continue;
+                launch_color(g, cfg[g].L, cfg[g].B, dev::kSolveFriction | ((it & 1) ? dev::kSolveParity : 0),
+                             use_pdl_ && after_solve, cfg[g].variant);
+                after_solve = true;
+            }
+    }
+    // Time of one iteration of a chain, in a graph as in the step.
+    float time_chain(const std::vector<ColorCfg>& cfg, int iters, const S4* save) {
+        struct Exec {
+            cudaGraphExec_t g = nullptr;
+            ~Exec() {
+                if (g) cudaGraphExecDestroy(g);
+            }
+        } exec;
+        exec.g = capture_one([&] { enqueue_chain(cfg, iters); });
+        float best = 1e30f;
+        for (int r = 0; r < 3; ++r) {  // the first one warms up
+            GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+            GAIA_CUDA(cudaEventRecord(ev_a_, st_));
+            GAIA_CUDA(cudaGraphLaunch(exec.g, st_));
+            GAIA_CUDA(cudaEventRecord(ev_b_, st_));
+            GAIA_CUDA(cudaEventSynchronize(ev_b_));
+            float ms = 0.f;
+            GAIA_CUDA(cudaEventElapsedTime(&ms, ev_a_, ev_b_));
+            if (r) best = std::min(best, ms);
+        }
+        return best / float(iters);
+    }
+
+    // Autotuner: the shape (kernel variant, lanes per vertex, block size) of every color, by the
+    // time of whole iterations in a graph on a state like a step's (TuneState): first one shape for
+    // all colors, then, color kind by color kind, every other shape for that kind, kept where the
+    // iteration gets faster. Timed by itself at rest, as it was, a color says little: a small one
+    // costs its launch whatever the shape (4.7 us apart from a graph, 2 us in one), a large one finds
+    // its records in the caches, and neither a wall nor a contact keeps a lane busy. Rules for what
+    // that got wrong (a warp per vertex up to 1024 vertices, no two lanes with contact detection)
+    // held only near the scenes they came from. Frame, us, before and now: 12^3 drop, double-float
+    // (432 vertices a color) 320 (32 lanes) and 295 (16); 16^3 drop, FP32 (1024) 355 (32) and 301
+    // (16); 8 colliding bodies in FP64 4800 (2 lanes) and 3050 (8); 10^3 drop, FP32 (100) 562 (32
+    // lanes) both ways.
+    // Fixed lanesPerVertex / blockSize / solveVariant parameters restrict the search.
     void autotune_impl() {
-        if (nactive_ == 0) return;
-        DevBuf<S4> save;
-        save.alloc(nslots_, nullptr);
-        GAIA_CUDA(cudaMemcpyAsync(save.p, d_pos_.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
-        const int Ls[] = {2, 4, 8, 16, 32};
-        // one block size in FP32 (64 and 128 threads measure the same, 256 slower): kernels of
-        // different shape in one chain make the SM drain and repartition its memory between them
-        // (collision drop: 10.2 us per color with one shape for all four, 12.2 us with two)
+        if (nactive_ == 0 || group_beg_.empty()) return;
+        TuneState tune(*this, true);
+        // one block size in FP32 (64 and 128 threads measure the same, 256 slower)
         const std::vector<int> Bs = block_ ? std::vector<int>{block_} : (sizeof(R) == 4 ? std::vector<int>{128} : std::vector<int>{64, 128});
         // kernel variants: 0 register gathers, 4 asynchronous one-ring copies, 6 as 0 with the data of
-        // the warps one resident wave ahead prefetched into L2 (FP32 compute only). The TMA
-        // variants 1 and 7 run on request only: with 8-byte records a block's range is a few KB,
-        // and waiting for all of it costs more than the loads it saves (100^3 twist, FP32, best
-        // shape: 47.3 us per color against 43.3 us for variant 0 and 41.2 us for 6).
+        // the warps one resident wave ahead prefetched into L2 (FP32 compute only); 4 and 6 are 0 at
+        // 16 and 32 lanes. The TMA variants 1 and 7 run on request only: with 8-byte records a
+        // block's range is a few KB, and waiting for all of it costs more than the loads it saves
+        // (100^3 twist, FP32, best shape: 47.3 us per color against 43.3 us for variant 0 and 41.2
+        // us for 6).
         std::vector<int> variants = {0, kVariantDeep};
         if (sizeof(R) == 4) variants.push_back(kVariantPrefetch);
         if (variant_fixed_ >= 0) variants = {variant_fixed_};
-        const int reps = 4;
-        ccfg_.assign(group_beg_.size(), ColorCfg{});
-        double total = 0.0;
-        for (size_t g = 0; g < group_beg_.size(); ++g) {
-            const int beg = group_beg_[g], end = group_end_[g];
-            if (end <= beg) continue;
-            ColorCfg best;
-            best.ms = 1e30f;
-            std::vector<ColorCfg> tried;
-            // A color of up to kLatencyColor vertices is one chain of loads and arithmetic, which a
-            // warp per vertex makes shortest; its time apart from the chain of launches is the
-            // launch itself (4.7 us whatever the shape), so timing it alone picks at random. 10^3
-            // drop, 100 vertices per color, FP32: 32 lanes 2.6 us per color in the chain, 16 lanes
-            // 2.8-3.1 us, 8 lanes 3.4-3.7 us; and one shape for all small colors keeps its code in
-            // the instruction cache from launch to launch.
-            const bool chain = sizeof(R) == 4 && end - beg <= kLatencyColor && variant_fixed_ < 0;
-            for (int var : variants) {
-                if (chain && var != 0) continue;
-                for (int L : Ls) {
-                    if (lanes_ && L != lanes_) continue;
-                    if (chain && !lanes_ && L != 32) continue;
-                    // With contact detection on, the launches timed here have no contact records yet, and
-                    // two lanes share a contact vertex's terms badly: 24 bodies, double-float, 12
-                    // iterations, all colors alike, a frame takes 1373 us with 2 lanes, 1239 with 4,
-                    // 1183 with 8, while the timing here puts 2 lanes first (10.8 against 11.7 us).
-                    if (sizeof(R) == 4 && cd_.enabled() && !lanes_ && L == 2) continue;
-                    for (int B : Bs) {
-                        if (chain && !block_ && B != 128) continue;
-                        const ColorCfg run = effective(g, ColorCfg{L, B, var, 0.f});
-                        if (!lanes_ && run.L != L) continue;  // another candidate runs so
-                        const float ms = time_color(g, L, B, var, reps);
-                        tried.push_back(ColorCfg{run.L, run.B, run.variant, ms});
-                        if (ms < best.ms) best = tried.back();
-                    }
+        std::vector<ColorCfg> shapes;
+        for (int var : variants)
+            for (int L : {32, 16, 8, 4, 2}) {
+                if (lanes_ && L != lanes_) continue;
+                if (L >= 16 && variant_fixed_ < 0 && var != 0) continue;
+                for (int B : Bs) shapes.push_back(ColorCfg{L, B, var, 0.f});
+            }
+        const size_t ng = group_beg_.size();
+        auto same = [](const ColorCfg& a, const ColorCfg& b) { return a.L == b.L && a.B == b.B && a.variant == b.variant; };
+        // colors of a kind: about as many vertices, with lists as long
+        std::map<std::tuple<int, int, int>, std::vector<size_t>> kinds;
+        for (size_t g = 0; g < ng; ++g) {
+            const int n = group_end_[g] - group_beg_[g];
+            if (n <= 0 || group_mid_[g] <= group_beg_[g]) continue;
+            const int2 lists = max_lists(group_beg_[g], group_mid_[g]);
+            kinds[std::make_tuple(-int(std::lround(2.0 * std::log2(double(n)))), lists.x, lists.y)].push_back(g);
+        }
+        int iters = 2;
+        std::vector<ColorCfg> best;
+        float tbest = 1e30f;
+        for (ColorCfg& c : shapes) {
+            std::vector<ColorCfg> cfg(ng);
+            for (size_t g = 0; g < ng; ++g) cfg[g] = effective(g, c);
+            if (best.empty()) {  // enough iterations for the events' resolution (about 2 us)
+                const float t = time_chain(cfg, iters, tune.state());
+                iters = std::max(1, std::min(10, int(std::ceil(0.3f / t))));
+            }
+            const float t = time_chain(cfg, iters, tune.state());
+            c.ms = t;
+            if (t < kFaster * tbest) {
+                tbest = t;
+                best = cfg;
+            }
+        }
+        // (a shape that takes twice the time for all colors is no better for one)
+        const float limit = 2.f * tbest;
+        for (auto& kind : kinds)  // largest colors first
+            for (const ColorCfg& c : shapes) {
+                if (c.ms > limit) continue;
+                std::vector<ColorCfg> cfg = best;
+                bool other = false;
+                for (size_t g : kind.second) {
+                    cfg[g] = effective(g, c);
+                    other = other || !same(cfg[g], best[g]);
+                }
+                if (!other) continue;
+                const float t = time_chain(cfg, iters, tune.state());
+                if (t < kFaster * tbest) {
+                    tbest = t;
+                    best = cfg;
                 }
             }
-            // the closest ones again, in turn, over more launches: one short timing picks at random
-            // among shapes within its noise (the step of a scene then varies by 10% from handle to handle)
-            std::sort(tried.begin(), tried.end(), [](const ColorCfg& x, const ColorCfg& y) { return x.ms < y.ms; });
-            if (tried.size() > 4) tried.resize(4);
-            if (tried.size() > 1) {
-                best.ms = 1e30f;
-                for (ColorCfg& t : tried) t.ms = 1e30f;
-                for (int round = 0; round < 3; ++round)
-                    for (ColorCfg& t : tried) t.ms = std::min(t.ms, time_color(g, t.L, t.B, t.variant, 2 * reps));
-                for (const ColorCfg& t : tried)
-                    if (t.ms < best.ms) best = t;
-            }
-            ccfg_[g] = best;
-            total += best.ms;
-            GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+        ccfg_ = best;
+        // one launch of each color, as reported
+        for (size_t g = 0; g < ng; ++g) {
+            if (group_end_[g] <= group_beg_[g]) continue;
+            ccfg_[g].ms = time_color(g, ccfg_[g].L, ccfg_[g].B, ccfg_[g].variant, 4);
         }
-        GAIA_CUDA(cudaMemsetAsync(d_counters_.p, 0, dev::CNT_N * sizeof(unsigned long long), st_));
-        GAIA_CUDA(cudaStreamSynchronize(st_));
-        tuned_ms_ = total;
+        tuned_ms_ = tbest;
         tuned_ = true;
     }
 
@@ -1574,9 +1684,7 @@ public:
     // sweep of the current state (restored afterwards); ms per iteration of the fastest.
     void autotune_scenes() {
         if (nactive_ == 0 || nscenes_ == 0 || sc_.p.iterations == 0) return;
-        DevBuf<S4> save;
-        save.alloc(nslots_, nullptr);
-        GAIA_CUDA(cudaMemcpyAsync(save.p, d_pos_.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+        TuneState tune(*this, false);
         const int Ls[] = {4, 8, 16, 32};
         const int Bs[] = {256, 512, 1024};
         float best = 1e30f;
@@ -1585,24 +1693,23 @@ public:
             for (int B : Bs) {
                 if (block_ && B != block_) continue;
                 if (!lanes_ && fit_sweep_lanes(L, B) != L) continue;  // another candidate runs so
-                enqueue_scenes_sweep(L, B);  // warm-up
-                GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
-                GAIA_CUDA(cudaEventRecord(ev_a_, st_));
-                enqueue_scenes_sweep(L, B);
-                GAIA_CUDA(cudaEventRecord(ev_b_, st_));
-                GAIA_CUDA(cudaEventSynchronize(ev_b_));
                 float ms = 0.f;
-                GAIA_CUDA(cudaEventElapsedTime(&ms, ev_a_, ev_b_));
-                GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
-                if (ms < best) {
+                for (int r = 0; r < 2; ++r) {  // the first one warms up
+                    GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, tune.state(), nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+                    GAIA_CUDA(cudaEventRecord(ev_a_, st_));
+                    enqueue_scenes_sweep(L, B);
+                    GAIA_CUDA(cudaEventRecord(ev_b_, st_));
+                    GAIA_CUDA(cudaEventSynchronize(ev_b_));
+                    ms = 0.f;
+                    GAIA_CUDA(cudaEventElapsedTime(&ms, ev_a_, ev_b_));
+                }
+                if (ms < kFaster * best) {
                     best = ms;
                     scene_L_ = L;
                     scene_B_ = B;
                 }
             }
         }
-        GAIA_CUDA(cudaMemsetAsync(d_counters_.p, 0, dev::CNT_N * sizeof(unsigned long long), st_));
-        GAIA_CUDA(cudaStreamSynchronize(st_));
         tuned_ms_ = double(best) / sc_.p.iterations;
         tuned_ = true;
     }
@@ -1807,9 +1914,7 @@ public:
     // timed on a full sweep of the current state (restored afterwards).
     void autotune_cluster() {
         if (nactive_ == 0 || nscenes_ == 0 || sc_.p.iterations == 0) return;
-        DevBuf<S4> save;
-        save.alloc(nslots_, nullptr);
-        GAIA_CUDA(cudaMemcpyAsync(save.p, d_pos_.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+        TuneState tune(*this, false);
         float best = 1e30f;
         for (const ClusterFit& f : cluster_fits_) {
             if (sc_.p.clusterSize && f.C != sc_.p.clusterSize) continue;
@@ -1820,16 +1925,17 @@ public:
                     int l = L, b = B;
                     fit_cluster(f, l, b);
                     if ((!lanes_ && l != L) || (!block_ && b != B && b == 128)) continue;  // another candidate runs so
-                    enqueue_cluster_sweep(f.C, L, B);  // warm-up
-                    GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
-                    GAIA_CUDA(cudaEventRecord(ev_a_, st_));
-                    enqueue_cluster_sweep(f.C, L, B);
-                    GAIA_CUDA(cudaEventRecord(ev_b_, st_));
-                    GAIA_CUDA(cudaEventSynchronize(ev_b_));
                     float ms = 0.f;
-                    GAIA_CUDA(cudaEventElapsedTime(&ms, ev_a_, ev_b_));
-                    GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
-                    if (ms < best) {
+                    for (int r = 0; r < 2; ++r) {  // the first one warms up
+                        GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, tune.state(), nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+                        GAIA_CUDA(cudaEventRecord(ev_a_, st_));
+                        enqueue_cluster_sweep(f.C, L, B);
+                        GAIA_CUDA(cudaEventRecord(ev_b_, st_));
+                        GAIA_CUDA(cudaEventSynchronize(ev_b_));
+                        ms = 0.f;
+                        GAIA_CUDA(cudaEventElapsedTime(&ms, ev_a_, ev_b_));
+                    }
+                    if (ms < kFaster * best) {
                         best = ms;
                         scene_C_ = f.C;
                         scene_L_ = L;
@@ -1838,8 +1944,6 @@ public:
                 }
             }
         }
-        GAIA_CUDA(cudaMemsetAsync(d_counters_.p, 0, dev::CNT_N * sizeof(unsigned long long), st_));
-        GAIA_CUDA(cudaStreamSynchronize(st_));
         if (!(best < 1e30f)) throw std::runtime_error("cluster sweep: no configuration was timed");
         tuned_ms_ = double(best) / sc_.p.iterations;
         tuned_ = true;
@@ -1937,33 +2041,30 @@ public:
     // the current state (restored afterwards).
     void autotune_grid() {
         if (nactive_ == 0 || grid_ncolors_ == 0 || sc_.p.iterations == 0) return;
-        DevBuf<S4> save;
-        save.alloc(nslots_, nullptr);
-        GAIA_CUDA(cudaMemcpyAsync(save.p, d_pos_.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+        TuneState tune(*this, false);
         float best = 1e30f;
         for (int L : {4, 8, 16, 32}) {
             if (lanes_ && L != lanes_) continue;
             for (int B : {128, 256}) {
                 if (block_ && B != block_) continue;
                 if (!lanes_ && fit_sweep_lanes(L, B) != L) continue;  // another candidate runs so
-                enqueue_grid_sweep(L, B);  // warm-up
-                GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
-                GAIA_CUDA(cudaEventRecord(ev_a_, st_));
-                enqueue_grid_sweep(L, B);
-                GAIA_CUDA(cudaEventRecord(ev_b_, st_));
-                GAIA_CUDA(cudaEventSynchronize(ev_b_));
                 float ms = 0.f;
-                GAIA_CUDA(cudaEventElapsedTime(&ms, ev_a_, ev_b_));
-                GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
-                if (ms < best) {
+                for (int r = 0; r < 2; ++r) {  // the first one warms up
+                    GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, tune.state(), nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+                    GAIA_CUDA(cudaEventRecord(ev_a_, st_));
+                    enqueue_grid_sweep(L, B);
+                    GAIA_CUDA(cudaEventRecord(ev_b_, st_));
+                    GAIA_CUDA(cudaEventSynchronize(ev_b_));
+                    ms = 0.f;
+                    GAIA_CUDA(cudaEventElapsedTime(&ms, ev_a_, ev_b_));
+                }
+                if (ms < kFaster * best) {
                     best = ms;
                     scene_L_ = L;
                     scene_B_ = B;
                 }
             }
         }
-        GAIA_CUDA(cudaMemsetAsync(d_counters_.p, 0, dev::CNT_N * sizeof(unsigned long long), st_));
-        GAIA_CUDA(cudaStreamSynchronize(st_));
         if (!(best < 1e30f)) throw std::runtime_error("grid sweep: no configuration was timed");
         tuned_ms_ = double(best) / sc_.p.iterations;
         tuned_ = true;
@@ -2015,6 +2116,7 @@ public:
         cd_.reset(st_);
         GAIA_CUDA(cudaStreamSynchronize(st_));
         reset_frames();
+        stepped_ = false;
     }
 
     void autotune() override {
@@ -2039,17 +2141,15 @@ public:
 
     double tuned_ms() const override { return tuned_ms_; }
 
-    // Device time of the captured sweep graph (all iterations of one substep) on the
-    // current state, per iteration; the state is restored afterwards.
+    // Device time of the captured sweep graph (all iterations of one substep) on the state of
+    // the autotuners, per iteration; the state is restored afterwards.
     double measure_sweep_ms() override {
-        DevBuf<S4> save;
-        save.alloc(nslots_, nullptr);
-        GAIA_CUDA(cudaMemcpyAsync(save.p, d_pos_.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+        TuneState tune(*this, false);
         GAIA_CUDA(cudaGraphLaunch(g_sweep_, st_));  // warm-up
         const int reps = 3;
         float total = 0.f;
         for (int r = 0; r < reps; ++r) {
-            GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
+            GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, tune.state(), nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
             GAIA_CUDA(cudaEventRecord(ev_a_, st_));
             GAIA_CUDA(cudaGraphLaunch(g_sweep_, st_));
             GAIA_CUDA(cudaEventRecord(ev_b_, st_));
@@ -2058,9 +2158,6 @@ public:
             GAIA_CUDA(cudaEventElapsedTime(&ms, ev_a_, ev_b_));
             total += ms;
         }
-        GAIA_CUDA(cudaMemcpyAsync(d_pos_.p, save.p, nslots_ * sizeof(S4), cudaMemcpyDeviceToDevice, st_));
-        GAIA_CUDA(cudaMemsetAsync(d_counters_.p, 0, dev::CNT_N * sizeof(unsigned long long), st_));
-        GAIA_CUDA(cudaStreamSynchronize(st_));
         return double(total) / reps / std::max(sc_.p.iterations, 1);
     }
 
@@ -2148,6 +2245,7 @@ public:
     // start-of-substep positions); returns the number of vertices with a contact.
     int collide() override {
         if (!cd_.enabled()) return 0;
+        stepped_ = true;
         enqueue_detection(false, true);
         std::vector<int32_t> rows;
         cd_.contacts(rows, st_);
@@ -2416,6 +2514,7 @@ private:
     int lanes_ = 0, block_ = 0;
     std::vector<ColorCfg> ccfg_;
     bool tuned_ = false;
+    bool stepped_ = false;  // a step or a detection ran since the start or the last reset
     bool use_pdl_ = true;
     int small_color_ = 16384;
     int variant_ = 0;          // 0 = register-pipelined k_solve, 1 = TMA-staged k_solve_tma, 2 = k_sweep_scenes,
@@ -2449,7 +2548,6 @@ private:
     std::map<std::tuple<const void*, int, size_t>, int> occ_cache_;  // (kernel, block, shared bytes) -> blocks per SM
     int sms_ = 0;
     static constexpr size_t kTmaSmemMax = 200 * 1024;
-    static constexpr int kLatencyColor = 1024;
     static constexpr int kContactBlocks = 64;
     double tuned_ms_ = 0.0;
     int64_t launches_per_substep_ = 0, launches_per_step_ = 0;

@@ -1542,6 +1542,27 @@ __global__ void k_initial_step(Ptrs<ST, R> P, Consts<R> c) {
     P.u[s] = xn;
 }
 
+// A state to time solves on: every solved vertex moved by up to a hundredth of the distance to
+// its first neighbour (at rest no vertex has a force, and the solves end at the force test).
+template <typename ST, typename R>
+__global__ void k_perturb(Ptrs<ST, R> P) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= P.nactive) return;
+    const int4 seg = P.vrec[s];
+    if (nbrs_of(seg.z) == 0) return;
+    const float4 a = P.rest[s], b = P.rest[P.nbr[record_index(seg.x, place_of(seg.z))].slot];
+    const float d = sqrtf((a.x - b.x) * (a.x - b.x) + (a.y - b.y) * (a.y - b.y) + (a.z - b.z) * (a.z - b.z));
+    using Sc = typename ST::Sc;
+    uint32_t h = uint32_t(s) * 2654435761u;
+    Sc m[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        h = (h ^ (h >> 15)) * 2246822519u + 374761393u;
+        m[c] = Sc(0.01f * d) * (Sc(h >> 8) * Sc(1.0 / 8388608.0) - Sc(1));
+    }
+    P.u[s] = ST::add(P.u[s], m[0], m[1], m[2]);
+}
+
 // Deformers (VBD/VBDDeformer.h:45-172). Rotator: p = root + R(theta) rootP with
 // theta = omega * t; Translator: p = orig + speed * t. t = time after this substep's
 // advance, clamped to the end time. Per selected vertex, in FP64 (a few thousand
