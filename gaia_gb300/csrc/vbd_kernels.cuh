@@ -608,6 +608,46 @@ __device__ __forceinline__ void halve(double* v, int off, bool upper) {
     }
 }
 
+// One halving step of N float pairs (k, l), as halve.
+template <int N>
+__device__ __forceinline__ void halve_pairs(float* k, float* l, int off, bool upper) {
+    constexpr int H = (N + 1) / 2;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        const float khi = i + H < N ? k[i + H] : 0.f, lhi = i + H < N ? l[i + H] : 0.f;
+        const float ko = __shfl_xor_sync(0xffffffffu, upper ? k[i] : khi, off);
+        const float lo = __shfl_xor_sync(0xffffffffu, upper ? l[i] : lhi, off);
+        float s, e;
+        two_sum(upper ? khi : k[i], ko, s, e);
+        k[i] = s;
+        l[i] = __fadd_rn(__fadd_rn(upper ? lhi : l[i], lo), e);
+    }
+}
+
+// The three pairs of the accumulator over the L lanes of a vertex, rounded once, on sub-lane 0 (in
+// k0, k1, k2): a lane holds two of them after the first step and one after the second.
+template <int L>
+__device__ __forceinline__ void reduce_pairs(Acc<float>& a) {
+    constexpr int W = 32 / L;
+    float k[3] = {a.k0, a.k1, a.k2}, l[3] = {a.l0, a.l1, a.l2};
+    const int sub = Lanes<L>::sub(), vw = Lanes<L>::vertex();
+    halve_pairs<3>(k, l, 16, (sub & (L / 2)) != 0);
+    if constexpr (L >= 4) halve_pairs<2>(k, l, 8, (sub & (L / 4)) != 0);
+#pragma unroll
+    for (int off = 4; off >= W; off >>= 1) {
+        const float ko = __shfl_xor_sync(0xffffffffu, k[0], off), lo = __shfl_xor_sync(0xffffffffu, l[0], off);
+        float s, e;
+        two_sum(k[0], ko, s, e);
+        k[0] = s;
+        l[0] = __fadd_rn(__fadd_rn(l[0], lo), e);
+    }
+    const float t = __fadd_rn(k[0], l[0]);
+    a.k0 = t;
+    a.k1 = L >= 4 ? __shfl_sync(0xffffffffu, t, (L / 4) * W + vw) : __fadd_rn(k[1], l[1]);
+    a.k2 = __shfl_sync(0xffffffffu, t, (L / 2) * W + vw);
+    a.l0 = a.l1 = a.l2 = 0.f;
+}
+
 // Sums over the L lanes of a vertex; valid on sub-lane 0.
 template <int L, typename R>
 __device__ __forceinline__ void reduce_group(Acc<R>& a) {
@@ -649,19 +689,8 @@ __device__ __forceinline__ void reduce_group(Acc<R>& a) {
             a.h12 += __shfl_xor_sync(0xffffffffu, a.h12, off);
             a.h22 += __shfl_xor_sync(0xffffffffu, a.h22, off);
             a.S += __shfl_xor_sync(0xffffffffu, a.S, off);
-            if constexpr (sizeof(R) == 4) {
-                auto join = [&](float& k, float& l) {
-                    const float ko = __shfl_xor_sync(0xffffffffu, k, off), lo = __shfl_xor_sync(0xffffffffu, l, off);
-                    float s, e;
-                    two_sum(k, ko, s, e);
-                    k = s;
-                    l = __fadd_rn(__fadd_rn(l, lo), e);
-                };
-                join(a.k0, a.l0);
-                join(a.k1, a.l1);
-                join(a.k2, a.l2);
-            }
         }
+        if constexpr (sizeof(R) == 4) reduce_pairs<L>(a);
     }
 }
 
