@@ -397,22 +397,59 @@ __device__ __forceinline__ void pair_fma(float x, float y, float& k, float& l) {
     k = s;
 }
 
-// x.y as a float pair s + er.
-__device__ __forceinline__ float dot_pair(const float* x, const float* y, float& er) {
-    float s = __fmul_rn(x[0], y[0]);
-    er = __fmaf_rn(x[0], y[0], -s);
-#pragma unroll
-    for (int c = 1; c < 3; ++c) pair_fma(x[c], y[c], s, er);
-    return s;
+// Two floats in a 64-bit register pair, operated on at once.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
 }
 
-// N.e + C.p, which cancel where the tet is rotated.
+// N.e + C.p, which cancel where the tet is rotated: FP32 as two dot products, each a float pair
+// (as pair_fma), the two in one packed sequence. Packed and scalar, the same operations, us a frame:
+// 24 cubes, double-float, 1062 and 1105; collision drop, FP32, 2010 and 2100; 47^3 twist,
+// double-float, 2076 and 2098; 100^3 twist and 200 cubes, FP32, 1% slower packed.
 template <typename R>
 __device__ __forceinline__ R volume_change(const R* N, const R* e, const R* C, const R* p) {
     if constexpr (sizeof(R) == 4) {
-        float en, ec;
-        const float n = dot_pair(N, e, en), c = dot_pair(C, p, ec);
-        return __fadd_rn(__fadd_rn(n, c), __fadd_rn(en, ec));
+        F2 x = pack2(N[0], C[0]), y = pack2(e[0], p[0]);
+        F2 s = mul2(x, y);
+        F2 er = fma2(x, y, sub2(pack2(0.f, 0.f), s));
+#pragma unroll
+        for (int c = 1; c < 3; ++c) {
+            x = pack2(N[c], C[c]);
+            y = pack2(e[c], p[c]);
+            const F2 t = add2(s, mul2(x, y));
+            const F2 nb = sub2(s, t);
+            er = add2(er, add2(sub2(s, add2(t, nb)), fma2(x, y, nb)));
+            s = t;
+        }
+        float s0, s1, e0, e1;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(s.v));
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(e0), "=f"(e1) : "l"(er.v));
+        return __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(e0, e1));
     } else {
         return (N[0] * e[0] + N[1] * e[1] + N[2] * e[2]) + (C[0] * p[0] + C[1] * p[1] + C[2] * p[2]);
     }
