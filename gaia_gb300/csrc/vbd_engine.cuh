@@ -1487,7 +1487,7 @@ public:
     // How much faster a shape has to be timed than one before it to take its place: more than the
     // timings of one shape differ, so that handles of a scene pick alike (lanes per vertex decide
     // the order of the sums, and so the last bits of the results).
-    static constexpr float kFaster = 0.97f;
+    static constexpr float kFaster = 0.98f;
 
     // One substep's color launches of `iters` iterations, as the sweep's graph chains them.
     void enqueue_chain(const std::vector<ColorCfg>& cfg, int iters) {
@@ -1531,10 +1531,10 @@ public:
     // costs its launch whatever the shape (4.7 us apart from a graph, 2 us in one), a large one finds
     // its records in the caches, and neither a wall nor a contact keeps a lane busy. Rules for what
     // that got wrong (a warp per vertex up to 1024 vertices, no two lanes with contact detection)
-    // held only near the scenes they came from. Frame, us, before and now: 12^3 drop, double-float
-    // (432 vertices a color) 320 (32 lanes) and 295 (16); 16^3 drop, FP32 (1024) 355 (32) and 301
-    // (16); 8 colliding bodies in FP64 4800 (2 lanes) and 3050 (8); 10^3 drop, FP32 (100) 562 (32
-    // lanes) both ways.
+    // held only near the scenes they came from. 12^3 drop, double-float (432 vertices a color): a
+    // frame of 320 us with 32 lanes, 295 with 16; 16^3 drop, FP32 (1024): a device step of 278 us
+    // with 32, 219 with 16; 8 colliding bodies in FP64: a frame of 4800 us with 2 lanes, 3050 with
+    // 8; 10^3 drop, FP32 (100): a device step of 190 us with 32, 205 with 16.
     // Fixed lanesPerVertex / blockSize / solveVariant parameters restrict the search.
     void autotune_impl() {
         if (nactive_ == 0 || group_beg_.empty()) return;
@@ -1567,28 +1567,40 @@ public:
             const int2 lists = max_lists(group_beg_[g], group_mid_[g]);
             kinds[std::make_tuple(-int(std::lround(2.0 * std::log2(double(n)))), lists.x, lists.y)].push_back(g);
         }
-        int iters = 2;
+        int iters = 2, narrow_var = -1, narrow = 0, last_var = -1;
+        float last = 0.f;
         std::vector<ColorCfg> best;
         float tbest = 1e30f;
         for (ColorCfg& c : shapes) {
             std::vector<ColorCfg> cfg(ng);
             for (size_t g = 0; g < ng; ++g) cfg[g] = effective(g, c);
-            if (best.empty()) {  // enough iterations for the events' resolution (about 2 us)
+            if (best.empty()) {  // enough iterations for the events' resolution, about 40 launches at most
                 const float t = time_chain(cfg, iters, tune.state());
-                iters = std::max(1, std::min(10, int(std::ceil(0.3f / t))));
+                iters = std::max(1, std::min(std::max(2, 40 / int(ng)), int(std::ceil(0.2f / t))));
             }
+            // narrower groups only take longer from here on
+            if (c.variant == narrow_var && c.L < narrow) continue;
             const float t = time_chain(cfg, iters, tune.state());
+            if (t > 1.5f * tbest && c.variant == last_var && t > last) {
+                narrow_var = c.variant;
+                narrow = c.L;
+            }
+            last_var = c.variant;
+            last = t;
             c.ms = t;
             if (t < kFaster * tbest) {
                 tbest = t;
                 best = cfg;
             }
         }
-        // (a shape that takes twice the time for all colors is no better for one)
+        // the four kinds of the largest colors; a shape that takes twice the time for all colors is
+        // no better for one
         const float limit = 2.f * tbest;
-        for (auto& kind : kinds)  // largest colors first
+        int left = 4;
+        for (auto& kind : kinds) {
+            if (left-- == 0) break;
             for (const ColorCfg& c : shapes) {
-                if (c.ms > limit) continue;
+                if (c.ms == 0.f || c.ms > limit) continue;
                 std::vector<ColorCfg> cfg = best;
                 bool other = false;
                 for (size_t g : kind.second) {
@@ -1602,6 +1614,7 @@ public:
                     best = cfg;
                 }
             }
+        }
         ccfg_ = best;
         // one launch of each color, as reported
         for (size_t g = 0; g < ng; ++g) {
