@@ -40,12 +40,12 @@ sys.path.insert(0, ROOT)
 
 METRIC = "VBD vertex-solves/s & steps/s, FP32-mixed vs plain FP64 at <=1e-5 rel pos err"
 # dram__bytes_read.sum + dram__bytes_write.sum per solved incidence of k_solve, measured by
-# ncu on 8 color launches each of the 60^3 twist (1.009 M incidences a launch; 21.89 MB FP32,
-# 26.18 MB double-float); see profiles/
+# ncu on 4 color launches each of the 60^3 twist (1.009 M incidences a launch; 21.89 MB FP32,
+# 26.18 MB double-float, cold caches); see profiles/k_solve_one_ring.md
 TRAFFIC_BYTES_PER_INCIDENCE = {"fp32": 21.7, "mixed": 25.9}
 # DRAM bytes (read + write) of one k_sweep_scenes launch per solved incidence and iteration:
-# 1.056 GB over 4 iterations of a 200-cube batch's 15.23 M incidences (FP32, mesh frames)
-SCENES_TRAFFIC_BYTES_PER_INCIDENCE_ITERATION = 17.3
+# 0.998 GB over 4 iterations of a 200-cube batch's 15.23 M incidences (FP32, mesh frames)
+SCENES_TRAFFIC_BYTES_PER_INCIDENCE_ITERATION = 16.4
 
 
 def load_peaks() -> tuple[float, str]:
@@ -806,34 +806,31 @@ def main():
     if rank == 0:
         st = head["stats"]
         nact, ninc, n = head["nact"], head["ninc"], head["n"]
-        # roofline of the solve kernel: algorithmic bytes per iteration 64 B/vertex + 61 B/incidence;
-        # the persistent schedules run a substep's iterations in one launch
-        alg_bytes_iter = 64.0 * nact + 61.0 * ninc
+        # roofline of the solve kernel: the DRAM bytes it moves (per solved incidence, from ncu
+        # captures of smaller scenes of the same kind), where they were measured, else a lower bound
+        # of what its layout reads and writes per iteration (8 B per incidence; per vertex 16 B each
+        # of list positions, rest position, inertia target, state in and state out). The solve is not
+        # bound by DRAM: its loads wait on one another (see "bound"). The persistent schedules run a
+        # substep's iterations in one launch.
         sweep_mode = st.get("sweep_mode", 0)
+        per_inc = TRAFFIC_BYTES_PER_INCIDENCE.get(head["precision"]) if sweep_mode == 0 else (
+            SCENES_TRAFFIC_BYTES_PER_INCIDENCE_ITERATION if sweep_mode == 1 and head["precision"] == "fp32" else None)
+        bytes_iter = per_inc * ninc if per_inc else 80.0 * nact + 8.0 * ninc
         if sweep_mode == 0:
-            launches_solve, kernel, per_launch = st["num_groups"] * args.iterations * args.steps, "k_solve", \
-                alg_bytes_iter / st["num_groups"]
+            launches_solve, kernel = st["num_groups"] * args.iterations * args.steps, "k_solve"
+            per_launch = bytes_iter / st["num_groups"]
         else:
             launches_solve = args.steps * head.get("substeps", 1)
             kernel = {1: "k_sweep_scenes", 2: "k_sweep_cluster", 3: "k_sweep_grid"}[sweep_mode]
-            per_launch = alg_bytes_iter * args.iterations
-        achieved = alg_bytes_iter * args.iterations * args.steps / (head["sweep_ms"] / 1e3) / 1e9
-        # DRAM bytes per solved incidence (records + per-vertex data) from the ncu captures
-        # (TRAFFIC_BYTES_PER_INCIDENCE), scaled to one average launch here
-        per_inc = TRAFFIC_BYTES_PER_INCIDENCE.get(head["precision"])
-        traffic, source = None, None
-        if per_inc and sweep_mode == 0:
-            traffic = per_inc * ninc / st["num_groups"]
-            source = ("ncu DRAM bytes per incidence (60^3 twist launches), times "
-                      "this launch's incidences")
-        elif sweep_mode == 1 and head["precision"] == "fp32":
-            traffic = SCENES_TRAFFIC_BYTES_PER_INCIDENCE_ITERATION * ninc * args.iterations
-            source = ("ncu DRAM bytes of the scene-major sweep per incidence and iteration (200-cube batch, FP32), "
-                      "times this launch's incidences and iterations")
-        roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                    "traffic": traffic, "traffic_source": source,
+            per_launch = bytes_iter * args.iterations
+        achieved = bytes_iter * args.iterations * args.steps / (head["sweep_ms"] / 1e3) / 1e9
+        roofline = {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                    "traffic": per_launch if per_inc else None,
+                    "bytes_source": ("DRAM bytes per incidence and iteration, ncu, %s" %
+                                     ("60^3 twist" if sweep_mode == 0 else "200 cubes")) if per_inc
+                    else "lower bound of the layout (not measured)",
                     "peak_kind": peak_kind, "kernel": kernel,
-                    "algorithmic_bytes_per_launch": per_launch,
+                    "bytes_per_launch": per_launch,
                     "avg_launch_us": 1e3 * head["sweep_ms"] / launches_solve}
         if fp64:
             fp64["speedup_over_fp64"] = head["value"] / fp64["value"]
